@@ -18,7 +18,7 @@ struct alignas(16) Bvh4Node {
     float lo_y[4], hi_y[4];
     float lo_z[4], hi_z[4];
     uint32_t child[4];
-    uint32_t pad[4];
+    uint32_t leaf[4];  // BLAS nodes: a leaf child's number within its BLAS (the flattened tree's leaf records)
 };
 static_assert(sizeof(Bvh4Node) == 128, "BVH4 node must be one 128-byte line");
 
@@ -27,18 +27,24 @@ constexpr uint32_t kLeafFirstMask = (1u << 27) - 1u;
 constexpr uint32_t kLeafMaxCount = 16u;
 
 // Device instance record (64 bytes): local_from_world rows, BLAS root node,
-// triangle range and flags (pack_instances rows 0-2 and word 8, word 6.w).
+// first triangle, the largest coordinate magnitude of its BLAS root box (the
+// slab test's padding) and flags (pack_instances rows 0-2 and word 8, word
+// 6.w).
 struct alignas(16) DeviceInstance {
     float row[3][4];
     uint32_t root;
     uint32_t first;
-    uint32_t count;
+    float extent;
     uint32_t flags;
 };
 
 // Scene data as the kernels see it (all device pointers).
 struct SceneView {
     const Bvh4Node *nodes;
+    const Bvh4Node *flat_nodes;     // flattened tree (world-space copies of the instances' nodes); nullptr: none
+    const uint2 *flat_leaves;       // flattened leaf k: (instance, first triangle)
+    const uint4 *flat_inst;         // per instance: first flat node, first leaf record, first BLAS node, BLAS root
+    uint32_t flat_tlas;             // flat nodes of the TLAS (the copies follow)
     const float4 *triangles;        // 3 float4 per triangle (local positions)
     const DeviceInstance *instances;
     const uint4 *scene_words;       // verbatim reference words (materials, transforms)
@@ -134,6 +140,12 @@ struct LuxScene {
     uint32_t *d_depth_start = nullptr;
     uint2 *d_slot_source = nullptr;             // (binary node, instance or kEmpty) per slot
     uint32_t light_count = 0;
+    // Flattened tree: per instance (first flat node, first leaf record, first
+    // BLAS node, BLAS root node), and its buffers (nullptr: the scene has none).
+    uint4 *d_flat_inst = nullptr;
+    Bvh4Node *d_flat_nodes = nullptr;
+    uint2 *d_flat_leaves = nullptr;
+    uint32_t flat_count = 0, flat_tlas = 0;     // flat nodes; of them the TLAS's
 };
 
 // local_from_world of a 3x4 world_from_local (row-major), inverted in f64

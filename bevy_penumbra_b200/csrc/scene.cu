@@ -74,7 +74,7 @@ struct Collapser {
             n.lo_x[i] = n.lo_y[i] = n.lo_z[i] = INFINITY;
             n.hi_x[i] = n.hi_y[i] = n.hi_z[i] = -INFINITY;
             n.child[i] = lux::kEmpty;
-            n.pad[i] = 0;
+            n.leaf[i] = 0;
         }
         out.push_back(n);
         if (sources)
@@ -188,10 +188,12 @@ struct Collapser {
 };
 
 // 128 threads per block; every lane of a warp walks together (whole-warp
-// leaf tests), lanes past `count` without a query.
-__global__ void __launch_bounds__(128) trace_rays_kernel(SceneView S, const LuxRay *__restrict__ rays, uint32_t count,
-                                                         uint32_t any_hit, LuxHit *__restrict__ hits,
-                                                         unsigned long long *__restrict__ counters) {
+// leaf tests), lanes past `count` without a query.  One kernel per query kind
+// and tree, so each is compiled for its own walk's registers.
+template <bool kAnyHit, bool kFlat>
+__global__ void __launch_bounds__(128, kFlat ? (kAnyHit ? 8 : 7) : 5)
+    trace_rays_kernel(const __grid_constant__ SceneView S, const LuxRay *__restrict__ rays, uint32_t count,
+                      LuxHit *__restrict__ hits, unsigned long long *__restrict__ counters) {
     __shared__ lux::LeafScratch scratch[4];
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     lux::TraceCounters cn{0, 0, 0};
@@ -202,10 +204,12 @@ __global__ void __launch_bounds__(128) trace_rays_kernel(SceneView S, const LuxR
     lux::f3 d{r.direction[0], r.direction[1], r.direction[2]};
     lux::Hit h;
     lux::LeafScratch *L = &scratch[threadIdx.x >> 5];
-    if (any_hit)
-        lux::trace_warp<true>(S, active, o, d, 0.0f, r.limit, h, cn, L);
-    else
-        lux::trace_warp<false>(S, active, o, d, r.tmin, r.limit, h, cn, L);
+    const float tmin = kAnyHit ? 0.0f : r.tmin;
+    if (kFlat) {
+        lux::trace_warp_flat<kAnyHit>(S, active, o, d, tmin, r.limit, h, cn, L);
+    } else {
+        lux::trace_warp<kAnyHit>(S, active, o, d, tmin, r.limit, h, cn, L);
+    }
     if (active) {
         LuxHit out;
         out.distance = h.t;
@@ -334,6 +338,85 @@ __global__ void __launch_bounds__(1024) refit_kernel(uint4 *__restrict__ sw, uin
     }
 }
 
+// The flattened tree from the current TLAS boxes and poses: one thread per
+// child slot.  Slots of the TLAS nodes are copied, a single-instance leaf
+// becoming the root of that instance's copy; slots of a copy take the BLAS
+// child's box through world_from_local (interval arithmetic per axis), padded
+// by 2^-17 of the summed term magnitudes, which is what the instance boxes of
+// the TLAS are padded by.  Memory bound: 128 bytes read and written per node
+// (the BLAS nodes of an instanced mesh come from L2).
+__global__ void __launch_bounds__(256) flatten_kernel(const uint4 *__restrict__ sw, uint32_t inst_base,
+                                                      const Bvh4Node *__restrict__ nodes, const uint4 *__restrict__ inst,
+                                                      uint32_t inst_count, uint32_t tlas, uint32_t total,
+                                                      Bvh4Node *__restrict__ out, uint2 *__restrict__ leaves) {
+    for (uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x; slot < total * 4u; slot += gridDim.x * blockDim.x) {
+        const uint32_t f = slot / 4u, c = slot % 4u;
+        uint32_t k = f, base = 0, leaf_base = 0, node0 = 0, instance = lux::kEmpty;
+        if (f >= tlas) {
+            uint32_t lo = 0, hi = inst_count;  // the instance whose copy holds node f
+            while (hi - lo > 1u) {
+                const uint32_t mid = (lo + hi) >> 1;
+                if (inst[mid].x <= f)
+                    lo = mid;
+                else
+                    hi = mid;
+            }
+            instance = lo;
+            const uint4 w = inst[lo];
+            base = w.x;
+            leaf_base = w.y;
+            node0 = w.z;
+            k = node0 + (f - base);
+        }
+        const Bvh4Node &n = nodes[k];
+        float mn[3] = {n.lo_x[c], n.lo_y[c], n.lo_z[c]}, mx[3] = {n.hi_x[c], n.hi_y[c], n.hi_z[c]};
+        uint32_t child = n.child[c];
+        if (instance == lux::kEmpty) {
+            if (child != lux::kEmpty && (child & kLeafBit)) {
+                const uint4 w = inst[child & kLeafFirstMask];
+                child = w.x + (w.w - w.z);
+            }
+        } else if (child != lux::kEmpty) {
+            if (child & kLeafBit) {
+                const uint32_t record = leaf_base + n.leaf[c];
+                leaves[record] = make_uint2(instance, child & kLeafFirstMask);
+                child = (child & ~kLeafFirstMask) | record;
+            } else {
+                child = base + (child - node0);
+            }
+            float wl[3], wh[3];
+            for (int r = 0; r < 3; ++r) {
+                const float4 row = word_f4(sw[inst_base + instance * 9u + 3u + r]);
+                const float m[3] = {row.x, row.y, row.z};
+                float a = row.w, b = row.w, terms = fabsf(row.w);
+                for (int x = 0; x < 3; ++x) {
+                    const float p = m[x] * mn[x], q = m[x] * mx[x];
+                    a += fminf(p, q);
+                    b += fmaxf(p, q);
+                    terms += fmaxf(fabsf(p), fabsf(q));
+                }
+                const float pad = terms * 7.62939453125e-6f + 1e-30f;
+                const bool finite = isfinite(terms) && isfinite(a) && isfinite(b);
+                wl[r] = finite ? a - pad : -INFINITY;
+                wh[r] = finite ? b + pad : INFINITY;
+            }
+            for (int r = 0; r < 3; ++r) {
+                mn[r] = wl[r];
+                mx[r] = wh[r];
+            }
+        }
+        Bvh4Node &o = out[f];
+        o.lo_x[c] = mn[0];
+        o.lo_y[c] = mn[1];
+        o.lo_z[c] = mn[2];
+        o.hi_x[c] = mx[0];
+        o.hi_y[c] = mx[1];
+        o.hi_z[c] = mx[2];
+        o.child[c] = child;
+        o.leaf[c] = 0u;
+    }
+}
+
 }  // namespace
 
 // Host half of an upload: validation of the reference word streams, the
@@ -347,7 +430,51 @@ struct HostScene {
     std::vector<uint32_t> refit_order, depth_start;
     uint32_t tlas_root = lux::kEmpty, inst_base = 0, inst_count = 0, tri_count = 0, tlas_slots = 0;
     float root_lo[3] = {0, 0, 0}, root_hi[3] = {0, 0, 0};
+    // Flattened tree (flat_count 0: none): per instance (first flat node,
+    // first leaf record, first BLAS node, BLAS root node).
+    std::vector<uint4> flat_inst;
+    uint32_t flat_count = 0, flat_leaves = 0, flat_tlas = 0;
 };
+
+// The flattened tree copies every instance's BLAS nodes into world space, so
+// it is built where that stays small: at most 2^19 nodes (64 MB, half of the
+// L2).  A scene of many instances of large meshes keeps the two-level walk.
+constexpr uint64_t kFlatMaxNodes = 1u << 19;
+
+// Levels of inner nodes at and below `root` (a node of a collapsed tree).
+static uint32_t tree_depth(const std::vector<Bvh4Node> &nodes, uint32_t root) {
+    uint32_t deepest = 0;
+    std::vector<std::pair<uint32_t, uint32_t>> todo = {{root, 1u}};
+    while (!todo.empty()) {
+        auto [index, depth] = todo.back();
+        todo.pop_back();
+        deepest = std::max(deepest, depth);
+        for (uint32_t c : nodes[index].child)
+            if (c != lux::kEmpty && !(c & kLeafBit)) todo.push_back({c, depth + 1u});
+    }
+    return deepest;
+}
+
+// Whether an instance's nodes may be tested in world space: the rounding of
+// the local ray (a few units in the last place of its terms) maps back to the
+// same few units of the world coordinates when max_i sum_j |M_ij| sum_k
+// |R_jk| is small (at most 3 for rotations with any scale per axis), which the
+// slab and box padding covers; sheared, ill-conditioned poses are left to the
+// two-level walk.
+static bool flat_conditioned(const float *lfw, const float *wfl) {
+    double worst = 0.0;
+    for (int i = 0; i < 3; ++i) {
+        double sum = 0.0;
+        for (int j = 0; j < 3; ++j) {
+            double row = 0.0;
+            for (int k = 0; k < 3; ++k) row += std::fabs((double)lfw[4 * j + k]);
+            sum += std::fabs((double)wfl[4 * i + j]) * row;
+        }
+        if (!(sum <= 4.0)) return false;
+        worst = std::max(worst, sum);
+    }
+    return std::isfinite(worst);
+}
 
 static lux_status prepare_scene(const uint32_t *sw, size_t sn, const uint32_t *gw, size_t gn, const LuxLight *lights,
                                 uint32_t light_count, uint32_t conventional, HostScene &H, std::string &message) {
@@ -405,9 +532,9 @@ static lux_status prepare_scene(const uint32_t *sw, size_t sn, const uint32_t *g
         inst[i].flags = w[4 * 6 + 3];
         uint32_t material = w[4 * 7 + 3];
         inst[i].first = w[4 * 8 + 1];
-        inst[i].count = w[4 * 8 + 2];
+        const uint32_t inst_tris = w[4 * 8 + 2];
         inst[i].root = w[4 * 8 + 0];
-        if ((uint64_t)inst[i].first + inst[i].count > tri_capacity)
+        if ((uint64_t)inst[i].first + inst_tris > tri_capacity)
             return fail(LUX_ERR_MALFORMED_SCENE, "scene upload: instance triangle range outside geometry");
         if (inst[i].root >= node_count)
             return fail(LUX_ERR_MALFORMED_SCENE, "scene upload: instance BLAS root outside the node words");
@@ -424,7 +551,10 @@ static lux_status prepare_scene(const uint32_t *sw, size_t sn, const uint32_t *g
             m[4 * 7] != lux::kEmpty)
             return fail(LUX_ERR_MALFORMED_SCENE,
                             "scene upload: textured materials are not supported by this build");
-        tri_count = std::max(tri_count, inst[i].first + inst[i].count);
+        tri_count = std::max(tri_count, inst[i].first + inst_tris);
+        const BinNode &box = bin[inst[i].root];
+        for (int r = 0; r < 3; ++r)
+            inst[i].extent = std::max({inst[i].extent, std::fabs(box.mn[r]), std::fabs(box.mx[r])});
     }
     // World box of every instance: the eight corners of its BLAS root box
     // through world_from_local (instance rows 3-5) in f64, padded by 2^-17
@@ -497,16 +627,48 @@ static lux_status prepare_scene(const uint32_t *sw, size_t sn, const uint32_t *g
         depth_start.push_back((uint32_t)refit_order.size());
     }
     uint32_t tlas_slots = (uint32_t)slot_source.size();
-    std::unordered_map<uint32_t, uint32_t> blas_root;
+    H.flat_tlas = (uint32_t)nodes.size();
+    struct Blas {
+        uint32_t root, node0, nodes, leaves, depth;
+    };
+    std::unordered_map<uint32_t, Blas> blas_root;
+    std::vector<uint4> &flat = H.flat_inst;
+    uint64_t flat_nodes = H.flat_tlas, flat_leaves = 0;
+    bool flat_ok = inst_count > 0;
+    const uint32_t tlas_depth = inst_count ? tree_depth(nodes, tlas_root) : 0u;
+    for (uint32_t k = 0; k < H.flat_tlas && flat_ok; ++k)  // leaves of several instances have no single root
+        for (uint32_t c : nodes[k].child) flat_ok = flat_ok && (c == lux::kEmpty || !(c & kLeafBit) || ((c >> 27) & 15u) == 0u);
     for (uint32_t i = 0; i < inst_count; ++i) {
         auto it = blas_root.find(inst[i].root);
         if (it == blas_root.end()) {
             Collapser bl{bin, nodes, {}, tri_count, nullptr, nullptr, &seen};
+            const uint32_t node0 = (uint32_t)nodes.size();
             uint32_t r = bl.root(inst[i].root);
             if (!bl.error.empty()) return fail(LUX_ERR_MALFORMED_SCENE, "scene upload (BLAS): " + bl.error);
-            it = blas_root.emplace(inst[i].root, r).first;
+            uint32_t leaves = 0;
+            for (size_t k = node0; k < nodes.size(); ++k)
+                for (int c = 0; c < 4; ++c)
+                    if (nodes[k].child[c] != lux::kEmpty && (nodes[k].child[c] & kLeafBit)) nodes[k].leaf[c] = leaves++;
+            const uint32_t depth = tree_depth(nodes, r);
+            it = blas_root.emplace(inst[i].root, Blas{r, node0, (uint32_t)nodes.size() - node0, leaves, depth}).first;
         }
-        inst[i].root = it->second;
+        const Blas &b = it->second;
+        inst[i].root = b.root;
+        if (!flat_ok) continue;
+        const uint32_t *w = sw + 4 * (size_t)(inst_base + 9 * i);
+        float lfw[12], wfl[12];
+        std::memcpy(lfw, w, sizeof lfw);
+        std::memcpy(wfl, w + 12, sizeof wfl);
+        if (flat.empty()) flat.reserve(inst_count);
+        flat.push_back(make_uint4((uint32_t)flat_nodes, (uint32_t)flat_leaves, b.node0, b.root));
+        flat_nodes += b.nodes;
+        flat_leaves += b.leaves;
+        flat_ok = flat_nodes <= kFlatMaxNodes && flat_leaves <= kLeafFirstMask &&
+                  3u * (tlas_depth + b.depth) <= (uint32_t)lux::kFlatStack && flat_conditioned(lfw, wfl);
+    }
+    if (flat_ok) {
+        H.flat_count = (uint32_t)flat_nodes;
+        H.flat_leaves = (uint32_t)flat_leaves;
     }
     // Triangle positions in packed (leaf) order.
     std::vector<float4> &tris = H.tris;
@@ -549,6 +711,35 @@ extern "C" lux_status lux_scene_validate(const uint32_t *sw, size_t sn, const ui
         message[n] = '\0';
     }
     return status;
+}
+
+static void flat_free(LuxScene *S) {
+    cudaFree(S->d_flat_inst);
+    cudaFree(S->d_flat_nodes);
+    cudaFree(S->d_flat_leaves);
+    S->d_flat_inst = nullptr;
+    S->d_flat_nodes = nullptr;
+    S->d_flat_leaves = nullptr;
+    S->flat_count = 0;
+}
+
+// Rebuilds the flattened tree from the scene's current words (on the context
+// stream); `conditioned`: every pose allows it, else the view falls back to
+// the two-level walk until a later refit does.
+static lux_status flatten(LuxScene *S, bool conditioned) {
+    SceneView &V = S->view;
+    V.flat_nodes = nullptr;
+    V.flat_leaves = nullptr;
+    if (!S->flat_count || !conditioned) return LUX_OK;
+    const uint32_t blocks = std::min<uint32_t>((S->flat_count * 4u + 255u) / 256u, (uint32_t)S->ctx->sm_count * 8u);
+    flatten_kernel<<<blocks, 256, 0, S->ctx->stream>>>(V.scene_words, S->instance_base, V.nodes, S->d_flat_inst,
+                                                       V.instance_count, S->flat_tlas, S->flat_count, S->d_flat_nodes,
+                                                       S->d_flat_leaves);
+    V.flat_nodes = S->d_flat_nodes;
+    V.flat_leaves = S->d_flat_leaves;
+    V.flat_inst = S->d_flat_inst;
+    V.flat_tlas = S->flat_tlas;
+    return lux_cuda_check(S->ctx, (int)cudaGetLastError(), "scene: flatten launch");
 }
 
 extern "C" lux_status lux_scene_upload(LuxContext *ctx, const uint32_t *sw, size_t sn, const uint32_t *gw, size_t gn,
@@ -610,6 +801,20 @@ extern "C" lux_status lux_scene_upload(LuxContext *ctx, const uint32_t *sw, size
         V.root_lo[k] = root_lo[k];
         V.root_hi[k] = root_hi[k];
     }
+    if (H.flat_count) {
+        // Without room for it the scene keeps the two-level walk.
+        if (cudaMalloc((void **)&S->d_flat_inst, H.flat_inst.size() * sizeof(uint4)) == cudaSuccess &&
+            cudaMalloc((void **)&S->d_flat_nodes, (size_t)H.flat_count * sizeof(Bvh4Node)) == cudaSuccess &&
+            cudaMalloc((void **)&S->d_flat_leaves, std::max<size_t>(H.flat_leaves, 1) * sizeof(uint2)) == cudaSuccess &&
+            cudaMemcpy(S->d_flat_inst, H.flat_inst.data(), H.flat_inst.size() * sizeof(uint4),
+                       cudaMemcpyHostToDevice) == cudaSuccess) {
+            S->flat_count = H.flat_count;
+            S->flat_tlas = H.flat_tlas;
+        } else {
+            cudaGetLastError();
+            flat_free(S);
+        }
+    }
     S->node_count = (uint32_t)nodes.size();
     S->instance_base = inst_base;
     S->instance_words.assign(sw + 4 * (size_t)inst_base, sw + 4 * ((size_t)inst_base + 9 * (size_t)inst_count));
@@ -617,6 +822,15 @@ extern "C" lux_status lux_scene_upload(LuxContext *ctx, const uint32_t *sw, size
     S->depth_start = depth_start;
     S->slot_count = tlas_slots;
     S->light_count = light_count;
+    if (S->flat_count) {
+        lux_status rc = lux_cuda_check(ctx, (int)cudaStreamSynchronize(nullptr), "scene upload");  // the copies above
+        if (rc == LUX_OK) rc = flatten(S, true);
+        if (rc == LUX_OK) rc = lux_cuda_check(ctx, (int)cudaStreamSynchronize(ctx->stream), "scene upload");
+        if (rc != LUX_OK) {
+            lux_scene_destroy(S);
+            return rc;
+        }
+    }
     *out = S;
     return LUX_OK;
 }
@@ -632,6 +846,7 @@ extern "C" lux_status lux_scene_destroy(LuxScene *S) {
     cudaFree(S->d_refit_order);
     cudaFree(S->d_depth_start);
     cudaFree(S->d_slot_source);
+    flat_free(S);
     delete S;
     return LUX_OK;
 }
@@ -664,6 +879,7 @@ extern "C" lux_status lux_scene_refit(LuxScene *S, const float *wfl, uint32_t co
     // Host half: instance rows 0-5 and the device instances' local_from_world.
     std::vector<uint32_t> words = S->instance_words;
     std::vector<DeviceInstance> inst = S->instances;
+    bool conditioned = true;
     for (uint32_t i = 0; i < n; ++i) {
         const float *m = wfl + 12 * (size_t)i;
         for (int k = 0; k < 12; ++k)
@@ -679,6 +895,7 @@ extern "C" lux_status lux_scene_refit(LuxScene *S, const float *wfl, uint32_t co
         }
         for (int r = 0; r < 3; ++r)
             for (int c = 0; c < 4; ++c) inst[i].row[r][c] = lfw[4 * r + c];
+        if (S->flat_count) conditioned = conditioned && flat_conditioned(lfw, m);
     }
     cudaStream_t st = ctx->stream;
     cudaSetDevice(ctx->device);
@@ -703,6 +920,7 @@ extern "C" lux_status lux_scene_refit(LuxScene *S, const float *wfl, uint32_t co
         refit_kernel<<<1, 1024, 0, st>>>(sw, S->instance_base, S->d_refit_order, S->d_depth_start, depths,
                                          (Bvh4Node *)S->d_nodes, S->d_slot_source, S->slot_count);
         rc = lux_cuda_check(ctx, (int)cudaGetLastError(), "scene refit: launch");
+        if (rc == LUX_OK) rc = flatten(S, conditioned);
         if (rc != LUX_OK) return rc;
     }
     // The pageable copies above may return before the transfer completes;
@@ -732,7 +950,10 @@ lux_status lux_launch_trace_rays(LuxContext *ctx, const LuxScene *scene, const L
     if (count == 0) return LUX_OK;
     uint32_t block = 128;
     uint32_t grid = (count + block - 1) / block;
-    trace_rays_kernel<<<grid, block, 0, ctx->stream>>>(scene->view, rays, count, any_hit, hits, counters);
+    const bool flat = scene->view.flat_nodes != nullptr;
+    auto kernel = any_hit ? (flat ? trace_rays_kernel<true, true> : trace_rays_kernel<true, false>)
+                          : (flat ? trace_rays_kernel<false, true> : trace_rays_kernel<false, false>);
+    kernel<<<grid, block, 0, ctx->stream>>>(scene->view, rays, count, hits, counters);
     return lux_cuda_check(ctx, (int)cudaGetLastError(), "trace_rays_kernel launch");
 }
 

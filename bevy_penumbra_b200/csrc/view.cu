@@ -45,6 +45,15 @@
 #ifndef LUX_SHADOW_MIN_BLOCKS
 #define LUX_SHADOW_MIN_BLOCKS 7
 #endif
+// The same over the flattened tree, whose walk needs fewer registers: 7
+// resident blocks (72 registers) for closest hits, 8 (64) for visibility, where
+// only a few words spill (6 and 7 blocks: 1.3% slower frame; 8 and 10: 4%).
+#ifndef LUX_FLAT_CLOSEST_MIN_BLOCKS
+#define LUX_FLAT_CLOSEST_MIN_BLOCKS 7
+#endif
+#ifndef LUX_FLAT_SHADOW_MIN_BLOCKS
+#define LUX_FLAT_SHADOW_MIN_BLOCKS 8
+#endif
 // The batched trace kernels keep a job's scene pointers per warp as well.
 #ifndef LUX_BATCH_MIN_BLOCKS
 #define LUX_BATCH_MIN_BLOCKS 6
@@ -88,11 +97,6 @@
 // registers with a few spills measured faster than 112 without.
 #ifndef LUX_SHADE_MIN_BLOCKS
 #define LUX_SHADE_MIN_BLOCKS 6
-#endif
-// Whole-warp traversal in the persistent trace kernels: the BLAS leaves the
-// lanes reach in a step are tested by the whole warp.
-#ifndef LUX_WARP_LEAVES
-#define LUX_WARP_LEAVES 1
 #endif
 // The fused batch trace kernel carries the shading phase's registers too.
 #ifndef LUX_FUSED_MIN_BLOCKS
@@ -534,84 +538,63 @@ __device__ __forceinline__ void load_ray(const ViewDevice &V, uint32_t ray, f3 &
     h.b2 = lux::as_float(c.w);
 }
 
-// Persistent warps with per-lane refill (lux::trace_persistent).
+// Persistent warps with per-lane refill (lux::trace_refill).
 __global__ void __launch_bounds__(128, LUX_REFILL_MIN_BLOCKS) closest_split_refill_kernel(ViewDevice V, FrameParams F, SceneView S,
                                                             const float4 *__restrict__ pos,
                                                             const float4 *__restrict__ nrm, uint32_t ray_count) {
     if (*V.error_flags) return;
-#if LUX_WARP_LEAVES
     __shared__ lux::LeafScratch scratch[4];
     lux::LeafScratch *L = &scratch[threadIdx.x >> 5];
-#else
-    lux::LeafScratch *L = nullptr;
-#endif
     unsigned long long st[7] = {0, 0, 0, 0, 0, 0, 0};
     lux::TraceCounters cn{0, 0, 0};
-    lux::trace_persistent<false>(
-        S, &V.ts.work_counter[0], ray_count,
-        [&](uint32_t slot, f3 &o, f3 &d, float &tmin, float &limit) {
-            uint32_t ray = V.ray_order ? V.ray_order[slot] : slot;
-            uint32_t i = ray / F.rays_per_receiver, k = ray % F.rays_per_receiver;
-            float4 p4 = pos[i], n4 = nrm[i];
-            f3 p{p4.x, p4.y, p4.z}, n{n4.x, n4.y, n4.z};
-            float u, v;
-            split_direction(V, F, F.shade.frame, i, k, n, d, u, v);
-            o = lux::ray_offset(p, n, F.shade.normal_bias);
-            tmin = 0.0f;
-            limit = 1e20f;
-            V.ts.ray_o[ray] = make_float4(o.x, o.y, o.z, 0.0f);
-            V.ts.ray_d[ray] = make_float4(d.x, d.y, d.z, 0.0f);
-        },
-        [&](uint32_t slot, const lux::Hit &h) {
-            uint32_t ray = V.ray_order ? V.ray_order[slot] : slot;
-            V.ts.ray_o[ray].w = h.t;
-            V.ts.ray_d[ray].w = h.b1;
-            V.ts.ray_h[ray] = make_uint4(h.tri, h.inst, h.errors, lux::as_uint(h.b2));
-            st[kStatInterval] += 1;
-        },
-        cn, L);
+    auto gen = [&](uint32_t slot, f3 &o, f3 &d, float &tmin, float &limit) {
+        uint32_t ray = V.ray_order ? V.ray_order[slot] : slot;
+        uint32_t i = ray / F.rays_per_receiver, k = ray % F.rays_per_receiver;
+        float4 p4 = pos[i], n4 = nrm[i];
+        f3 p{p4.x, p4.y, p4.z}, n{n4.x, n4.y, n4.z};
+        float u, v;
+        split_direction(V, F, F.shade.frame, i, k, n, d, u, v);
+        o = lux::ray_offset(p, n, F.shade.normal_bias);
+        tmin = 0.0f;
+        limit = 1e20f;
+        V.ts.ray_o[ray] = make_float4(o.x, o.y, o.z, 0.0f);
+        V.ts.ray_d[ray] = make_float4(d.x, d.y, d.z, 0.0f);
+    };
+    auto done = [&](uint32_t slot, const lux::Hit &h) {
+        uint32_t ray = V.ray_order ? V.ray_order[slot] : slot;
+        V.ts.ray_o[ray].w = h.t;
+        V.ts.ray_d[ray].w = h.b1;
+        V.ts.ray_h[ray] = make_uint4(h.tri, h.inst, h.errors, lux::as_uint(h.b2));
+        st[kStatInterval] += 1;
+    };
+    lux::trace_refill<false>(S, &V.ts.work_counter[0], ray_count, gen, done, cn, L);
     st[kStatNodes] = cn.nodes;
     st[kStatTris] = cn.triangles;
     st[kStatInst] = cn.instances;
     add_stats(V.stats, st);
 }
 
-// One Split interval ray (traceTransport, shaders/split.slang:1122-1163):
-// receiver i = ray / R, sample k = ray % R, from the biased receiver position
-// to 1e20; the hit is stored for shading.
-// Returns false for the rays of an absent receiver of a sparse set (stored
-// as unsupported, not traced).
-template <int kDepth = lux::kStack>
-__device__ __forceinline__ bool closest_split_ray(const ViewDevice &V, const FrameParams &F, uint32_t frame,
-                                                  const SceneView &S, const float4 *__restrict__ pos,
-                                                  const float4 *__restrict__ nrm, uint32_t slot,
-                                                  lux::TraceCounters &cn) {
-    uint32_t ray = V.ray_order ? V.ray_order[slot] : slot;
-    uint32_t i = ray / F.rays_per_receiver, k = ray % F.rays_per_receiver;
-    float4 p4 = pos[i], n4 = nrm[i];
-    if (F.sparse && p4.w == 0.0f) {
-        lux::Hit none;
-        none.t = 0.0f;
-        none.b1 = none.b2 = 0.0f;
-        none.tri = none.inst = lux::kEmpty;
-        none.errors = lux::kQueryUnsupported;
-        store_ray(V, ray, f3{0.0f, 0.0f, 0.0f}, f3{0.0f, 0.0f, 0.0f}, none);
-        return false;
-    }
-    f3 p{p4.x, p4.y, p4.z}, n{n4.x, n4.y, n4.z};
-    f3 dir;
-    float u, v;
-    split_direction(V, F, frame, i, k, n, dir, u, v);
-    f3 origin = lux::ray_offset(p, n, F.shade.normal_bias);
+// The closest hits of a warp's rays, stored for shading (every lane calls it;
+// active: the lane has ray `ray`).  kFlat: over the flattened tree, which takes
+// no stack depth.
+template <int kDepth, bool kFlat>
+__device__ __forceinline__ void closest_ray_warp(const ViewDevice &V, const SceneView &S, uint32_t ray, bool active,
+                                                 f3 origin, f3 dir, float tmin, float limit, lux::TraceCounters &cn,
+                                                 lux::LeafScratch *L) {
     lux::Hit hit;
-    lux::trace<false, kDepth>(S, origin, dir, 0.0f, 1e20f, hit, cn);
-    store_ray(V, ray, origin, dir, hit);
-    return true;
+    if (kFlat)
+        lux::trace_warp_flat<false>(S, active, origin, dir, tmin, limit, hit, cn, L);
+    else
+        lux::trace_warp<false, kDepth>(S, active, origin, dir, tmin, limit, hit, cn, L);
+    if (active) store_ray(V, ray, origin, dir, hit);
 }
 
-// closest_split_ray for a whole warp (every lane calls it; `valid`: the
-// lane has a slot), with the warp's leaves tested together.
-template <int kDepth = lux::kStack>
+// Split interval rays (traceTransport, shaders/split.slang:1122-1163) of a
+// whole warp (every lane calls it; `valid`: the lane has a slot): receiver i =
+// ray / R, sample k = ray % R, from the biased receiver position to 1e20; the
+// hit is stored for shading.  Returns false for the rays of an absent
+// receiver of a sparse set (stored as unsupported, not traced).
+template <int kDepth, bool kFlat>
 __device__ __forceinline__ bool closest_split_ray_warp(const ViewDevice &V, const FrameParams &F, uint32_t frame,
                                                        const SceneView &S, const float4 *__restrict__ pos,
                                                        const float4 *__restrict__ nrm, uint32_t slot, bool valid,
@@ -638,9 +621,7 @@ __device__ __forceinline__ bool closest_split_ray_warp(const ViewDevice &V, cons
             origin = lux::ray_offset(p, n, F.shade.normal_bias);
         }
     }
-    lux::Hit hit;
-    lux::trace_warp<false, kDepth>(S, active, origin, dir, 0.0f, 1e20f, hit, cn, L);
-    if (active) store_ray(V, ray, origin, dir, hit);
+    closest_ray_warp<kDepth, kFlat>(V, S, ray, active, origin, dir, 0.0f, 1e20f, cn, L);
     return active;
 }
 
@@ -652,70 +633,73 @@ __device__ __forceinline__ uint32_t warp_fetch(uint32_t *counter, uint32_t tile 
     return __shfl_sync(0xffffffffu, base, 0);
 }
 
-template <int kDepth>
-__global__ void __launch_bounds__(128, LUX_CLOSEST_MIN_BLOCKS) closest_split_kernel(ViewDevice V, FrameParams F, SceneView S,
+template <int kDepth, bool kFlat>
+__global__ void __launch_bounds__(128, kFlat ? LUX_FLAT_CLOSEST_MIN_BLOCKS : LUX_CLOSEST_MIN_BLOCKS)
+    closest_split_kernel(ViewDevice V, FrameParams F, const __grid_constant__ SceneView S,
                                                             const float4 *__restrict__ pos,
                                                             const float4 *__restrict__ nrm, uint32_t ray_count,
                                                             uint32_t tile) {
     if (*V.error_flags) return;
-#if LUX_WARP_LEAVES
     __shared__ lux::LeafScratch scratch[4];
     lux::LeafScratch *L = &scratch[threadIdx.x >> 5];
-#endif
-    unsigned long long st[7] = {0, 0, 0, 0, 0, 0, 0};
+    uint32_t traced = 0;
     lux::TraceCounters cn{0, 0, 0};
     while (true) {
         uint32_t base = warp_fetch(&V.ts.work_counter[0], tile);
         if (base >= ray_count) break;
         for (uint32_t k = 0; k < tile && base + k < ray_count; k += 32u) {
             uint32_t slot = base + k + (threadIdx.x & 31u);
-#if LUX_WARP_LEAVES
-            if (closest_split_ray_warp<kDepth>(V, F, F.shade.frame, S, pos, nrm, slot, slot < ray_count, cn, L))
-                st[kStatInterval] += 1;
-#else
-            if (slot < ray_count && closest_split_ray<kDepth>(V, F, F.shade.frame, S, pos, nrm, slot, cn))
-                st[kStatInterval] += 1;
-#endif
+            if (closest_split_ray_warp<kDepth, kFlat>(V, F, F.shade.frame, S, pos, nrm, slot, slot < ray_count, cn, L))
+                ++traced;
         }
     }
+    unsigned long long st[7] = {0, 0, 0, 0, 0, 0, 0};
+    st[kStatInterval] = traced;
     st[kStatNodes] = cn.nodes;
     st[kStatTris] = cn.triangles;
     st[kStatInst] = cn.instances;
     add_stats(V.stats, st);
 }
 
-// Dense layout: one ray per (cell, direction) record of one level; the ray
+// Dense layout: one ray per (cell, direction) record of every level; the ray
 // starts at the cell centre and covers the level's interval (the dense
 // reference of src/transport_tests.rs:179-248 with BVH geometry).  The ray
-// index is the record index.
-__global__ void __launch_bounds__(128, LUX_CLOSEST_MIN_BLOCKS) closest_dense_kernel(ViewDevice V, FrameParams F, SceneView S, uint32_t level) {
+// index is the record index, so one launch takes all levels.
+template <bool kFlat>
+__global__ void __launch_bounds__(128, kFlat ? LUX_FLAT_CLOSEST_MIN_BLOCKS : LUX_CLOSEST_MIN_BLOCKS)
+    closest_dense_kernel(ViewDevice V, FrameParams F, const __grid_constant__ SceneView S) {
     if (*V.error_flags) return;
-    unsigned long long n = (unsigned long long)V.cell_count[level] * F.dirs[level];
-    unsigned long long base = V.level_base[level];
-    const bool terminal = level + 1u == F.levels;
-    const float tmin = F.start[level];
-    const float limit = terminal ? 1e20f : nextafterf(F.end[level], INFINITY);
-    const float sp = F.spacing[level];
-    const uint32_t dirs = F.dirs[level];
+    __shared__ lux::LeafScratch scratch[4];
+    lux::LeafScratch *L = &scratch[threadIdx.x >> 5];
+    const unsigned long long n = total_entries(V, F);
+    uint32_t traced = 0;
+    lux::TraceCounters cn{0, 0, 0};
     for (unsigned long long e = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
          e < ((n + 31ull) & ~31ull); e += (unsigned long long)gridDim.x * blockDim.x) {
-        unsigned long long st[7] = {0, 0, 0, 0, 0, 0, 0};
-        if (e < n) {
-            uint32_t cell = (uint32_t)(e / dirs), d = (uint32_t)(e % dirs);
+        const bool active = e < n;
+        f3 origin{0.0f, 0.0f, 0.0f}, dir{0.0f, 0.0f, 0.0f};
+        float tmin = 0.0f, limit = 0.0f;
+        if (active) {
+            uint32_t level = 0;
+            while (level + 1u < F.levels && e >= V.level_base[level + 1u]) ++level;
+            const uint32_t r = (uint32_t)(e - V.level_base[level]), dirs = F.dirs[level];
+            const uint32_t cell = r / dirs, d = r % dirs;
+            const float sp = F.spacing[level];
             int4 key = V.cell_keys[(size_t)level * F.cell_capacity + cell];
-            f3 origin{((float)key.x + 0.5f) * sp, ((float)key.y + 0.5f) * sp, ((float)key.z + 0.5f) * sp};
-            f3 dir = lux::bin_direction(d, F.columns[level], F.rows[level]);
-            lux::TraceCounters cn{0, 0, 0};
-            lux::Hit hit;
-            lux::trace<false>(S, origin, dir, tmin, limit, hit, cn);
-            store_ray(V, (uint32_t)(base + e), origin, dir, hit);
-            st[kStatInterval] = 1;
-            st[kStatNodes] = cn.nodes;
-            st[kStatTris] = cn.triangles;
-            st[kStatInst] = cn.instances;
+            origin = f3{((float)key.x + 0.5f) * sp, ((float)key.y + 0.5f) * sp, ((float)key.z + 0.5f) * sp};
+            dir = lux::bin_direction(d, F.columns[level], F.rows[level]);
+            tmin = F.start[level];
+            limit = level + 1u == F.levels ? 1e20f : nextafterf(F.end[level], INFINITY);
+            ++traced;
         }
-        add_stats(V.stats, st);
+        closest_ray_warp<lux::kStack, kFlat>(V, S, (uint32_t)e, active, origin, dir, tmin, limit, cn, L);
     }
+    unsigned long long st[7] = {0, 0, 0, 0, 0, 0, 0};
+    st[kStatInterval] = traced;
+    st[kStatNodes] = cn.nodes;
+    st[kStatTris] = cn.triangles;
+    st[kStatInst] = cn.instances;
+    add_stats(V.stats, st);
 }
 
 // Coherence keys of split interval rays: (direction bin of an 8 x 4 grid,
@@ -840,31 +824,25 @@ __global__ void __launch_bounds__(128, LUX_SHADE_MIN_BLOCKS) shade_kernel(ViewDe
 // result: 0 visible, 1 blocked, 2 unsupported.
 __global__ void __launch_bounds__(128, LUX_REFILL_MIN_BLOCKS) shadow_refill_kernel(ViewDevice V, FrameParams F, SceneView S) {
     if (*V.error_flags) return;
-#if LUX_WARP_LEAVES
     __shared__ lux::LeafScratch scratch[4];
     lux::LeafScratch *L = &scratch[threadIdx.x >> 5];
-#else
-    lux::LeafScratch *L = nullptr;
-#endif
     uint32_t n = min(*V.ts.queue_count, F.queue_capacity);
     unsigned long long st[7] = {0, 0, 0, 0, 0, 0, 0};
     lux::TraceCounters cn{0, 0, 0};
-    lux::trace_persistent<true>(
-        S, &V.ts.work_counter[1], n,
-        [&](uint32_t i, f3 &o, f3 &d, float &tmin, float &limit) {
-            uint32_t qi = V.ts.query_slot[V.query_order ? V.query_order[i] : i];
-            float4 a = V.ts.queue_o[qi], b = V.ts.queue_d[qi];
-            o = f3{a.x, a.y, a.z};
-            d = f3{b.x, b.y, b.z};
-            tmin = 0.0f;
-            limit = a.w;
-        },
-        [&](uint32_t i, const lux::Hit &sh) {
-            uint32_t qi = V.ts.query_slot[V.query_order ? V.query_order[i] : i];
-            V.ts.queue_result[qi] = sh.tri != lux::kEmpty ? 1 : ((sh.errors & lux::kQueryUnsupported) ? 2 : 0);
-            st[kStatShadow] += 1;
-        },
-        cn, L);
+    auto gen = [&](uint32_t i, f3 &o, f3 &d, float &tmin, float &limit) {
+        uint32_t qi = V.ts.query_slot[V.query_order ? V.query_order[i] : i];
+        float4 a = V.ts.queue_o[qi], b = V.ts.queue_d[qi];
+        o = f3{a.x, a.y, a.z};
+        d = f3{b.x, b.y, b.z};
+        tmin = 0.0f;
+        limit = a.w;
+    };
+    auto done = [&](uint32_t i, const lux::Hit &sh) {
+        uint32_t qi = V.ts.query_slot[V.query_order ? V.query_order[i] : i];
+        V.ts.queue_result[qi] = sh.tri != lux::kEmpty ? 1 : ((sh.errors & lux::kQueryUnsupported) ? 2 : 0);
+        st[kStatShadow] += 1;
+    };
+    lux::trace_refill<true>(S, &V.ts.work_counter[1], n, gen, done, cn, L);
     st[kStatNodes] = cn.nodes;
     st[kStatTris] = cn.triangles;
     st[kStatInst] = cn.instances;
@@ -872,21 +850,10 @@ __global__ void __launch_bounds__(128, LUX_REFILL_MIN_BLOCKS) shadow_refill_kern
     add_stats(V.stats, st, extra);
 }
 
-// One visibility query (traceVisibility, shaders/split.slang:1326-1339):
-// result 0 visible, 1 blocked, 2 unsupported.
-template <int kDepth = lux::kStack>
-__device__ __forceinline__ void shadow_query(const ViewDevice &V, const SceneView &S, uint32_t i,
-                                             lux::TraceCounters &cn) {
-    uint32_t qi = V.ts.query_slot[V.query_order ? V.query_order[i] : i];
-    float4 a = V.ts.queue_o[qi], b = V.ts.queue_d[qi];
-    lux::Hit sh;
-    lux::trace<true, kDepth>(S, f3{a.x, a.y, a.z}, f3{b.x, b.y, b.z}, 0.0f, a.w, sh, cn);
-    V.ts.queue_result[qi] = sh.tri != lux::kEmpty ? 1 : ((sh.errors & lux::kQueryUnsupported) ? 2 : 0);
-}
-
-// shadow_query for a whole warp (every lane calls it; `valid`: the lane has
-// a query).
-template <int kDepth = lux::kStack>
+// A warp's visibility queries (traceVisibility, shaders/split.slang:1326-1339;
+// every lane calls it; `valid`: the lane has a query): result 0 visible, 1
+// blocked, 2 unsupported.
+template <int kDepth, bool kFlat>
 __device__ __forceinline__ void shadow_query_warp(const ViewDevice &V, const SceneView &S, uint32_t i, bool valid,
                                                   lux::TraceCounters &cn, lux::LeafScratch *L) {
     uint32_t qi = 0;
@@ -897,37 +864,34 @@ __device__ __forceinline__ void shadow_query_warp(const ViewDevice &V, const Sce
         b = V.ts.queue_d[qi];
     }
     lux::Hit sh;
-    lux::trace_warp<true, kDepth>(S, valid, f3{a.x, a.y, a.z}, f3{b.x, b.y, b.z}, 0.0f, a.w, sh, cn, L);
+    if (kFlat)
+        lux::trace_warp_flat<true>(S, valid, f3{a.x, a.y, a.z}, f3{b.x, b.y, b.z}, 0.0f, a.w, sh, cn, L);
+    else
+        lux::trace_warp<true, kDepth>(S, valid, f3{a.x, a.y, a.z}, f3{b.x, b.y, b.z}, 0.0f, a.w, sh, cn, L);
     if (valid) V.ts.queue_result[qi] = sh.tri != lux::kEmpty ? 1 : ((sh.errors & lux::kQueryUnsupported) ? 2 : 0);
 }
 
-template <int kDepth>
-__global__ void __launch_bounds__(128, LUX_SHADOW_MIN_BLOCKS) shadow_kernel(ViewDevice V, FrameParams F, SceneView S,
+template <int kDepth, bool kFlat>
+__global__ void __launch_bounds__(128, kFlat ? LUX_FLAT_SHADOW_MIN_BLOCKS : LUX_SHADOW_MIN_BLOCKS)
+    shadow_kernel(ViewDevice V, FrameParams F, const __grid_constant__ SceneView S,
                                                                              uint32_t tile) {
     if (*V.error_flags) return;
-#if LUX_WARP_LEAVES
     __shared__ lux::LeafScratch scratch[4];
     lux::LeafScratch *L = &scratch[threadIdx.x >> 5];
-#endif
     uint32_t n = min(*V.ts.queue_count, F.queue_capacity);
-    unsigned long long st[7] = {0, 0, 0, 0, 0, 0, 0};
+    uint32_t traced = 0;
     lux::TraceCounters cn{0, 0, 0};
     while (true) {
         uint32_t base = warp_fetch(&V.ts.work_counter[1], tile);
         if (base >= n) break;
         for (uint32_t k = 0; k < tile && base + k < n; k += 32u) {
             uint32_t i = base + k + (threadIdx.x & 31u);
-#if LUX_WARP_LEAVES
-            shadow_query_warp<kDepth>(V, S, i, i < n, cn, L);
-            if (i < n) st[kStatShadow] += 1;
-#else
-            if (i < n) {
-                shadow_query<kDepth>(V, S, i, cn);
-                st[kStatShadow] += 1;
-            }
-#endif
+            shadow_query_warp<kDepth, kFlat>(V, S, i, i < n, cn, L);
+            if (i < n) ++traced;
         }
     }
+    unsigned long long st[7] = {0, 0, 0, 0, 0, 0, 0};
+    st[kStatShadow] = traced;
     st[kStatNodes] = cn.nodes;
     st[kStatTris] = cn.triangles;
     st[kStatInst] = cn.instances;
@@ -1886,6 +1850,7 @@ __device__ __forceinline__ void flush_stats(unsigned long long *stats, unsigned 
 // The four trace phases over all jobs' rays and queries; each is a kernel of
 // its own or one phase of trace_batch_kernel.
 // A tile of `tile` rays may span jobs: the job is found per 32-ray chunk.
+template <bool kFlat>
 __device__ __forceinline__ void closest_batch_phase(const BatchJob *__restrict__ jobs,
                                                     const uint32_t *__restrict__ begin, uint32_t n, uint32_t total,
                                                     uint32_t fr, uint32_t *counter, uint32_t tile,
@@ -1906,8 +1871,7 @@ __device__ __forceinline__ void closest_batch_phase(const BatchJob *__restrict__
             }
             if (__shfl_sync(0xffffffffu, *J.V.error_flags, 0)) continue;  // one value for the warp
             uint32_t slot = base - __ldg(begin + j) + lane;
-            SceneView S = J.S;
-            closest_split_ray_warp(J.V, J.F, fr, S, J.pos, J.nrm, slot, slot < J.rays, cn, L);
+            closest_split_ray_warp<lux::kStack, kFlat>(J.V, J.F, fr, J.S, J.pos, J.nrm, slot, slot < J.rays, cn, L);
             if (slot < J.rays) st[kStatInterval] += 1;
         }
     }
@@ -1981,6 +1945,7 @@ __device__ __forceinline__ uint32_t find_query_job(const uint32_t *qbegin, uint3
     return lo;
 }
 
+template <bool kFlat>
 __device__ __forceinline__ void shadow_batch_phase(const BatchJob *__restrict__ jobs, const uint32_t *qbegin,
                                                    uint32_t n, uint32_t *counter, uint32_t tile, lux::LeafScratch *L) {
     const uint32_t total = qbegin[n];
@@ -2000,8 +1965,7 @@ __device__ __forceinline__ void shadow_batch_phase(const BatchJob *__restrict__ 
             }
             uint32_t i = base - qbegin[j] + lane;
             const bool valid = i < job_queries(J);
-            SceneView S = J.S;
-            shadow_query_warp(J.V, S, i, valid, cn, L);
+            shadow_query_warp<lux::kStack, kFlat>(J.V, J.S, i, valid, cn, L);
             if (valid) st[kStatShadow] += 1;
         }
     }
@@ -2025,11 +1989,12 @@ __device__ __forceinline__ void deposit_batch_phase(const BatchJob *__restrict__
     }
 }
 
+template <bool kFlat>
 __global__ void __launch_bounds__(128, LUX_BATCH_MIN_BLOCKS)
     closest_batch_kernel(const BatchJob *__restrict__ jobs, const uint32_t *__restrict__ begin, uint32_t n,
                          uint32_t total, const uint32_t *__restrict__ frame, uint32_t *counter, uint32_t tile) {
     __shared__ lux::LeafScratch scratch[4];
-    closest_batch_phase(jobs, begin, n, total, *frame, counter, tile, &scratch[threadIdx.x >> 5]);
+    closest_batch_phase<kFlat>(jobs, begin, n, total, *frame, counter, tile, &scratch[threadIdx.x >> 5]);
 }
 
 __global__ void __launch_bounds__(128, LUX_SHADE_MIN_BLOCKS) shade_batch_kernel(const BatchJob *__restrict__ jobs,
@@ -2043,11 +2008,12 @@ __global__ void __launch_bounds__(128) query_prefix_kernel(const BatchJob *__res
     if (blockIdx.x == 0) query_prefix_block(jobs, n, qbegin);
 }
 
+template <bool kFlat>
 __global__ void __launch_bounds__(128, LUX_BATCH_MIN_BLOCKS)
     shadow_batch_kernel(const BatchJob *__restrict__ jobs, const uint32_t *qbegin, uint32_t n, uint32_t *counter,
                         uint32_t tile) {
     __shared__ lux::LeafScratch scratch[4];
-    shadow_batch_phase(jobs, qbegin, n, counter, tile, &scratch[threadIdx.x >> 5]);
+    shadow_batch_phase<kFlat>(jobs, qbegin, n, counter, tile, &scratch[threadIdx.x >> 5]);
 }
 
 __global__ void __launch_bounds__(128) deposit_batch_kernel(const BatchJob *__restrict__ jobs,
@@ -2113,6 +2079,7 @@ __device__ bool grid_sync(const GridBarrier &B, uint32_t index, const BatchJob *
     return passed != 0u;
 }
 
+template <bool kFlat>
 __global__ void __launch_bounds__(128, LUX_FUSED_MIN_BLOCKS)
     trace_batch_kernel(const BatchJob *__restrict__ jobs, const uint32_t *__restrict__ begin, uint32_t n,
                        uint32_t total, const uint32_t *__restrict__ frame, uint32_t *counters,
@@ -2120,13 +2087,13 @@ __global__ void __launch_bounds__(128, LUX_FUSED_MIN_BLOCKS)
     __shared__ lux::LeafScratch scratch[4];
     lux::LeafScratch *L = &scratch[threadIdx.x >> 5];
     const uint32_t fr = *frame;
-    closest_batch_phase(jobs, begin, n, total, fr, counters, tile, L);
+    closest_batch_phase<kFlat>(jobs, begin, n, total, fr, counters, tile, L);
     if (!grid_sync(B, 1, jobs, n)) return;
     shade_batch_phase(jobs, begin, n, total, fr);
     if (!grid_sync(B, 2, jobs, n)) return;
     if (blockIdx.x == 0) query_prefix_block(jobs, n, qbegin);
     if (!grid_sync(B, 3, jobs, n)) return;
-    shadow_batch_phase(jobs, qbegin, n, counters + 1, tile, L);
+    shadow_batch_phase<kFlat>(jobs, qbegin, n, counters + 1, tile, L);
     if (!grid_sync(B, 4, jobs, n)) return;
     deposit_batch_phase(jobs, begin, n, total, fr);
 }
@@ -2541,8 +2508,9 @@ __device__ __forceinline__ unsigned long long receiver_key(const FrameParams &F,
 // fallback cells, otherwise up to the cutoff; a truncated ray that meets
 // nothing is answered by the cache at level `cutoff` (its stored distance
 // is that level's interval end, so the deposit terminates there).
-__global__ void __launch_bounds__(128, LUX_CLOSEST_MIN_BLOCKS)
-    closest_cache_kernel(ViewDevice V, FrameParams F, SceneView S, const float4 *__restrict__ pos,
+template <bool kFlat>
+__global__ void __launch_bounds__(128, kFlat ? LUX_FLAT_CLOSEST_MIN_BLOCKS : LUX_CLOSEST_MIN_BLOCKS)
+    closest_cache_kernel(ViewDevice V, FrameParams F, const __grid_constant__ SceneView S, const float4 *__restrict__ pos,
                          const float4 *__restrict__ nrm, uint32_t ray_count, CacheDevice C) {
     if (*V.error_flags) return;
     __shared__ lux::LeafScratch scratch[4];
@@ -2571,19 +2539,18 @@ __global__ void __launch_bounds__(128, LUX_CLOSEST_MIN_BLOCKS)
             split_direction(V, F, F.shade.frame, i, k, n, dir, u, v);
             origin = lux::ray_offset(p, n, F.shade.normal_bias);
         }
-        lux::Hit hit;
-        lux::trace_warp<false>(S, active, origin, dir, 0.0f, full ? 1e20f : C.near_limit, hit, cn, L);
+        closest_ray_warp<lux::kStack, kFlat>(V, S, ray, active, origin, dir, 0.0f, full ? 1e20f : C.near_limit, cn, L);
         uint8_t flag = kRayPlain;
         if (active) {
-            if (!full && hit.tri == lux::kEmpty) {
+            const float t = V.ts.ray_o[ray].w;
+            if (!full && V.ts.ray_h[ray].x == lux::kEmpty) {
                 flag = kRayCached;
-                hit.t = C.far_t;
-            } else if (validate && hit.t > F.end[C.cutoff - 1u]) {
+                V.ts.ray_o[ray].w = C.far_t;
+            } else if (validate && t > F.end[C.cutoff - 1u]) {
                 flag = kRayValidated;
             }
             fallback_rays += fallback ? 1u : 0u;
             C.flags[ray] = flag;
-            store_ray(V, ray, origin, dir, hit);
             st[kStatInterval] += 1;
         }
         // The cache query of every cached or validated ray, keyed by its
@@ -3435,6 +3402,7 @@ static lux_status view_frame(LuxView *v, const LuxScene *scene, const LuxSetting
             }
             const bool cached = v->cache_alloc && v->cache.cutoff_level < F.levels;
             CacheDevice C = v->cdev;
+            const bool flat = scene->view.flat_nodes != nullptr;
             if (cached) {
                 C.cutoff = v->cache.cutoff_level;
                 C.period = v->cache.validate_period;
@@ -3446,17 +3414,18 @@ static lux_status view_frame(LuxView *v, const LuxScene *scene, const LuxSetting
                 C.bound = v->cache.error_bound;
                 cudaMemsetAsync(C.counters, 0, kCntCount * 4, st);
                 cudaMemsetAsync(C.global_error, 0, 8, st);
-                closest_cache_kernel<<<ctx->sm_count * T.closest_blocks_per_sm, 128, 0, st>>>(D, F, scene->view, pos,
-                                                                                             nrm, rays, C);
+                (flat ? closest_cache_kernel<true> : closest_cache_kernel<false>)
+                    <<<ctx->sm_count * T.closest_blocks_per_sm, 128, 0, st>>>(D, F, scene->view, pos, nrm, rays, C);
             } else if (T.closest_mode == 1)
                 closest_split_refill_kernel<<<ctx->sm_count * T.closest_blocks_per_sm, 128, 0, st>>>(
                     Dr, F, scene->view, pos, nrm, rays);
-            else if (T.stack_depth == 32)
-                closest_split_kernel<32><<<ctx->sm_count * T.closest_blocks_per_sm, 128, 0, st>>>(
-                    Dr, F, scene->view, pos, nrm, rays, tile_of(T));
-            else
-                closest_split_kernel<64><<<ctx->sm_count * T.closest_blocks_per_sm, 128, 0, st>>>(
-                    Dr, F, scene->view, pos, nrm, rays, tile_of(T));
+            else {
+                auto kernel = flat ? closest_split_kernel<64, true>
+                                   : (T.stack_depth == 32 ? closest_split_kernel<32, false>
+                                                          : closest_split_kernel<64, false>);
+                kernel<<<ctx->sm_count * T.closest_blocks_per_sm, 128, 0, st>>>(Dr, F, scene->view, pos, nrm, rays,
+                                                                                 tile_of(T));
+            }
             if (forked) cudaStreamWaitEvent(st, v->laid_out, 0);  // join the setup stream
             ViewDevice Dq = D;  // query pass view: keys written by shade, optional order
             if (!T.sort_queries) Dq.sort_keys = nullptr;
@@ -3470,12 +3439,11 @@ static lux_status view_frame(LuxView *v, const LuxScene *scene, const LuxSetting
             }
             if (T.shadow_mode == 1)
                 shadow_refill_kernel<<<ctx->sm_count * T.shadow_blocks_per_sm, 128, 0, st>>>(Dq, F, scene->view);
-            else if (T.stack_depth == 32)
-                shadow_kernel<32><<<ctx->sm_count * T.shadow_blocks_per_sm, 128, 0, st>>>(Dq, F, scene->view,
-                                                                                         tile_of(T));
-            else
-                shadow_kernel<64><<<ctx->sm_count * T.shadow_blocks_per_sm, 128, 0, st>>>(Dq, F, scene->view,
-                                                                                         tile_of(T));
+            else {
+                auto kernel = flat ? shadow_kernel<64, true>
+                                   : (T.stack_depth == 32 ? shadow_kernel<32, false> : shadow_kernel<64, false>);
+                kernel<<<ctx->sm_count * T.shadow_blocks_per_sm, 128, 0, st>>>(Dq, F, scene->view, tile_of(T));
+            }
             if (cached) {
                 const int g = ctx->sm_count * 8;
                 lux_status qrc = lux_cache_query_device_count(v->cache.cache, C.queries, C.counters + kCntQueries, rays,
@@ -3495,11 +3463,12 @@ static lux_status view_frame(LuxView *v, const LuxScene *scene, const LuxSetting
             }
         }
     } else {
-        for (uint32_t l = 0; l < F.levels; ++l)
-            closest_dense_kernel<<<ctx->sm_count * 16, 128, 0, st>>>(D, F, scene->view, l);
+        const bool flat = scene->view.flat_nodes != nullptr;
+        (flat ? closest_dense_kernel<true> : closest_dense_kernel<false>)<<<ctx->sm_count * 16, 128, 0, st>>>(
+            D, F, scene->view);
         shade_kernel<<<ctx->sm_count * 16, 128, 0, st>>>(D, F, scene->view, F.ray_capacity, true);
-        shadow_kernel<64><<<ctx->sm_count * v->tuning.shadow_blocks_per_sm, 128, 0, st>>>(D, F, scene->view,
-                                                                                      tile_of(v->tuning));
+        (flat ? shadow_kernel<64, true> : shadow_kernel<64, false>)
+            <<<ctx->sm_count * v->tuning.shadow_blocks_per_sm, 128, 0, st>>>(D, F, scene->view, tile_of(v->tuning));
         deposit_dense_kernel<<<ctx->sm_count * 16, 128, 0, st>>>(D, F);
     }
     mark(2);
@@ -3750,23 +3719,29 @@ __global__ void scratch_clear_kernel(ViewDevice V) {
     if (blockIdx.x == 0 && threadIdx.x < 16) V.stats[threadIdx.x] = 0;
 }
 
-__global__ void __launch_bounds__(128, LUX_CLOSEST_MIN_BLOCKS) closest_rays_kernel(ViewDevice V, SceneView S, const LuxRay *__restrict__ rays,
-                                                           uint32_t count) {
-    unsigned long long st[7] = {0, 0, 0, 0, 0, 0, 0};
+template <bool kFlat>
+__global__ void __launch_bounds__(128, kFlat ? LUX_FLAT_CLOSEST_MIN_BLOCKS : LUX_CLOSEST_MIN_BLOCKS)
+    closest_rays_kernel(ViewDevice V, const __grid_constant__ SceneView S, const LuxRay *__restrict__ rays,
+                        uint32_t count) {
+    __shared__ lux::LeafScratch scratch[4];
+    lux::LeafScratch *L = &scratch[threadIdx.x >> 5];
+    uint32_t traced = 0;
     lux::TraceCounters cn{0, 0, 0};
     while (true) {
         uint32_t base = warp_fetch(&V.ts.work_counter[0]);
         if (base >= count) break;
-        uint32_t i = base + (threadIdx.x & 31u);
-        if (i < count) {
-            LuxRay r = rays[i];
-            f3 o{r.origin[0], r.origin[1], r.origin[2]}, d{r.direction[0], r.direction[1], r.direction[2]};
-            lux::Hit hit;
-            lux::trace<false>(S, o, d, r.tmin, r.limit, hit, cn);
-            store_ray(V, i, o, d, hit);
-            st[kStatInterval] += 1;
+        const uint32_t i = base + (threadIdx.x & 31u);
+        const bool active = i < count;
+        LuxRay r{};
+        if (active) {
+            r = rays[i];
+            ++traced;
         }
+        closest_ray_warp<lux::kStack, kFlat>(V, S, i, active, f3{r.origin[0], r.origin[1], r.origin[2]},
+                                             f3{r.direction[0], r.direction[1], r.direction[2]}, r.tmin, r.limit, cn, L);
     }
+    unsigned long long st[7] = {0, 0, 0, 0, 0, 0, 0};
+    st[kStatInterval] = traced;
     st[kStatNodes] = cn.nodes;
     st[kStatTris] = cn.triangles;
     st[kStatInst] = cn.instances;
@@ -3804,9 +3779,12 @@ lux_status launch_interval_radiance(LuxContext *ctx, const LuxScene *scene, cons
     cudaStream_t st = ctx->stream;
     scratch_clear_kernel<<<1, 32, 0, st>>>(V);
     if (count) {
-        closest_rays_kernel<<<ctx->sm_count * 16, 128, 0, st>>>(V, scene->view, rays, count);
+        const bool flat = scene->view.flat_nodes != nullptr;
+        (flat ? closest_rays_kernel<true> : closest_rays_kernel<false>)<<<ctx->sm_count * 16, 128, 0, st>>>(
+            V, scene->view, rays, count);
         shade_kernel<<<(count + 127) / 128, 128, 0, st>>>(V, F, scene->view, count, false);
-        shadow_kernel<64><<<ctx->sm_count * 16, 128, 0, st>>>(V, F, scene->view, 32u);
+        (flat ? shadow_kernel<64, true> : shadow_kernel<64, false>)<<<ctx->sm_count * 16, 128, 0, st>>>(
+            V, F, scene->view, 32u);
         radiance_out_kernel<<<(count + 127) / 128, 128, 0, st>>>(V, count, (float4 *)out);
     }
     return lux_cuda_check(ctx, (int)cudaGetLastError(), "interval_radiance launch");
@@ -3935,6 +3913,7 @@ struct LuxBatch {
     std::vector<LuxBatchJob> jobs;
     LuxSettings settings{};  // frame_index zeroed
     bool history = false;    // the settings blend history: retain and history mapping run
+    bool flat = false;       // every job's scene has a flattened tree: the trace stage walks those
     std::vector<FrameParams> params;
     uint32_t total = 0;      // padded interval rays
     uint64_t rays = 0;
@@ -4010,7 +3989,7 @@ extern "C" lux_status lux_batch_create(LuxContext *ctx, LuxBatch **out) {
     if (!b) return LUX_ERR_OUT_OF_MEMORY;
     b->ctx = ctx;
     cudaSetDevice(ctx->device);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b->fused_per_sm, trace_batch_kernel, 128, 0) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b->fused_per_sm, trace_batch_kernel<false>, 128, 0) != cudaSuccess) {
         cudaGetLastError();
         b->fused_per_sm = 0;
     }
@@ -4135,6 +4114,7 @@ static void batch_enqueue(LuxBatch *b, cudaStream_t st) {
     }
     batch_layout_kernel<<<1, 1024, 0, st>>>(b->d_jobs, n, b->d_dom, b->d_count);
     batch_clear_entries_kernel<<<grid, 256, 0, st>>>(b->d_jobs, b->d_dom, n, b->d_count);
+    const bool flat = b->flat;
     if (b->total && b->tuning.fused_trace) {
         // One cooperative launch: no more blocks than can be resident.
         const uint32_t per_sm = std::min(b->tuning.closest_blocks_per_sm, (uint32_t)std::max(b->fused_per_sm, 1));
@@ -4148,15 +4128,15 @@ static void batch_enqueue(LuxBatch *b, cudaStream_t st) {
         attr[0].val.cooperative = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        cudaLaunchKernelEx(&cfg, trace_batch_kernel, (const BatchJob *)b->d_jobs, (const uint32_t *)b->d_begin, n,
+        cudaLaunchKernelEx(&cfg, flat ? trace_batch_kernel<true> : trace_batch_kernel<false>, (const BatchJob *)b->d_jobs, (const uint32_t *)b->d_begin, n,
                            b->total, (const uint32_t *)b->d_frame, b->d_counters, b->d_qbegin, B,
                            tile_of(b->tuning));
     } else if (b->total) {
-        closest_batch_kernel<<<ctx->sm_count * b->tuning.closest_blocks_per_sm, 128, 0, st>>>(
+        (flat ? closest_batch_kernel<true> : closest_batch_kernel<false>)<<<ctx->sm_count * b->tuning.closest_blocks_per_sm, 128, 0, st>>>(
             b->d_jobs, b->d_begin, n, b->total, b->d_frame, b->d_counters, tile_of(b->tuning));
         shade_batch_kernel<<<grid, 128, 0, st>>>(b->d_jobs, b->d_begin, n, b->total, b->d_frame);
         query_prefix_kernel<<<1, 128, 0, st>>>(b->d_jobs, n, b->d_qbegin);
-        shadow_batch_kernel<<<ctx->sm_count * b->tuning.shadow_blocks_per_sm, 128, 0, st>>>(
+        (flat ? shadow_batch_kernel<true> : shadow_batch_kernel<false>)<<<ctx->sm_count * b->tuning.shadow_blocks_per_sm, 128, 0, st>>>(
             b->d_jobs, b->d_qbegin, n, b->d_counters + 1, tile_of(b->tuning));
         deposit_batch_kernel<<<grid, 128, 0, st>>>(b->d_jobs, b->d_begin, n, b->total, b->d_frame);
     }
@@ -4370,8 +4350,12 @@ extern "C" lux_status lux_batch_trace_merge(LuxBatch *b, const LuxBatchJob *jobs
     key.frame_index = 0;
     // The graph depends on the jobs' sizes and the settings, not on the
     // views' buffers (the job table is copied every frame).
-    bool same = b->built && same_jobs(b->jobs, jobs, n) && std::memcmp(&key, &b->settings, sizeof key) == 0;
+    bool flat = true;  // a refit can give or take a scene's flattened tree
+    for (uint32_t j = 0; j < n; ++j) flat = flat && jobs[j].scene->view.flat_nodes;
+    bool same = b->built && b->flat == flat && same_jobs(b->jobs, jobs, n) &&
+                std::memcmp(&key, &b->settings, sizeof key) == 0;
     if (!same) {
+        b->flat = flat;
         lux_status rc = batch_build(b, jobs, n, s, params);
         if (rc != LUX_OK) return rc;
     }

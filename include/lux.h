@@ -157,7 +157,7 @@ typedef struct LuxStats {
     uint64_t shadow_rays;       /* NEE visibility rays traced */
     uint64_t nodes_visited;     /* BVH4 nodes visited by all rays */
     uint64_t triangles_tested;  /* triangle tests by all rays */
-    uint64_t instances_visited; /* instance transforms applied */
+    uint64_t instances_visited; /* instance transforms applied (per leaf on a flattened tree) */
     uint64_t deposits;          /* (level, entry) samples deposited */
     uint64_t unsupported;       /* rays whose query was unsupported */
     uint64_t shadow_nodes;      /* of nodes_visited: by visibility queries */
@@ -377,7 +377,8 @@ typedef struct LuxTuning {
                                      grid over the scene box) before tracing */
     uint32_t sort_rays;           /* 1: order interval rays by (direction bin, origin cell) before tracing */
     uint32_t stack_depth;         /* traversal stack entries per thread: 32 or 64 (0 = 64); an overflowing
-                                     walk continues with the reference's ordered scan, same answers */
+                                     walk continues with the reference's ordered scan, same answers
+                                     (scenes walked on their flattened tree always take 64) */
     uint32_t fused_trace;         /* batches only: 1 = the trace stage (closest hits, shading, visibility,
                                      deposit) as one persistent cooperative launch with bounded grid
                                      barriers between the phases; 0 = four launches */
