@@ -79,12 +79,6 @@
 #define LUX_MERGE_COMPACT 1
 #endif
 
-// The merge preparation takes one thread per (cell, corner) instead of one
-// per cell.
-#ifndef LUX_MERGE_PREP_SPLIT
-#define LUX_MERGE_PREP_SPLIT 1
-#endif
-
 #ifndef LUX_MERGE_CORNER_OUTER
 #define LUX_MERGE_CORNER_OUTER 1
 #endif
@@ -1170,30 +1164,38 @@ __device__ __forceinline__ void history_map_item(const ViewDevice &V, const Fram
     V.hist_cell[(size_t)level * F.cell_capacity + c] = id;
 }
 
+// fn(level, c) for every (level, c < per_cell x the level's cells), all levels
+// one range, so that a small frame's levels run beside one another instead of
+// one latency after another.
+template <typename Fn>
+__device__ __forceinline__ void for_level_cells(const uint32_t *__restrict__ cell_count, const FrameParams &F,
+                                                uint32_t per_cell, Fn &&fn) {
+    unsigned long long begin = 0;
+    uint32_t l = 0;
+    unsigned long long n = (unsigned long long)min(cell_count[0], F.cell_capacity) * per_cell;
+    for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;;
+         i += (unsigned long long)gridDim.x * blockDim.x) {
+        while (i - begin >= n) {
+            begin += n;
+            if (++l >= F.levels) return;
+            n = (unsigned long long)min(cell_count[l], F.cell_capacity) * per_cell;
+        }
+        fn(l, (uint32_t)(i - begin));
+    }
+}
+
 // Before the merge, one launch for every level: each cell's corners in the
 // next level, and with history its previous frame's id.
 __global__ void merge_prep_kernel(ViewDevice V, FrameParams F, HistoryDevice H) {
     if (*V.error_flags) return;
     if (blockIdx.x == 0 && threadIdx.x < F.levels) V.pass_count[threadIdx.x] = 0u;
-    for (uint32_t l = 0; l < F.levels; ++l) {
-        const uint32_t cells = min(V.cell_count[l], F.cell_capacity);
-#if LUX_MERGE_PREP_SPLIT
-        // Eight threads per cell, one corner each; the history map goes to
-        // the thread of corner 7.
-        const unsigned long long items = (unsigned long long)cells * 8u;
-        for (unsigned long long k = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; k < items;
-             k += (unsigned long long)gridDim.x * blockDim.x) {
-            const uint32_t c = (uint32_t)(k >> 3), corner = (uint32_t)k & 7u;
-            if (l + 1u < F.levels) corner_item(V, F, l, c, corner);
-            if (F.history && corner == 7u) history_map_item(V, F, H, l, c);
-        }
-#else
-        for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < cells; c += gridDim.x * blockDim.x) {
-            if (l + 1u < F.levels) corners_item(V, F, l, c);
-            if (F.history) history_map_item(V, F, H, l, c);
-        }
-#endif
-    }
+    // Eight threads per cell, one corner each; the history map goes to the
+    // thread of corner 7.
+    for_level_cells(V.cell_count, F, 8u, [&](uint32_t l, uint32_t k) {
+        const uint32_t c = k >> 3, corner = k & 7u;
+        if (l + 1u < F.levels) corner_item(V, F, l, c, corner);
+        if (F.history && corner == 7u) history_map_item(V, F, H, l, c);
+    });
 }
 
 // A record's history is invalid when the region its rays may have crossed
@@ -1239,46 +1241,54 @@ __device__ __forceinline__ uint32_t retain_bin(const ViewDevice &V, const FrameP
 }
 
 __global__ void retain_count_kernel(ViewDevice V, FrameParams F, HistoryDevice H) {
-    for (uint32_t l = 0; l < F.levels; ++l) {
-        uint32_t cells = min(H.cell_count[l], F.cell_capacity);
-        for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < cells; c += gridDim.x * blockDim.x) {
-            int4 key;
-            uint32_t bin = retain_bin(V, F, H, l, c, key);
-            if (bin < kRetainBins) atomicAdd(&V.retain_hist[l * kRetainBins + bin], 1u);
-        }
-    }
+    for_level_cells(H.cell_count, F, 1u, [&](uint32_t l, uint32_t c) {
+        int4 key;
+        uint32_t bin = retain_bin(V, F, H, l, c, key);
+        if (bin < kRetainBins) atomicAdd(&V.retain_hist[l * kRetainBins + bin], 1u);
+    });
 }
 
 // One block of kRetainBins threads: per level, an inclusive scan of the age
-// histogram; the limit is the number of classes whose running total fits.
+// histogram (a warp per level, kRetainBins / 32 classes per lane); the limit is
+// the number of classes whose running total fits, found level by level by the
+// first warp, since what a level takes is gone for the next.
 __device__ __forceinline__ void retain_limit_block(const ViewDevice &V, const FrameParams &F) {
-    __shared__ unsigned long long scan[kRetainBins];
-    __shared__ unsigned long long remaining;
-    const uint32_t t = threadIdx.x;
-    if (t == 0) {
+    constexpr uint32_t kPer = kRetainBins / 32u;
+    __shared__ uint32_t scan[LUX_MAX_LEVELS][kRetainBins];
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint32_t l = threadIdx.x >> 5; l < F.levels; l += blockDim.x >> 5) {
+        uint32_t v[kPer], sum = 0;
+#pragma unroll
+        for (uint32_t k = 0; k < kPer; ++k) v[k] = sum += V.retain_hist[l * kRetainBins + lane * kPer + k];
+        uint32_t before = sum;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const uint32_t t = __shfl_up_sync(0xffffffffu, before, off);
+            if (lane >= (uint32_t)off) before += t;
+        }
+        before -= sum;
+#pragma unroll
+        for (uint32_t k = 0; k < kPer; ++k) scan[l][lane * kPer + k] = before + v[k];
+    }
+    __syncthreads();
+    if (threadIdx.x < 32u) {
         unsigned long long used = 0;
         for (uint32_t l = 0; l < F.levels; ++l)
             used += (unsigned long long)min(V.cell_count[l], F.cell_capacity) * F.dirs[l];
-        remaining = used < F.entry_capacity ? F.entry_capacity - used : 0ull;
-    }
-    for (uint32_t l = 0; l < F.levels; ++l) {
-        scan[t] = V.retain_hist[l * kRetainBins + t];
-        __syncthreads();
-        for (uint32_t off = 1; off < kRetainBins; off <<= 1) {
-            unsigned long long add = t >= off ? scan[t - off] : 0ull;
-            __syncthreads();
-            scan[t] += add;
-            __syncthreads();
+        unsigned long long remaining = used < F.entry_capacity ? F.entry_capacity - used : 0ull;
+        for (uint32_t l = 0; l < F.levels; ++l) {
+            const unsigned long long seeded = min(V.cell_count[l], F.cell_capacity);
+            const unsigned long long room =
+                min((unsigned long long)F.cell_capacity - seeded, remaining / F.dirs[l]);
+            uint32_t fits = 0;  // the scan is non-decreasing
+#pragma unroll
+            for (uint32_t k = 0; k < kPer; ++k) fits += scan[l][k * 32u + lane] <= room ? 1u : 0u;
+            fits = __reduce_add_sync(0xffffffffu, fits);
+            if (lane == 0) V.retain_limit[l] = fits;
+            remaining -= (fits ? scan[l][fits - 1u] : 0u) * (unsigned long long)F.dirs[l];
         }
-        unsigned long long seeded = min(V.cell_count[l], F.cell_capacity);
-        unsigned long long room = min((unsigned long long)F.cell_capacity - seeded, remaining / F.dirs[l]);
-        uint32_t fits = (uint32_t)__syncthreads_count(scan[t] <= room);  // the scan is non-decreasing
-        if (t == 0) {
-            V.retain_limit[l] = fits;
-            remaining -= (fits ? scan[fits - 1] : 0ull) * F.dirs[l];
-        }
-        __syncthreads();
     }
+    __syncthreads();
 }
 
 __global__ void __launch_bounds__(kRetainBins) retain_limit_kernel(ViewDevice V, FrameParams F) {
@@ -1309,13 +1319,10 @@ __device__ __forceinline__ void retain_cell(const ViewDevice &V, const FramePara
 }
 
 __global__ void retain_insert_kernel(ViewDevice V, FrameParams F, HistoryDevice H) {
-    for (uint32_t l = 0; l < F.levels; ++l) {
-        uint32_t cells = min(H.cell_count[l], F.cell_capacity);
-        for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < cells; c += gridDim.x * blockDim.x) {
-            int4 key;
-            if (retain_bin(V, F, H, l, c, key) < V.retain_limit[l]) retain_cell(V, F, H, l, c, key);
-        }
-    }
+    for_level_cells(H.cell_count, F, 1u, [&](uint32_t l, uint32_t c) {
+        int4 key;
+        if (retain_bin(V, F, H, l, c, key) < V.retain_limit[l]) retain_cell(V, F, H, l, c, key);
+    });
 }
 
 // mergeEntry (shaders/split.slang:1624-1725) for one record: the fresh mean
@@ -1709,6 +1716,33 @@ __device__ __forceinline__ void diffuse_at_lod(const ViewDevice &V, const FrameP
     float b[3] = {floorf(g[0]), floorf(g[1]), floorf(g[2])};
     float fr[3] = {g[0] - b[0], g[1] - b[1], g[2] - b[2]};
     float sx = 0.0f, sy = 0.0f, sz = 0.0f, observed = 0.0f, potential = 0.0f;
+    // In phases, so that each phase's loads of all eight corners are in
+    // flight together: first directory slots, then cell ids, then the texels
+    // corner by corner (a corner at a time end to end ran one chain of three
+    // dependent loads after another: 27 us for 3072 points).
+    unsigned long long found[8], key[8];
+    uint32_t slot[8], cell[8];
+    bool probe[8];
+    const unsigned long long *keys = V.dir_keys;  // level 0
+#pragma unroll
+    for (uint32_t corner = 0; corner < 8u; ++corner) {
+        const int32_t x = (int32_t)b[0] + (int32_t)(corner & 1u), y = (int32_t)b[1] + (int32_t)((corner >> 1) & 1u),
+                      z = (int32_t)b[2] + (int32_t)(corner >> 2);
+        probe[corner] = lux::cell_in_range(x, y, z);
+        key[corner] = lux::pack_cell(x, y, z, lod);
+        slot[corner] = lux::hash_key(x, y, z, (int32_t)(lod << 18), F.dir_capacity);
+        found[corner] = probe[corner] ? __ldg(keys + slot[corner]) : lux::kEmptyCell;
+    }
+#pragma unroll
+    for (uint32_t corner = 0; corner < 8u; ++corner) {
+        for (uint32_t attempt = 1; found[corner] != key[corner] && found[corner] != lux::kEmptyCell &&
+                                   attempt < F.dir_capacity; ++attempt) {
+            slot[corner] = (slot[corner] + 1u) & (F.dir_capacity - 1u);
+            found[corner] = __ldg(keys + slot[corner]);
+        }
+        cell[corner] = probe[corner] && found[corner] == key[corner] ? __ldg(V.dir_ids + slot[corner]) : lux::kEmpty;
+    }
+#pragma unroll
     for (uint32_t corner = 0; corner < 8u; ++corner) {
         float ax = (corner & 1u) == 0u ? 1.0f - fr[0] : fr[0];
         float ay = ((corner >> 1) & 1u) == 0u ? 1.0f - fr[1] : fr[1];
@@ -1716,15 +1750,16 @@ __device__ __forceinline__ void diffuse_at_lod(const ViewDevice &V, const FrameP
         float w = (ax * ay) * az;
         if (!(w > 0.0f)) continue;
         potential += w;
-        uint32_t cell = cell_id(V, F, 0, (int32_t)b[0] + (int32_t)(corner & 1u),
-                                (int32_t)b[1] + (int32_t)((corner >> 1) & 1u), (int32_t)b[2] + (int32_t)(corner >> 2),
-                                lod);
-        if (cell == lux::kEmpty) continue;
+        if (cell[corner] == lux::kEmpty) continue;
+        float4 texels[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) texels[c] = __ldg(V.tables + (size_t)cell[corner] * 36 + texel[c]);
         float px = 0.0f, py = 0.0f, pz = 0.0f, pobs = 0.0f;
+#pragma unroll
         for (int c = 0; c < 4; ++c) {
             float bw = weight[c];
             if (!(bw > 0.0f)) continue;
-            float4 s = __ldg(V.tables + (size_t)cell * 36 + texel[c]);
+            float4 s = texels[c];
             if (!(s.w > 0.0f) || !(isfinite(s.x) && isfinite(s.y) && isfinite(s.z) && isfinite(s.w))) continue;
             float ww = bw * lux::saturate(s.w);
             px = px + s.x * ww;
@@ -3063,21 +3098,46 @@ static HistoryDevice history_device(const LuxView *v) {
                          v->hist.raw,      v->hist.mass,    v->hist.cell_last, v->hist.cell_keys};
 }
 
+// Blocks of `threads` for at most `items` items, no more than `most` (a
+// grid-stride launch).  A block that finds nothing to do still costs its
+// launch, and in the trace kernels one fetch of the shared work counter per
+// warp: a frame of a few hundred rays ran its closest-hit pass with 9472 warps
+// (27 us against 21 with the blocks its rays need).
+static int blocks_for(uint64_t items, uint32_t threads, int most) {
+    const uint64_t need = (items + threads - 1) / threads;
+    return (int)std::max<uint64_t>(1, std::min<uint64_t>(need, (uint64_t)most));
+}
+
+// Blocks of a persistent trace launch over at most `items` rays or queries.
+static int trace_blocks(const LuxContext *ctx, uint32_t per_sm, uint32_t tile, uint64_t items) {
+    return blocks_for(items, 4u * tile, ctx->sm_count * (int)per_sm);
+}
+
+// The most visibility queries `rays` rays of a frame can queue.
+static uint64_t most_queries(const FrameParams &F, const LuxScene *scene, uint64_t rays) {
+    const uint32_t emissive = std::max(1u, F.shade.emissive_samples / 2u);
+    const bool sky = F.shade.environment.x > 0.0f || F.shade.environment.y > 0.0f || F.shade.environment.z > 0.0f;
+    return rays * std::min<uint64_t>(lux::kMaxNeeSamples,
+                                     emissive * (sky ? 2u : 1u) + scene->view.conventional_lights);
+}
+
 // seed: clear, the receivers' cells and dense ids, the sample-sequence order.
 static void enqueue_seed(LuxView *v, const FrameParams &F, const float4 *pos, cudaStream_t st) {
     const ViewDevice &D = v->dev;
-    const int grid = v->ctx->sm_count * 8;
-    clear_kernel<<<grid, 256, 0, st>>>(D, F);
+    const int most = v->ctx->sm_count * 8;
+    const uint64_t slots = (uint64_t)F.levels * F.dir_capacity, places = (uint64_t)F.receivers * F.levels;
+    clear_kernel<<<blocks_for(slots, 256, most), 256, 0, st>>>(D, F);
     if (F.receivers) {
-        seed_insert_kernel<<<grid, 256, 0, st>>>(D, F, pos);
-        seed_assign_kernel<<<grid, 256, 0, st>>>(D, F);
-        seed_lookup_kernel<<<grid, 256, 0, st>>>(D, F, pos);
+        seed_insert_kernel<<<blocks_for(places, 256, most), 256, 0, st>>>(D, F, pos);
+        seed_assign_kernel<<<blocks_for(slots, 256, most), 256, 0, st>>>(D, F);
+        seed_lookup_kernel<<<blocks_for(places, 256, most), 256, 0, st>>>(D, F, pos);
         if (F.layout == LUX_LAYOUT_SPLIT) {  // the receivers' places in the sample sequence
             size_t bytes = D.order_temp_bytes;
             cub::DeviceRadixSort::SortPairs(D.order_temp, bytes, D.order_keys, D.order_keys + v->desc.max_receivers,
                                             D.order_vals, D.order_vals + v->desc.max_receivers, (int)F.receivers, 0,
                                             62, st);
-            ordinal_kernel<<<grid, 256, 0, st>>>(D, D.order_vals + v->desc.max_receivers, F.receivers);
+            ordinal_kernel<<<blocks_for(F.receivers, 256, most), 256, 0, st>>>(D, D.order_vals + v->desc.max_receivers,
+                                                                              F.receivers);
         }
     }
 }
@@ -3085,16 +3145,17 @@ static void enqueue_seed(LuxView *v, const FrameParams &F, const float4 *pos, cu
 // layout: retained cells, record offsets, cleared records.
 static void enqueue_layout(LuxView *v, const FrameParams &F, cudaStream_t st) {
     const ViewDevice &D = v->dev;
-    const int grid = v->ctx->sm_count * 8;
+    const int most = v->ctx->sm_count * 8;
     if (F.history && F.layout == LUX_LAYOUT_SPLIT) {  // retain: the previous frame's unseen cells stay
         const HistoryDevice H = history_device(v);
         cudaMemsetAsync(D.retain_hist, 0, (size_t)LUX_MAX_LEVELS * kRetainBins * sizeof(uint32_t), st);
-        retain_count_kernel<<<grid, 256, 0, st>>>(D, F, H);
+        const int blocks = blocks_for((uint64_t)F.cell_capacity * F.levels, 256, most);
+        retain_count_kernel<<<blocks, 256, 0, st>>>(D, F, H);
         retain_limit_kernel<<<1, kRetainBins, 0, st>>>(D, F);
-        retain_insert_kernel<<<grid, 256, 0, st>>>(D, F, H);
+        retain_insert_kernel<<<blocks, 256, 0, st>>>(D, F, H);
     }
     layout_kernel<<<1, 32, 0, st>>>(D, F);
-    clear_entries_kernel<<<grid, 256, 0, st>>>(D, F);
+    clear_entries_kernel<<<blocks_for(F.entry_capacity, 256, most), 256, 0, st>>>(D, F);
 }
 
 static void enqueue_setup(LuxView *v, const FrameParams &F, const float4 *pos, cudaStream_t st) {
@@ -3106,21 +3167,24 @@ static void enqueue_setup(LuxView *v, const FrameParams &F, const float4 *pos, c
 // levels n-1 .. 0, shaders/split.slang:1624-1725).
 static void enqueue_merge(LuxView *v, const FrameParams &F, cudaStream_t st) {
     const ViewDevice &D = v->dev;
-    const int grid = v->ctx->sm_count * 8;
+    const int most = v->ctx->sm_count * 8;
     const HistoryDevice H = history_device(v);
-    if (F.levels > 1 || F.history) merge_prep_kernel<<<grid, 128, 0, st>>>(D, F, H);
+    // Records bound every pass; a view's capacity is usually close to its use.
+    const int own_blocks = blocks_for(F.entry_capacity, 256, most * 2);
+    const int child_blocks = blocks_for(F.entry_capacity, LUX_MERGE_THREADS, most * 512 / LUX_MERGE_THREADS);
+    if (F.levels > 1 || F.history)
+        merge_prep_kernel<<<blocks_for((uint64_t)F.cell_capacity * F.levels * 8u, 128, most), 128, 0, st>>>(D, F, H);
     // Record indices in the pass list are 32-bit (a level's records).
     const bool listed = LUX_MERGE_COMPACT && F.levels > 1 && v->desc.max_entries <= 0xffffffffull;
     if (listed) {
-        merge_own_list_kernel<<<grid * 2, 256, 0, st>>>(D, F, H);
+        merge_own_list_kernel<<<own_blocks, 256, 0, st>>>(D, F, H);
         for (int l = (int)F.levels - 2; l >= 0; --l)
-            merge_children_list_kernel<<<grid * 512 / LUX_MERGE_THREADS, LUX_MERGE_THREADS, 0, st>>>(D, F,
-                                                                                                   (uint32_t)l);
+            merge_children_list_kernel<<<child_blocks, LUX_MERGE_THREADS, 0, st>>>(D, F, (uint32_t)l);
         return;
     }
-    merge_own_kernel<<<grid * 2, 256, 0, st>>>(D, F, H);
+    merge_own_kernel<<<own_blocks, 256, 0, st>>>(D, F, H);
     for (int l = (int)F.levels - 2; l >= 0; --l)
-        merge_children_kernel<<<grid * 512 / LUX_MERGE_THREADS, LUX_MERGE_THREADS, 0, st>>>(D, F, (uint32_t)l);
+        merge_children_kernel<<<child_blocks, LUX_MERGE_THREADS, 0, st>>>(D, F, (uint32_t)l);
 }
 
 // Start of an unbatched frame: the last frame's records become the history
@@ -3166,7 +3230,7 @@ static void end_history(LuxView *v, const FrameParams &F) {
 // checked by make_params.
 static void enqueue_pack(LuxView *v, const FrameParams &F, cudaStream_t st) {
     size_t smem = (size_t)F.dirs[0] * 2 * sizeof(float4);
-    pack_kernel<<<v->ctx->sm_count * 8, 64, smem, st>>>(v->dev, F);
+    pack_kernel<<<blocks_for(F.cell_capacity, 1, v->ctx->sm_count * 8), 64, smem, st>>>(v->dev, F);
 }
 
 // Next-event slots of one hit: the emissive samples (max(1, n / 2)), as many
@@ -3415,16 +3479,17 @@ static lux_status view_frame(LuxView *v, const LuxScene *scene, const LuxSetting
                 cudaMemsetAsync(C.counters, 0, kCntCount * 4, st);
                 cudaMemsetAsync(C.global_error, 0, 8, st);
                 (flat ? closest_cache_kernel<true> : closest_cache_kernel<false>)
-                    <<<ctx->sm_count * T.closest_blocks_per_sm, 128, 0, st>>>(D, F, scene->view, pos, nrm, rays, C);
+                    <<<trace_blocks(ctx, T.closest_blocks_per_sm, 32u, rays), 128, 0, st>>>(D, F, scene->view, pos, nrm,
+                                                                                            rays, C);
             } else if (T.closest_mode == 1)
-                closest_split_refill_kernel<<<ctx->sm_count * T.closest_blocks_per_sm, 128, 0, st>>>(
+                closest_split_refill_kernel<<<trace_blocks(ctx, T.closest_blocks_per_sm, 32u, rays), 128, 0, st>>>(
                     Dr, F, scene->view, pos, nrm, rays);
             else {
                 auto kernel = flat ? closest_split_kernel<64, true>
                                    : (T.stack_depth == 32 ? closest_split_kernel<32, false>
                                                           : closest_split_kernel<64, false>);
-                kernel<<<ctx->sm_count * T.closest_blocks_per_sm, 128, 0, st>>>(Dr, F, scene->view, pos, nrm, rays,
-                                                                                 tile_of(T));
+                kernel<<<trace_blocks(ctx, T.closest_blocks_per_sm, tile_of(T), rays), 128, 0, st>>>(
+                    Dr, F, scene->view, pos, nrm, rays, tile_of(T));
             }
             if (forked) cudaStreamWaitEvent(st, v->laid_out, 0);  // join the setup stream
             ViewDevice Dq = D;  // query pass view: keys written by shade, optional order
@@ -3437,12 +3502,15 @@ static lux_status view_frame(LuxView *v, const LuxScene *scene, const LuxSetting
                 sort_scatter_kernel<<<ctx->sm_count * 8, 256, 0, st>>>(D, D.ts.queue_count, F.queue_capacity);
                 Dq.query_order = D.sort_perm;
             }
+            const uint64_t queries = most_queries(F, scene, rays);
             if (T.shadow_mode == 1)
-                shadow_refill_kernel<<<ctx->sm_count * T.shadow_blocks_per_sm, 128, 0, st>>>(Dq, F, scene->view);
+                shadow_refill_kernel<<<trace_blocks(ctx, T.shadow_blocks_per_sm, 32u, queries), 128, 0, st>>>(
+                    Dq, F, scene->view);
             else {
                 auto kernel = flat ? shadow_kernel<64, true>
                                    : (T.stack_depth == 32 ? shadow_kernel<32, false> : shadow_kernel<64, false>);
-                kernel<<<ctx->sm_count * T.shadow_blocks_per_sm, 128, 0, st>>>(Dq, F, scene->view, tile_of(T));
+                kernel<<<trace_blocks(ctx, T.shadow_blocks_per_sm, tile_of(T), queries), 128, 0, st>>>(Dq, F, scene->view,
+                                                                                                     tile_of(T));
             }
             if (cached) {
                 const int g = ctx->sm_count * 8;
@@ -3464,12 +3532,14 @@ static lux_status view_frame(LuxView *v, const LuxScene *scene, const LuxSetting
         }
     } else {
         const bool flat = scene->view.flat_nodes != nullptr;
-        (flat ? closest_dense_kernel<true> : closest_dense_kernel<false>)<<<ctx->sm_count * 16, 128, 0, st>>>(
-            D, F, scene->view);
-        shade_kernel<<<ctx->sm_count * 16, 128, 0, st>>>(D, F, scene->view, F.ray_capacity, true);
+        const uint64_t rays = std::min<uint64_t>(F.ray_capacity, F.entry_capacity);  // one per record
+        const int blocks = blocks_for(rays, 128, ctx->sm_count * 16);
+        (flat ? closest_dense_kernel<true> : closest_dense_kernel<false>)<<<blocks, 128, 0, st>>>(D, F, scene->view);
+        shade_kernel<<<blocks, 128, 0, st>>>(D, F, scene->view, F.ray_capacity, true);
         (flat ? shadow_kernel<64, true> : shadow_kernel<64, false>)
-            <<<ctx->sm_count * v->tuning.shadow_blocks_per_sm, 128, 0, st>>>(D, F, scene->view, tile_of(v->tuning));
-        deposit_dense_kernel<<<ctx->sm_count * 16, 128, 0, st>>>(D, F);
+            <<<trace_blocks(ctx, v->tuning.shadow_blocks_per_sm, tile_of(v->tuning), most_queries(F, scene, rays)), 128, 0,
+               st>>>(D, F, scene->view, tile_of(v->tuning));
+        deposit_dense_kernel<<<blocks, 128, 0, st>>>(D, F);
     }
     mark(2);
     enqueue_merge(v, F, st);
@@ -3780,11 +3850,11 @@ lux_status launch_interval_radiance(LuxContext *ctx, const LuxScene *scene, cons
     scratch_clear_kernel<<<1, 32, 0, st>>>(V);
     if (count) {
         const bool flat = scene->view.flat_nodes != nullptr;
-        (flat ? closest_rays_kernel<true> : closest_rays_kernel<false>)<<<ctx->sm_count * 16, 128, 0, st>>>(
+        (flat ? closest_rays_kernel<true> : closest_rays_kernel<false>)<<<trace_blocks(ctx, 16u, 32u, count), 128, 0, st>>>(
             V, scene->view, rays, count);
         shade_kernel<<<(count + 127) / 128, 128, 0, st>>>(V, F, scene->view, count, false);
-        (flat ? shadow_kernel<64, true> : shadow_kernel<64, false>)<<<ctx->sm_count * 16, 128, 0, st>>>(
-            V, F, scene->view, 32u);
+        (flat ? shadow_kernel<64, true> : shadow_kernel<64, false>)
+            <<<trace_blocks(ctx, 16u, 32u, most_queries(F, scene, count)), 128, 0, st>>>(V, F, scene->view, 32u);
         radiance_out_kernel<<<(count + 127) / 128, 128, 0, st>>>(V, count, (float4 *)out);
     }
     return lux_cuda_check(ctx, (int)cudaGetLastError(), "interval_radiance launch");
