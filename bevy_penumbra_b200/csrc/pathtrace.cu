@@ -305,7 +305,7 @@ extern "C" lux_status lux_path_reference(LuxContext *ctx, const LuxScene *scene,
     lux_settings_sanitize(&s);
     PathParams P{};
     P.shade.normal_bias = s.normal_bias;
-    P.shade.exposure = s.exposure;
+    P.shade.inv_exposure = 1.0f / std::fmax(s.exposure, 1e-20f);
     P.shade.environment = f3{s.environment[0], s.environment[1], s.environment[2]};
     P.spp = spp;
     P.bounces = bounces;

@@ -34,7 +34,7 @@ struct Feedback {
 struct ShadeParams {
     float probe_spacing;
     float normal_bias;
-    float exposure;
+    float inv_exposure;  // 1 / max(exposure, 1e-20)
     uint32_t emissive_samples;
     uint32_t frame;
     uint32_t skip_emission;  // secondary cache: no first-hit emission (next-event estimation carries it)
@@ -98,6 +98,12 @@ __device__ __forceinline__ uint32_t instance_base(const SceneView &S, uint32_t i
     return h.y + inst * h.w;
 }
 
+// The exposure weighting of hitEmission.
+__device__ __forceinline__ float emission_factor(const ShadeParams &P, uint32_t flags, float exposure_weight) {
+    const float weight = (flags & 16u) != 0u ? 0.0f : exposure_weight;
+    return P.inv_exposure + weight * (1.0f - P.inv_exposure);
+}
+
 // materialBaseColor / hitEmission (shaders/material.slang:139-141,
 // shaders/traversal.slang:287-300), untextured.
 __device__ __forceinline__ Surface surface_at(const SceneView &S, const ShadeParams &P, uint32_t inst, uint32_t tri,
@@ -117,15 +123,23 @@ __device__ __forceinline__ Surface surface_at(const SceneView &S, const ShadePar
     Surface sf;
     sf.base_color = f3{as_float(m0.x) * color.x, as_float(m0.y) * color.y, as_float(m0.z) * color.z};
     sf.emission = (flags & 16u) != 0u ? sf.base_color : f3{as_float(m1.x), as_float(m1.y), as_float(m1.z)};
-    float weight = (flags & 16u) != 0u ? 0.0f : as_float(m2.w);
-    float exposure = fmaxf(P.exposure, 1e-20f);
-    float inv = 1.0f / exposure;
-    float factor = inv + weight * (1.0f - inv);
-    sf.emission = sf.emission * factor;
+    sf.emission = sf.emission * emission_factor(P, flags, as_float(m2.w));
     sf.metallic = as_float(m2.x);
     sf.roughness = as_float(m2.y);
     sf.flags = flags;
     return sf;
+}
+
+// surface_at(...).emission: a lit emitter's emission is its material's, so the
+// triangle's vertex colours are read for unlit ones only (5 loads for 12).
+__device__ __forceinline__ f3 emission_at(const SceneView &S, const ShadeParams &P, uint32_t inst, uint32_t tri,
+                                          float b0, float b1, float b2) {
+    const uint32_t base = instance_base(S, inst);
+    const uint32_t flags = sword(S, base + 6).w;
+    if ((flags & 16u) != 0u) return surface_at(S, P, inst, tri, b0, b1, b2).emission;
+    const uint32_t material = sword(S, base + 7).w;
+    const uint4 m1 = sword(S, material + 1), m2 = sword(S, material + 2);
+    return f3{as_float(m1.x), as_float(m1.y), as_float(m1.z)} * emission_factor(P, flags, as_float(m2.w));
 }
 
 // disneyDiffuseMultiplier, shaders/common.slang:298-314.
@@ -228,200 +242,175 @@ struct NeeQuery {
     NeeGroup group;  // emissive and environment samples are averaged per group, conventional lights summed
 };
 
-// emissiveResponseTracked, shaders/cascades.slang:57-134, up to (but not
-// including) the visibility trace: every sample that survives the geometric
-// tests becomes a query with its contribution emission * (response * cos / pdf).
-// Samples are emitted in sample order; `count` is the estimator's divisor.
-template <typename Emit>
-__device__ void emissive_queries(const SceneView &S, const ShadeParams &P, f3 position, f3 normal, f3 gnormal,
-                                 f3 view, float roughness, f3 diffuse, uint32_t &count, Emit &&emit) {
-    uint32_t emissive = S.emissive_lights;
-    count = P.emissive_samples / 2u;
-    count = count < 1u ? 1u : count;
-    if (emissive == 0u) return;
-    float cell = P.probe_spacing * 0.05f;
-    uint32_t seed = hash_key((int32_t)floorf(position.x / cell), (int32_t)floorf(position.y / cell),
-                             (int32_t)floorf(position.z / cell), 0, 16777216u);
-    float rot_x, rot_y;
-    r2(seed, rot_x, rot_y);
-    float s0 = P.probe_spacing * 1.0f;
-    uint32_t selection_seed = hash_key((int32_t)floorf(position.x / s0), (int32_t)floorf(position.y / s0),
-                                       (int32_t)floorf(position.z / s0), 0, 65536u);
-    uint32_t sample_frame = P.frame ^ 0xE11E0001u;
-    float ax, ay, bx, by;
-    r2(sample_frame, ax, ay);
-    r2(selection_seed, bx, by);
-    float phase = fracf(ax + bx);
+// A lit hit as its next-event samples need it: surface, scattering, and the
+// parts of the sample sequences that depend on the hit alone.
+struct NeeVertex {
+    f3 position, normal, gnormal, view, diffuse;
+    float roughness;
+    float rot_x, rot_y, phase;  // emissive samples: sequence rotation, light selection phase
+    uint32_t sky_seed;          // environment samples
+};
+
+// The estimator's divisor: emissive samples per hit (and environment samples,
+// with a non-black environment).
+__device__ __forceinline__ uint32_t nee_count(const ShadeParams &P) { return max(P.emissive_samples / 2u, 1u); }
+
+// Sample `sample` of emissiveResponseTracked, shaders/cascades.slang:57-134,
+// up to (but not including) the visibility trace: false when it does not
+// survive the geometric tests, else its query with contribution emission *
+// (response * cos / pdf).
+__device__ __forceinline__ bool emissive_sample(const SceneView &S, const ShadeParams &P, const NeeVertex &v,
+                                                uint32_t count, uint32_t sample, NeeQuery &q) {
+    const uint32_t emissive = S.emissive_lights;
+    const uint32_t sample_frame = P.frame ^ 0xE11E0001u;
     const float bias = P.normal_bias;
     const LuxLight *lights = S.lights + S.conventional_lights;
-    for (uint32_t sample = 0; sample < count; ++sample) {
-        float rx, ry;
-        r2(sample + sample_frame * count + 1u, rx, ry);
-        float ux = fracf(rx + rot_x), uy = fracf(ry + rot_y);
-        float selection = fracf(((float)sample + 0.5f) / (float)count + phase);
-        uint32_t low = 0, high = emissive - 1u;
-        while (low < high) {
-            uint32_t middle = (low + high) / 2u;
-            if (__ldg(&lights[middle].direction[3]) < selection)
-                low = middle + 1u;
-            else
-                high = middle;
-        }
-        const LuxLight *L = lights + low;
-        f3 lp{__ldg(&L->position[0]), __ldg(&L->position[1]), __ldg(&L->position[2])};
-        float lpw = __ldg(&L->position[3]);
-        f3 ldir{__ldg(&L->direction[0]), __ldg(&L->direction[1]), __ldg(&L->direction[2])};
-        f3 e1{__ldg(&L->edge1[0]), __ldg(&L->edge1[1]), __ldg(&L->edge1[2])};
-        float e1w = __ldg(&L->edge1[3]);
-        f3 e2{__ldg(&L->edge2[0]), __ldg(&L->edge2[1]), __ldg(&L->edge2[2])};
-        float area = __ldg(&L->color[3]);
-        f3 rel = position - lp;
-        if (e1w <= 0.0f || (lpw != -2.0f && dot(ldir, rel) <= 0.0f)) continue;
-        float root = sqrtf(ux);
-        float w1 = root * (1.0f - uy), w2 = root * uy;
-        f3 target{(lp.x + e1.x * w1) + e2.x * w2, (lp.y + e1.y * w1) + e2.y * w2, (lp.z + e1.z * w1) + e2.z * w2};
-        f3 to_light = target - position;
-        float light_distance = length(to_light);
-        if (light_distance <= bias * 0.25f) continue;
-        f3 ld = to_light / light_distance;
-        float cosine = fmaxf(0.0f, dot(normal, ld));
-        float c_emit = dot(ldir, -ld);
-        if (lpw == -2.0f) c_emit = fabsf(c_emit);
-        float emitter_cosine = fmaxf(0.0f, c_emit);
-        if (cosine <= 0.0f || emitter_cosine <= 0.0f || dot(gnormal, ld) <= 0.0f) continue;
-        Surface es = surface_at(S, P, __ldg(&L->source[0]), __ldg(&L->source[1]), 1.0f - root, w1, w2);
-        f3 emission{fmaxf(es.emission.x, 0.0f), fmaxf(es.emission.y, 0.0f), fmaxf(es.emission.z, 0.0f)};
-        if (!(emission.x > 0.0f || emission.y > 0.0f || emission.z > 0.0f)) continue;
-        float pdf = ((e1w * light_distance) * light_distance) / (area * emitter_cosine);
-        float plane = fabsf(dot(ldir, rel));
-        f3 origin = ray_offset(position, gnormal, fminf(bias, plane * 0.25f));
-        f3 delta = target - origin;
-        float distance = length(delta);
-        if (distance <= bias * 0.25f) continue;
-        NeeQuery q;
-        q.origin = origin;
-        q.direction = delta / distance;
-        q.limit = distance - fminf(bias * 0.25f, distance * 0.001f);
-        float factor = disney_multiplier(normal, ld, view, roughness) / kPi;
-        float p = fmaxf(pdf, 1e-20f);
-        q.contribution = f3{emission.x * (((diffuse.x * factor) * cosine) / p),
-                            emission.y * (((diffuse.y * factor) * cosine) / p),
-                            emission.z * (((diffuse.z * factor) * cosine) / p)};
-        q.light = low;
-        q.group = kNeeEmissive;
-        emit(sample, q);
+    float rx, ry;
+    r2(sample + sample_frame * count + 1u, rx, ry);
+    float ux = fracf(rx + v.rot_x), uy = fracf(ry + v.rot_y);
+    float selection = fracf(((float)sample + 0.5f) / (float)count + v.phase);
+    uint32_t low = 0, high = emissive - 1u;
+    while (low < high) {
+        uint32_t middle = (low + high) / 2u;
+        if (__ldg(&lights[middle].direction[3]) < selection)
+            low = middle + 1u;
+        else
+            high = middle;
     }
+    const float4 *L = reinterpret_cast<const float4 *>(lights + low);  // position, color, direction, edge1, edge2, source
+    const float4 l0 = __ldg(L), l2 = __ldg(L + 2), l3 = __ldg(L + 3), l4 = __ldg(L + 4);
+    const float area = __ldg(reinterpret_cast<const float *>(L + 1) + 3);
+    const uint2 source = __ldg(reinterpret_cast<const uint2 *>(L + 5));
+    f3 lp{l0.x, l0.y, l0.z};
+    const float lpw = l0.w;
+    f3 ldir{l2.x, l2.y, l2.z}, e1{l3.x, l3.y, l3.z}, e2{l4.x, l4.y, l4.z};
+    const float e1w = l3.w;
+    f3 rel = v.position - lp;
+    if (e1w <= 0.0f || (lpw != -2.0f && dot(ldir, rel) <= 0.0f)) return false;
+    float root = sqrtf(ux);
+    float w1 = root * (1.0f - uy), w2 = root * uy;
+    f3 target{(lp.x + e1.x * w1) + e2.x * w2, (lp.y + e1.y * w1) + e2.y * w2, (lp.z + e1.z * w1) + e2.z * w2};
+    f3 to_light = target - v.position;
+    float light_distance = length(to_light);
+    if (light_distance <= bias * 0.25f) return false;
+    f3 ld = to_light / light_distance;
+    float cosine = fmaxf(0.0f, dot(v.normal, ld));
+    float c_emit = dot(ldir, -ld);
+    if (lpw == -2.0f) c_emit = fabsf(c_emit);
+    float emitter_cosine = fmaxf(0.0f, c_emit);
+    if (cosine <= 0.0f || emitter_cosine <= 0.0f || dot(v.gnormal, ld) <= 0.0f) return false;
+    const f3 es = emission_at(S, P, source.x, source.y, 1.0f - root, w1, w2);
+    f3 emission{fmaxf(es.x, 0.0f), fmaxf(es.y, 0.0f), fmaxf(es.z, 0.0f)};
+    if (!(emission.x > 0.0f || emission.y > 0.0f || emission.z > 0.0f)) return false;
+    float pdf = ((e1w * light_distance) * light_distance) / (area * emitter_cosine);
+    float plane = fabsf(dot(ldir, rel));
+    f3 origin = ray_offset(v.position, v.gnormal, fminf(bias, plane * 0.25f));
+    f3 delta = target - origin;
+    float distance = length(delta);
+    if (distance <= bias * 0.25f) return false;
+    q.origin = origin;
+    q.direction = delta / distance;
+    q.limit = distance - fminf(bias * 0.25f, distance * 0.001f);
+    float factor = disney_multiplier(v.normal, ld, v.view, v.roughness) / kPi;
+    float p = fmaxf(pdf, 1e-20f);
+    q.contribution = f3{emission.x * (((v.diffuse.x * factor) * cosine) / p),
+                        emission.y * (((v.diffuse.y * factor) * cosine) / p),
+                        emission.z * (((v.diffuse.z * factor) * cosine) / p)};
+    q.light = low;
+    q.group = kNeeEmissive;
+    return true;
 }
 
-// conventionalLightResponseTracked (shaders/cascades.slang:136-176) up to the
-// visibility traces: one query per conventional light that faces the
-// surface, from the biased hit point to the light (finite lights: range fade
-// (1 - (d/range)^4)^2 / d^2, spot cone squared; directional lights: the
-// direction in position.xyz at distance 1e20), contribution color x
-// (attenuation x cos x response).  Light i takes slot first_slot + i.
+// Light i of conventionalLightResponseTracked (shaders/cascades.slang:136-176)
+// up to the visibility trace: a query when it faces the surface, from the
+// biased hit point to the light (finite lights: range fade (1 - (d/range)^4)^2 /
+// d^2, spot cone squared; directional lights: the direction in position.xyz at
+// distance 1e20), contribution color x (attenuation x cos x response).
 // (d/range)^4 is (x^2)^2 here and in the oracle.
-template <typename Emit>
-__device__ void conventional_queries(const SceneView &S, const ShadeParams &P, f3 position, f3 normal, f3 gnormal,
-                                     f3 view, float roughness, f3 diffuse, uint32_t first_slot, Emit &&emit) {
-    const uint32_t n = S.conventional_lights;
-    if (n == 0u) return;
+__device__ __forceinline__ bool conventional_sample(const SceneView &S, const ShadeParams &P, const NeeVertex &v,
+                                                    uint32_t i, NeeQuery &q) {
     const float bias = P.normal_bias;
-    const f3 offset = ray_offset(position, gnormal, bias);
-    for (uint32_t i = 0; i < n; ++i) {
-        const LuxLight *L = S.lights + i;
-        f3 lp{__ldg(&L->position[0]), __ldg(&L->position[1]), __ldg(&L->position[2])};
-        float range = __ldg(&L->position[3]);
-        const bool finite = range > 0.0f;
-        f3 to_light = lp;
-        float distance = 1e20f, attenuation = 1.0f;
-        if (finite) {
-            to_light = lp - position;
-            distance = length(to_light);
-            if (distance >= range || distance < bias) continue;
-            to_light = to_light / distance;
-            float x = distance / range;
-            float x2 = x * x;
-            float fade = saturate(1.0f - x2 * x2);
-            attenuation = (fade * fade) / fmaxf(distance * distance, 0.0001f);
-            float spot = __ldg(&L->direction[3]);
-            if (spot > 0.0f) {
-                f3 ldir{__ldg(&L->direction[0]), __ldg(&L->direction[1]), __ldg(&L->direction[2])};
-                float cone = saturate(dot(ldir, -to_light) * spot + __ldg(&L->color[3]));
-                attenuation *= cone * cone;
-            }
+    const LuxLight *L = S.lights + i;
+    f3 lp{__ldg(&L->position[0]), __ldg(&L->position[1]), __ldg(&L->position[2])};
+    float range = __ldg(&L->position[3]);
+    const bool finite = range > 0.0f;
+    f3 to_light = lp;
+    float distance = 1e20f, attenuation = 1.0f;
+    if (finite) {
+        to_light = lp - v.position;
+        distance = length(to_light);
+        if (distance >= range || distance < bias) return false;
+        to_light = to_light / distance;
+        float x = distance / range;
+        float x2 = x * x;
+        float fade = saturate(1.0f - x2 * x2);
+        attenuation = (fade * fade) / fmaxf(distance * distance, 0.0001f);
+        float spot = __ldg(&L->direction[3]);
+        if (spot > 0.0f) {
+            f3 ldir{__ldg(&L->direction[0]), __ldg(&L->direction[1]), __ldg(&L->direction[2])};
+            float cone = saturate(dot(ldir, -to_light) * spot + __ldg(&L->color[3]));
+            attenuation *= cone * cone;
         }
-        float cosine = fmaxf(0.0f, dot(normal, to_light));
-        if (!(cosine > 0.0f && dot(gnormal, to_light) > 0.0f && attenuation > 0.0f)) continue;
-        NeeQuery q;
-        q.origin = offset;
-        q.direction = to_light;
-        q.limit = distance - bias;
-        float factor = disney_multiplier(normal, to_light, view, roughness) / kPi;
-        float scale = attenuation * cosine;
-        q.contribution = f3{__ldg(&L->color[0]) * (scale * (diffuse.x * factor)),
-                            __ldg(&L->color[1]) * (scale * (diffuse.y * factor)),
-                            __ldg(&L->color[2]) * (scale * (diffuse.z * factor))};
-        q.light = i;
-        q.group = kNeeConventional;
-        emit(first_slot + i, q);
     }
+    float cosine = fmaxf(0.0f, dot(v.normal, to_light));
+    if (!(cosine > 0.0f && dot(v.gnormal, to_light) > 0.0f && attenuation > 0.0f)) return false;
+    q.origin = ray_offset(v.position, v.gnormal, bias);
+    q.direction = to_light;
+    q.limit = distance - bias;
+    float factor = disney_multiplier(v.normal, to_light, v.view, v.roughness) / kPi;
+    float scale = attenuation * cosine;
+    q.contribution = f3{__ldg(&L->color[0]) * (scale * (v.diffuse.x * factor)),
+                        __ldg(&L->color[1]) * (scale * (v.diffuse.y * factor)),
+                        __ldg(&L->color[2]) * (scale * (v.diffuse.z * factor))};
+    q.light = i;
+    q.group = kNeeConventional;
+    return true;
 }
 
-// environmentResponseTracked (shaders/environment.slang:154-230) for a
-// constant environment, up to the visibility traces: `count` cosine
-// proposals (no alias samples without an environment map, so pdf = cos / pi),
+// Sample `sample` of environmentResponseTracked (shaders/environment.slang:
+// 154-230) for a constant environment, up to the visibility trace: a cosine
+// proposal (no alias samples without an environment map, so pdf = cos / pi),
 // direction cosineDirection(normal, transportRandom lanes 0 and 1) of the
-// seed transportHash(seed ^ transportHash(sequence + 0x85ebca6b)),
-// sequence = sample + (frame ^ 0xE17A0002) x count, seed = hashKey of the
-// hit's cell of 0.05 probe spacings with w = 37; each a query from the biased
-// hit point to distance 1e20 with contribution environment x (response x
-// cos / pdf).  Sample i takes slot first_slot + i.
-template <typename Emit>
-__device__ void environment_queries(const ShadeParams &P, f3 position, f3 normal, f3 gnormal, f3 view,
-                                    float roughness, f3 diffuse, uint32_t count, uint32_t first_slot, Emit &&emit) {
-    if (!environment_on(P)) return;
+// seed transportHash(seed ^ transportHash(sequence + 0x85ebca6b)), sequence =
+// sample + (frame ^ 0xE17A0002) x count; a query from the biased hit point to
+// distance 1e20 with contribution environment x (response x cos / pdf).
+__device__ __forceinline__ bool environment_sample(const ShadeParams &P, const NeeVertex &v, uint32_t count,
+                                                   uint32_t sample, NeeQuery &q) {
     const f3 env = P.environment;
-    float cell = P.probe_spacing * 0.05f;
-    uint32_t seed = hash_key((int32_t)floorf(position.x / cell), (int32_t)floorf(position.y / cell),
-                             (int32_t)floorf(position.z / cell), 37, 16777216u);
     uint32_t sample_frame = P.frame ^ 0xE17A0002u;
-    const f3 offset = ray_offset(position, gnormal, P.normal_bias);
-    for (uint32_t sample = 0; sample < count; ++sample) {
-        uint32_t sequence = sample + sample_frame * count;
-        uint32_t sample_seed = transport_hash(seed ^ transport_hash(sequence + 0x85ebca6bu));
-        f3 d = cosine_direction_frame(normal, transport_random(sample_seed, 0u), transport_random(sample_seed, 1u));
-        float cosine = fmaxf(0.0f, dot(normal, d));
-        if (cosine <= 0.0f || dot(gnormal, d) <= 0.0f) continue;
-        float pdf = cosine / kPi;
-        if (!(pdf > 0.0f) || !isfinite(pdf)) continue;
-        NeeQuery q;
-        q.origin = offset;
-        q.direction = d;
-        q.limit = 1e20f;
-        float factor = disney_multiplier(normal, d, view, roughness) / kPi;
-        q.contribution = f3{env.x * (((diffuse.x * factor) * cosine) / pdf),
-                            env.y * (((diffuse.y * factor) * cosine) / pdf),
-                            env.z * (((diffuse.z * factor) * cosine) / pdf)};
-        q.light = 63u;
-        q.group = kNeeEnvironment;
-        emit(first_slot + sample, q);
-    }
+    uint32_t sequence = sample + sample_frame * count;
+    uint32_t sample_seed = transport_hash(v.sky_seed ^ transport_hash(sequence + 0x85ebca6bu));
+    f3 d = cosine_direction_frame(v.normal, transport_random(sample_seed, 0u), transport_random(sample_seed, 1u));
+    float cosine = fmaxf(0.0f, dot(v.normal, d));
+    if (cosine <= 0.0f || dot(v.gnormal, d) <= 0.0f) return false;
+    float pdf = cosine / kPi;
+    if (!(pdf > 0.0f) || !isfinite(pdf)) return false;
+    q.origin = ray_offset(v.position, v.gnormal, P.normal_bias);
+    q.direction = d;
+    q.limit = 1e20f;
+    float factor = disney_multiplier(v.normal, d, v.view, v.roughness) / kPi;
+    q.contribution = f3{env.x * (((v.diffuse.x * factor) * cosine) / pdf),
+                        env.y * (((v.diffuse.y * factor) * cosine) / pdf),
+                        env.z * (((v.diffuse.z * factor) * cosine) / pdf)};
+    q.light = 63u;
+    q.group = kNeeEnvironment;
+    return true;
 }
 
 // outgoingTransportRadianceTracked, shaders/cascades.slang:196-268, up to the
-// visibility traces.  Writes the hit's own emission to `base`, the
-// multi-bounce term (diffuse x secondary-cache irradiance) to `extra`, the
-// surface a secondary receiver would take to `rec`, and emits the next-event
-// queries; returns false when the query is unsupported (no deposit).
-// `count` = 0 when no next-event estimate applies; `sky` is set when the
-// hit takes environment samples (slots count .. 2 count - 1).
-template <typename Emit>
-__device__ bool outgoing_record(const SceneView &S, const ShadeParams &P, f3 origin, f3 direction, const Hit &hit,
-                                f3 &base, f3 &extra, SurfaceRecord &rec, uint32_t &count, bool &sky, Emit &&emit) {
+// next-event samples: the hit's own emission in `base`, the multi-bounce term
+// (diffuse x secondary-cache irradiance) in `extra`, the surface a secondary
+// receiver would take in `rec`, and with `lit` the vertex its samples take
+// (emissive ones in slots 0 .. count - 1; with `sky` environment ones in slots
+// count .. 2 count - 1; then one per conventional light).  Returns false when
+// the query is unsupported (no deposit).
+__device__ __forceinline__ bool outgoing_vertex(const SceneView &S, const ShadeParams &P, f3 origin, f3 direction,
+                                                const Hit &hit, f3 &base, f3 &extra, SurfaceRecord &rec, bool &lit,
+                                                bool &sky, NeeVertex &v) {
     base = f3{0.0f, 0.0f, 0.0f};
     extra = f3{0.0f, 0.0f, 0.0f};
     rec.valid = false;
-    count = 0;
+    lit = false;
     sky = false;
     if ((hit.errors & kQueryUnsupported) != 0u) return false;
     if (hit.tri == kEmpty) {
@@ -464,7 +453,6 @@ __device__ bool outgoing_record(const SceneView &S, const ShadeParams &P, f3 ori
     f3 neg = -direction;
     if (dot(normal, neg) <= 0.0f || dot(normal, flipped) <= 0.0f) return true;
     float nl = length(neg);
-    f3 view = neg / nl;
     float metallic = saturate(sf.metallic);
     float roughness = saturate(sf.roughness);
     if (!isfinite(roughness)) roughness = 1.0f;
@@ -483,19 +471,28 @@ __device__ bool outgoing_record(const SceneView &S, const ShadeParams &P, f3 ori
     // skyFromCache (shaders/cascades.slang:242): a covered hit takes its sky
     // light from the secondary cache's probe instead of environment samples.
     sky = environment_on(P) && !(P.cached_sky && coverage > 0.0f);
-    emissive_queries(S, P, position, normal, flipped, view, roughness, diffuse, count, emit);
-    if (sky) environment_queries(P, position, normal, flipped, view, roughness, diffuse, count, count, emit);
-    conventional_queries(S, P, position, normal, flipped, view, roughness, diffuse, sky ? 2u * count : count, emit);
+    lit = true;
+    v.position = position;
+    v.normal = normal;
+    v.gnormal = flipped;
+    v.view = neg / nl;
+    v.diffuse = diffuse;
+    v.roughness = roughness;
+    // The sample sequences' hit terms (shaders/cascades.slang:57-80,
+    // shaders/environment.slang:154-170).
+    const float cell = P.probe_spacing * 0.05f;
+    const int32_t cx = (int32_t)floorf(position.x / cell), cy = (int32_t)floorf(position.y / cell),
+                  cz = (int32_t)floorf(position.z / cell);
+    r2(hash_key(cx, cy, cz, 0, 16777216u), v.rot_x, v.rot_y);
+    const float s0 = P.probe_spacing * 1.0f;
+    float ax, ay, bx, by;
+    r2(P.frame ^ 0xE11E0001u, ax, ay);
+    r2(hash_key((int32_t)floorf(position.x / s0), (int32_t)floorf(position.y / s0), (int32_t)floorf(position.z / s0), 0,
+                65536u),
+       bx, by);
+    v.phase = fracf(ax + bx);
+    v.sky_seed = hash_key(cx, cy, cz, 37, 16777216u);
     return true;
-}
-
-template <typename Emit>
-__device__ bool outgoing_record(const SceneView &S, const ShadeParams &P, f3 origin, f3 direction, const Hit &hit,
-                                f3 &base, uint32_t &count, Emit &&emit) {
-    f3 extra;
-    SurfaceRecord rec;
-    bool sky;
-    return outgoing_record(S, P, origin, direction, hit, base, extra, rec, count, sky, emit);
 }
 
 // clampOutgoingTransportRadiance, shaders/cascades.slang:179-188, after the
