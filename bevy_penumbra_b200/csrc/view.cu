@@ -58,6 +58,12 @@
 #ifndef LUX_BATCH_MIN_BLOCKS
 #define LUX_BATCH_MIN_BLOCKS 6
 #endif
+// Visibility queries a frame must be able to queue for them to be ordered
+// without the tuning asking for it.
+#ifndef LUX_ORDER_QUERIES
+#define LUX_ORDER_QUERIES (1u << 21)
+#endif
+constexpr unsigned long long kOrderQueries = LUX_ORDER_QUERIES;
 // Merge launch shape: threads per block and the resident blocks the
 // register budget is sized for.
 #ifndef LUX_MERGE_THREADS
@@ -180,40 +186,43 @@ struct ViewDevice {
     unsigned long long *stats;      // 8 counters
     TraceScratch ts;                // wavefront trace state
     // Coherence ordering of rays / visibility queries (counting sort by bin).
-    uint32_t *sort_keys;            // [max(rays, queries)]
-    uint32_t *sort_perm;            // [max(rays, queries)] processing order -> item
-    uint32_t *sort_hist;            // [kSortBins]
-    uint32_t *sort_offs;            // [kSortBins] exclusive prefix of sort_hist, then scatter cursors
+    uint32_t *sort_keys;            // [rays] interval-ray keys (a query's key is in its queue_d.w)
+    uint32_t *sort_perm;            // [rays x kMaxNeeSamples] processing order -> ray, or query slot
+    uint32_t *sort_hist;            // [sort bins]
+    uint32_t *sort_offs;            // [sort bins] exclusive prefix of sort_hist, then scatter cursors
+    uint32_t query_bits;            // bits per axis of the queries' origin grid (0: queries are not ordered)
     void *scan_temp;                // device-wide scan scratch
     size_t scan_temp_bytes;
     const uint32_t *ray_order;      // closest-hit processing order (nullptr: identity)
-    const uint32_t *query_order;    // visibility processing order (nullptr: identity)
+    const uint32_t *query_order;    // query slots in processing order (nullptr: the order of query_slot)
 };
 
 // Rays per work-queue fetch of a tuning (0 means 32).
 static inline uint32_t tile_of(const LuxTuning &t) { return t.tile_rays ? t.tile_rays : 32u; }
 
 constexpr uint32_t kSortCells = 4096;           // 16^3 origin cells over the TLAS root box
-constexpr uint32_t kQueryCells = 2097152;       // 128^3 origin cells of visibility queries
 constexpr uint32_t kRaySortBins = 32 * kSortCells;  // 32 direction bins x 16^3 origin cells of interval rays
-constexpr uint32_t kSortBins = 8 * kQueryCells; // 8 emitter buckets x 128^3 origin cells of queries,
-                                                // or 32 direction bins x 16^3 cells of interval rays
 
-// Morton index of a point's cell in a 128^3 grid over the scene box (an order of
-// processing only, so an approximate reciprocal will do).
-__device__ __forceinline__ uint32_t cell128(const SceneView &S, lux::f3 p) {
-    float e[3] = {p.x, p.y, p.z};
-    uint32_t c[3];
+// Counting-sort bins of visibility queries: 8 emitter buckets x (2^bits)^3
+// origin cells.
+static inline uint32_t query_bins(uint32_t bits) { return 8u << (3u * bits); }
+
+// Morton index of a point's cell in a (2^bits)^3 grid over the scene box (an
+// order of processing only, so an approximate reciprocal will do).
+__device__ __forceinline__ uint32_t query_cell(const SceneView &S, lux::f3 p, uint32_t bits) {
+    const float e[3] = {p.x, p.y, p.z}, cells = (float)(1u << bits);
+    const int last = (1 << bits) - 1;
+    uint32_t m = 0;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
         const float span = S.root_hi[a] - S.root_lo[a];
-        const int q = (int)((e[a] - S.root_lo[a]) * (span > 0.0f ? 128.0f * lux::rcp_approx(span) : 0.0f));
-        c[a] = (uint32_t)(q < 0 ? 0 : (q > 127 ? 127 : q));
+        int q = (int)((e[a] - S.root_lo[a]) * (span > 0.0f ? cells * lux::rcp_approx(span) : 0.0f));
+        uint32_t c = (uint32_t)(q < 0 ? 0 : (q > last ? last : q));  // at most 7 bits, spread to every third
+        c = (c | (c << 8)) & 0x700fu;
+        c = (c | (c << 4)) & 0x430c3u;
+        c = (c | (c << 2)) & 0x49249u;
+        m |= c << a;
     }
-    uint32_t m = 0;
-#pragma unroll
-    for (int b = 0; b < 7; ++b)
-        m |= (((c[0] >> b) & 1u) << (3 * b)) | (((c[1] >> b) & 1u) << (3 * b + 1)) | (((c[2] >> b) & 1u) << (3 * b + 2));
     return m;
 }
 
@@ -710,19 +719,26 @@ __global__ void ray_keys_kernel(ViewDevice V, FrameParams F, SceneView S, const 
     }
 }
 
-// Counting sort of keys in [0, kSortBins): histogram, exclusive scan, scatter.
-// Order within a bin is arbitrary; every item is processed exactly once and
-// its result is written to its own slot, so the outputs do not depend on it.
-__global__ void sort_hist_kernel(ViewDevice V, const uint32_t *count_ptr, uint32_t cap) {
-    uint32_t n = count_ptr ? min(*count_ptr, cap) : cap;
+// Counting sort: histogram, exclusive scan, scatter.  Order within a bin is
+// arbitrary; every item is processed exactly once and its result is written to
+// its own slot, so the outputs do not depend on it.
+__global__ void sort_hist_kernel(ViewDevice V, uint32_t n) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         atomicAdd(&V.sort_hist[V.sort_keys[i]], 1u);
 }
 
-__global__ void sort_scatter_kernel(ViewDevice V, const uint32_t *count_ptr, uint32_t cap) {
-    uint32_t n = count_ptr ? min(*count_ptr, cap) : cap;
+__global__ void sort_scatter_kernel(ViewDevice V, uint32_t n) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         V.sort_perm[atomicAdd(&V.sort_offs[V.sort_keys[i]], 1u)] = i;
+}
+
+// The queries' slots in key order (counted by hit shading).
+__global__ void query_scatter_kernel(ViewDevice V, uint32_t capacity) {
+    const uint32_t n = min(*V.ts.queue_count, capacity);
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint32_t slot = V.ts.query_slot[i];
+        V.sort_perm[atomicAdd(&V.sort_offs[lux::as_uint(V.ts.queue_d[slot].w)], 1u)] = slot;
+    }
 }
 
 // Exclusive prefix of the first `bins` counting-sort bins over the whole
@@ -814,12 +830,17 @@ __device__ __forceinline__ void shade_warp(const ViewDevice &V, const FrameParam
         sky_mask = __reduce_or_sync(0xffffffffu, sky ? 1u << rank : 0u);
     }
     __syncwarp();
-    const bool keys = V.sort_keys != nullptr;
+    const uint32_t bits = V.query_bits;
     auto emit = [&](uint32_t k, uint32_t sample, const lux::NeeQuery &q) {
         if (sample >= lux::kMaxNeeSamples) return;  // host checks the slot count
         const size_t slot = (size_t)L->ray[k] * lux::kMaxNeeSamples + sample;
-        // w of the direction: the query's coherence sort key.
-        const uint32_t key = keys ? (q.light & 7u) * kQueryCells + cell128(S, q.origin) : 0u;
+        // w of the direction: the query's coherence sort key, counted here so
+        // that the sort needs no histogram pass over the queries.
+        uint32_t key = 0;
+        if (bits) {
+            key = ((q.light & 7u) << (3u * bits)) | query_cell(S, q.origin, bits);
+            atomicAdd(&V.sort_hist[key], 1u);
+        }
         V.ts.queue_o[slot] = make_float4(q.origin.x, q.origin.y, q.origin.z, q.limit);
         V.ts.queue_d[slot] = make_float4(q.direction.x, q.direction.y, q.direction.z, lux::as_float(key));
         V.ts.slot_contrib[slot] = make_float4(q.contribution.x, q.contribution.y, q.contribution.z, (float)q.group);
@@ -863,7 +884,6 @@ __device__ __forceinline__ void shade_warp(const ViewDevice &V, const FrameParam
         const size_t slot = slot0 + (uint32_t)(__ffs(m) - 1);
         if (qi < F.queue_capacity) {
             V.ts.query_slot[qi] = (uint32_t)slot;
-            if (keys) V.sort_keys[qi] = lux::as_uint(V.ts.queue_d[slot].w);
         } else {
             V.ts.queue_result[slot] = 2;  // list overflow: unsupported
         }
@@ -896,7 +916,7 @@ __global__ void __launch_bounds__(128, LUX_REFILL_MIN_BLOCKS) shadow_refill_kern
     unsigned long long st[7] = {0, 0, 0, 0, 0, 0, 0};
     lux::TraceCounters cn{0, 0, 0};
     auto gen = [&](uint32_t i, f3 &o, f3 &d, float &tmin, float &limit) {
-        uint32_t qi = V.ts.query_slot[V.query_order ? V.query_order[i] : i];
+        uint32_t qi = (V.query_order ? V.query_order : V.ts.query_slot)[i];
         float4 a = V.ts.queue_o[qi], b = V.ts.queue_d[qi];
         o = f3{a.x, a.y, a.z};
         d = f3{b.x, b.y, b.z};
@@ -904,7 +924,7 @@ __global__ void __launch_bounds__(128, LUX_REFILL_MIN_BLOCKS) shadow_refill_kern
         limit = a.w;
     };
     auto done = [&](uint32_t i, const lux::Hit &sh) {
-        uint32_t qi = V.ts.query_slot[V.query_order ? V.query_order[i] : i];
+        uint32_t qi = (V.query_order ? V.query_order : V.ts.query_slot)[i];
         V.ts.queue_result[qi] = sh.tri != lux::kEmpty ? 1 : ((sh.errors & lux::kQueryUnsupported) ? 2 : 0);
         st[kStatShadow] += 1;
     };
@@ -925,7 +945,7 @@ __device__ __forceinline__ void shadow_query_warp(const ViewDevice &V, const Sce
     uint32_t qi = 0;
     float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f), b = a;
     if (valid) {
-        qi = V.ts.query_slot[V.query_order ? V.query_order[i] : i];
+        qi = (V.query_order ? V.query_order : V.ts.query_slot)[i];
         a = V.ts.queue_o[qi];
         b = V.ts.queue_d[qi];
     }
@@ -2809,6 +2829,7 @@ constexpr int kTimingEvents = 7;
 
 struct LuxView {
     LuxContext *ctx = nullptr;
+    uint32_t sort_bins = 0;  // bins of the coherence-sort buffers
     LuxTuning tuning{0, 0, 16, 16, 0, 0, 64, 0, 32, 0};
     bool timing = false;
     cudaEvent_t ev[kTimingEvents] = {};
@@ -2875,9 +2896,9 @@ static void cache_buffers_free(LuxView *v) {
 }
 
 // Device-wide scan scratch for the counting-sort histogram.
-static size_t scan_temp_bytes() {
+static size_t scan_temp_bytes(uint32_t bins) {
     size_t bytes = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, bytes, (const uint32_t *)nullptr, (uint32_t *)nullptr, (int)kSortBins);
+    cub::DeviceScan::ExclusiveSum(nullptr, bytes, (const uint32_t *)nullptr, (uint32_t *)nullptr, (int)bins);
     return std::max<size_t>(bytes, 16);
 }
 
@@ -2961,34 +2982,58 @@ static lux_status view_alloc(LuxView *v) {
     return lux_cuda_check(ctx, (int)cudaGetLastError(), "view allocation");
 }
 
-// Coherence-sort buffers (keys and permutation per ray or query, the 2^24-bin
-// histogram and its offsets, the scan scratch: about 8 x max_rays x 16 B +
-// 128 MiB), allocated when a frame of the view first runs with sort_rays or
-// sort_queries set; views that never sort do not hold them.
-static lux_status ensure_sort_buffers(LuxView *v) {
+// Coherence-sort buffers: the processing order (4 bytes per ray and sample),
+// ray keys (4 per ray), and two arrays of `bins` counters with the scan
+// scratch, allocated when a frame of the view first needs them.
+static lux_status ensure_sort_buffers(LuxView *v, uint32_t bins) {
     ViewDevice &D = v->dev;
-    if (D.sort_hist) return LUX_OK;
-    const size_t items = (size_t)v->desc.max_rays * lux::kMaxNeeSamples;
-    D.scan_temp_bytes = scan_temp_bytes();
+    if (D.sort_hist && bins <= v->sort_bins) return LUX_OK;
+    if (D.sort_hist) {  // a finer grid than before
+        cudaStreamSynchronize(v->ctx->stream);
+        if (v->setup_stream) cudaStreamSynchronize(v->setup_stream);
+        cudaFree(D.sort_hist);
+        cudaFree(D.sort_offs);
+        cudaFree(D.scan_temp);
+        D.sort_hist = D.sort_offs = nullptr;
+        D.scan_temp = nullptr;
+    }
+    D.scan_temp_bytes = scan_temp_bytes(bins);
     struct A {
         void **p;
         size_t bytes;
     } allocs[] = {
-        {(void **)&D.sort_keys, items * sizeof(uint32_t)},
-        {(void **)&D.sort_perm, items * sizeof(uint32_t)},
-        {(void **)&D.sort_offs, (size_t)kSortBins * sizeof(uint32_t)},
+        {(void **)&D.sort_keys, (size_t)v->desc.max_rays * sizeof(uint32_t)},
+        {(void **)&D.sort_perm, (size_t)v->desc.max_rays * lux::kMaxNeeSamples * sizeof(uint32_t)},
+        {(void **)&D.sort_offs, (size_t)bins * sizeof(uint32_t)},
         {(void **)&D.scan_temp, D.scan_temp_bytes},
-        {(void **)&D.sort_hist, (size_t)kSortBins * sizeof(uint32_t)},  // last: marks the set complete
+        {(void **)&D.sort_hist, (size_t)bins * sizeof(uint32_t)},  // last: marks the set complete
     };
     for (auto &a : allocs) {
         if (*a.p) continue;
         if (cudaMalloc(a.p, std::max<size_t>(a.bytes, 16)) != cudaSuccess) {
             cudaGetLastError();
             *a.p = nullptr;
+            cudaFree(D.sort_offs);
+            cudaFree(D.scan_temp);
+            D.sort_offs = nullptr;
+            D.scan_temp = nullptr;
             return lux_fail(v->ctx, LUX_ERR_OUT_OF_MEMORY, "view: coherence-sort buffer allocation failed");
         }
     }
+    v->sort_bins = bins;
     return LUX_OK;
+}
+
+// Bits per axis of the origin grid the frame's visibility queries are ordered
+// on, 0 for none: about a bin per two queries, since finer bins than queries
+// order nothing and the bins themselves cost their clearing and their scan.
+// Without the tuning's flag only frames that can queue kOrderQueries or more
+// are ordered: below it the order's launches cost what the walks gain (961x541,
+// 130,000 rays, at most 1.4 M queries: 1189 us ordered, 1179 not; 1920x1080, 4.4 M
+// rays: 12.8 ms ordered, 15.4 not).
+static uint32_t query_order_bits(uint64_t queries, bool asked) {
+    if (queries < kOrderQueries && !asked) return 0u;
+    return queries >= (6u << 20) ? 7u : (queries >= (1u << 20) ? 6u : 5u);
 }
 
 extern "C" lux_status lux_view_create(LuxContext *ctx, const LuxViewDesc *desc, LuxView **out) {
@@ -3488,9 +3533,16 @@ static lux_status view_frame(LuxView *v, const LuxScene *scene, const LuxSetting
     }
     if (F.layout == LUX_LAYOUT_SPLIT && (uint64_t)rc->count * F.rays_per_receiver > v->desc.max_rays)
         return lux_fail(ctx, LUX_ERR_CAPACITY, "trace_merge: receivers x rays_per_receiver exceeds max_rays");
-    if (F.layout == LUX_LAYOUT_SPLIT && (v->tuning.sort_rays || v->tuning.sort_queries)) {
-        lux_status sb = ensure_sort_buffers(v);  // before any work of the frame is queued
-        if (sb != LUX_OK) return sb;
+    uint32_t query_bits = 0;
+    if (F.layout == LUX_LAYOUT_SPLIT) {  // before any work of the frame is queued
+        const bool asked = v->tuning.sort_queries != 0u;
+        query_bits = query_order_bits(most_queries(F, scene, (uint64_t)rc->count * F.rays_per_receiver), asked);
+        const uint32_t bins = std::max(query_bits ? query_bins(query_bits) : 0u, v->tuning.sort_rays ? kRaySortBins : 0u);
+        if (bins) {
+            lux_status sb = ensure_sort_buffers(v, bins);
+            if (sb != LUX_OK && (asked || v->tuning.sort_rays)) return sb;
+            if (sb != LUX_OK) query_bits = 0;  // no room: in the order they come
+        }
     }
     const ViewDevice &D = v->dev;
     cudaStream_t st = ctx->stream;
@@ -3528,6 +3580,10 @@ static lux_status view_frame(LuxView *v, const LuxScene *scene, const LuxSetting
         cudaEventRecord(v->seeded, st);
         cudaStreamWaitEvent(v->setup_stream, v->seeded, 0);
         enqueue_layout(v, F, v->setup_stream);
+        // The query order's bins are cleared here too (the ray order uses the
+        // same ones beside this stream).
+        if (query_bits && !v->tuning.sort_rays)
+            cudaMemsetAsync(D.sort_hist, 0, (size_t)query_bins(query_bits) * 4, v->setup_stream);
         cudaEventRecord(v->laid_out, v->setup_stream);
         forked = true;
     } else {
@@ -3538,14 +3594,15 @@ static lux_status view_frame(LuxView *v, const LuxScene *scene, const LuxSetting
         uint32_t rays = rc->count * F.rays_per_receiver;
         if (rays) {
             const LuxTuning &T = v->tuning;
+            const int most = ctx->sm_count * 8;
             ViewDevice Dr = D;  // ray pass view: optional coherence order of interval rays
-            Dr.sort_keys = nullptr;
             if (T.sort_rays) {
+                const int blocks = blocks_for(rays, 256, most);
                 cudaMemsetAsync(D.sort_hist, 0, (size_t)kRaySortBins * 4, st);
-                ray_keys_kernel<<<ctx->sm_count * 8, 256, 0, st>>>(D, F, scene->view, pos, nrm, rays);
-                sort_hist_kernel<<<ctx->sm_count * 8, 256, 0, st>>>(D, nullptr, rays);
+                ray_keys_kernel<<<blocks, 256, 0, st>>>(D, F, scene->view, pos, nrm, rays);
+                sort_hist_kernel<<<blocks, 256, 0, st>>>(D, rays);
                 enqueue_sort_scan(D, kRaySortBins, st);
-                sort_scatter_kernel<<<ctx->sm_count * 8, 256, 0, st>>>(D, nullptr, rays);
+                sort_scatter_kernel<<<blocks, 256, 0, st>>>(D, rays);
                 Dr.ray_order = D.sort_perm;
             }
             const bool cached = v->cache_alloc && v->cache.cutoff_level < F.levels;
@@ -3576,17 +3633,17 @@ static lux_status view_frame(LuxView *v, const LuxScene *scene, const LuxSetting
                     Dr, F, scene->view, pos, nrm, rays, tile_of(T));
             }
             if (forked) cudaStreamWaitEvent(st, v->laid_out, 0);  // join the setup stream
-            ViewDevice Dq = D;  // query pass view: keys written by shade, optional order
-            if (!T.sort_queries) Dq.sort_keys = nullptr;
+            ViewDevice Dq = D;  // query pass view: keys counted by shade, optional order
+            Dq.query_bits = query_bits;
+            if (query_bits && (!forked || T.sort_rays))
+                cudaMemsetAsync(D.sort_hist, 0, (size_t)query_bins(query_bits) * 4, st);
             launch_shade(ctx, Dq, F, scene, rays, false, st);
-            if (T.sort_queries) {
-                cudaMemsetAsync(D.sort_hist, 0, (size_t)kSortBins * 4, st);
-                sort_hist_kernel<<<ctx->sm_count * 8, 256, 0, st>>>(D, D.ts.queue_count, F.queue_capacity);
-                enqueue_sort_scan(D, kSortBins, st);
-                sort_scatter_kernel<<<ctx->sm_count * 8, 256, 0, st>>>(D, D.ts.queue_count, F.queue_capacity);
+            const uint64_t queries = most_queries(F, scene, rays);
+            if (query_bits) {
+                enqueue_sort_scan(D, query_bins(query_bits), st);
+                query_scatter_kernel<<<blocks_for(queries, 256, most), 256, 0, st>>>(D, F.queue_capacity);
                 Dq.query_order = D.sort_perm;
             }
-            const uint64_t queries = most_queries(F, scene, rays);
             if (T.shadow_mode == 1)
                 shadow_refill_kernel<<<trace_blocks(ctx, T.shadow_blocks_per_sm, 32u, queries), 128, 0, st>>>(
                     Dq, F, scene->view);
@@ -3845,8 +3902,10 @@ extern "C" lux_status lux_view_set_tuning(LuxView *v, const LuxTuning *t) {
         t->fused_trace > 1)
         return lux_fail(v->ctx, LUX_ERR_INVALID_ARGUMENT, "set_tuning: value out of range");
     v->tuning = *t;
-    if (t->sort_queries || t->sort_rays) return ensure_sort_buffers(v);
-    return LUX_OK;
+    const uint64_t queries = (uint64_t)v->desc.max_rays * lux::kMaxNeeSamples;  // of the view's largest frame
+    const uint32_t bins = std::max(t->sort_queries ? query_bins(query_order_bits(queries, true)) : 0u,
+                                   t->sort_rays ? kRaySortBins : 0u);
+    return bins ? ensure_sort_buffers(v, bins) : LUX_OK;
 }
 
 extern "C" lux_status lux_view_get_tuning(const LuxView *v, LuxTuning *t) {
@@ -4531,7 +4590,7 @@ extern "C" lux_status lux_batch_trace_merge(LuxBatch *b, const LuxBatchJob *jobs
         BatchJob &J = h[j];
         std::memset(&J, 0, sizeof J);
         J.V = jobs[j].view->dev;
-        J.V.sort_keys = nullptr;
+        J.V.query_bits = 0;
         J.V.ray_order = nullptr;
         J.V.query_order = nullptr;
         J.F = F;
