@@ -58,6 +58,10 @@
 #ifndef LUX_BATCH_MIN_BLOCKS
 #define LUX_BATCH_MIN_BLOCKS 6
 #endif
+#ifndef LUX_SMALL_DIRECTORY
+#define LUX_SMALL_DIRECTORY 32768u
+#endif
+constexpr uint32_t kSmallDirectory = LUX_SMALL_DIRECTORY;  // slots per level
 // Visibility queries a frame must be able to queue for them to be ordered
 // without the tuning asking for it.
 #ifndef LUX_ORDER_QUERIES
@@ -162,7 +166,8 @@ struct ViewDevice {
     uint32_t *receiver_cell;        // [levels][max_receivers]
     uint32_t *receiver_lod;         // [max_receivers] the LOD each receiver's rays deposit into
     uint32_t *receiver_ordinal;     // [max_receivers] the receiver's place in the sample sequence
-    unsigned long long *order_keys; // [2][max_receivers] sequence-order sort keys (in, out)
+    unsigned long long *order_keys; // [2][max_receivers] sequence-order sort keys (in, out; 32-bit when ranked)
+    uint32_t *cell_rank;            // [max_cells] place of each cascade-0 cell in the sequence order
     uint32_t *order_vals;           // [2][max_receivers] receiver indices (in, out)
     void *order_temp;               // radix-sort scratch
     size_t order_temp_bytes;
@@ -344,21 +349,29 @@ __device__ __forceinline__ void seed_cell(const ViewDevice &V, const FrameParams
         return;
     }
     unsigned long long key = lux::pack_cell(x, y, z, lod);
+    // One lane per distinct cell of the warp inserts it: neighbouring receivers
+    // share their coarse cells, and all of a level's atomics on one slot run
+    // one after another.
+    const unsigned active = __activemask();
+    const unsigned peers = __match_any_sync(active, key) & __match_any_sync(active, level);
+    if ((uint32_t)(__ffs(peers) - 1) != (threadIdx.x & 31u)) return;
     unsigned long long *keys = V.dir_keys + (size_t)level * F.dir_capacity;
     uint32_t slot = lux::hash_key(x, y, z, (int32_t)(level | (lod << 18)), F.dir_capacity);
     for (uint32_t attempt = 0; attempt < F.dir_capacity; ++attempt) {
-        unsigned long long prev = atomicCAS(&keys[slot], lux::kEmptyCell, key);
+        unsigned long long prev = *(volatile unsigned long long *)&keys[slot];
+        if (prev == lux::kEmptyCell) prev = atomicCAS(&keys[slot], lux::kEmptyCell, key);
         if (prev == lux::kEmptyCell || prev == key) return;
         slot = (slot + 1u) & (F.dir_capacity - 1u);
     }
     atomicOr(V.error_flags, LUX_VIEW_ERR_CELL_CAPACITY);
 }
 
-// Item i = receiver x levels + level.
+// Item i = level x receivers + receiver: a warp takes neighbouring receivers of
+// one level.
 __device__ __forceinline__ void seed_insert_item(const ViewDevice &V, const FrameParams &F, const float4 *__restrict__ pos,
                                                  unsigned long long i) {
     if (i >= (unsigned long long)F.receivers * F.levels) return;
-    uint32_t r = (uint32_t)(i / F.levels), level = (uint32_t)(i % F.levels);
+    const uint32_t level = (uint32_t)(i / F.receivers), r = (uint32_t)(i - (unsigned long long)level * F.receivers);
     float4 p = pos[r];
     if (F.sparse && p.w == 0.0f) return;
     const f3 q{p.x, p.y, p.z};
@@ -393,6 +406,7 @@ __device__ __forceinline__ void seed_assign_item(const ViewDevice &V, const Fram
     lux::unpack_cell(key, x, y, z, lod);
     V.cell_keys[(size_t)level * F.cell_capacity + id] = make_int4(x, y, z, (int32_t)((level << 12) | (lod << 18)));
     V.cell_last[(size_t)level * F.cell_capacity + id] = F.shade.frame;
+    if (level == 0u) V.cell_rank[id] = 0u;
 }
 
 __global__ void seed_assign_kernel(ViewDevice V, FrameParams F) {
@@ -425,13 +439,48 @@ __global__ void ordinal_kernel(ViewDevice V, const uint32_t *__restrict__ sorted
         V.receiver_ordinal[sorted[j]] = j;
 }
 
-// Item i = receiver x levels + level; the receiver's sequence key and index
-// go to keys[r], vals[r].
+// The sequence order by cells: receivers of one cell are consecutive and in
+// index order, so a receiver's key can be its cell's place among the frame's
+// cascade-0 cells, a number of few bits, instead of the cell's 62-bit key: the
+// radix sort then takes 2 passes where it took 8 (14,400 receivers: 100 us with
+// its clears, 30 now with the ranking).  The place is a count over all pairs
+// of cells, which is cheap while the cells are few (kRankedCells); above that
+// the 62-bit keys are sorted.  Block (x, y): 256 cells, two per thread, against
+// 256.
+constexpr uint32_t kRankedCells = 16384, kRankChunk = 256;
+__global__ void __launch_bounds__(128) cell_rank_kernel(ViewDevice V, FrameParams F) {
+    __shared__ __align__(16) unsigned long long key[kRankChunk];
+    const uint32_t cells = min(V.cell_count[0], F.cell_capacity);
+    const uint32_t c = blockIdx.x * 256u + threadIdx.x, first = blockIdx.y * kRankChunk;
+    if (blockIdx.x * 256u >= cells || first >= cells) return;
+    const uint32_t n = min(kRankChunk, cells - first);
+    auto key_of = [&](uint32_t cell) {
+        const int4 q = V.cell_keys[cell];
+        return sequence_key(q.x, q.y, q.z, lux::key_lod(q.w));
+    };
+    for (uint32_t k = threadIdx.x; k < kRankChunk; k += 128u) key[k] = k < n ? key_of(first + k) : ~0ull;  // before no cell
+    __syncthreads();
+    if (c >= cells) return;
+    const unsigned long long a = key_of(c), b = c + 128u < cells ? key_of(c + 128u) : 0ull;
+    uint32_t before_a = 0, before_b = 0;
+#pragma unroll 8
+    for (uint32_t k = 0; k < kRankChunk; k += 2u) {
+        const ulonglong2 two = *reinterpret_cast<const ulonglong2 *>(&key[k]);
+        before_a += (two.x < a ? 1u : 0u) + (two.y < a ? 1u : 0u);
+        before_b += (two.x < b ? 1u : 0u) + (two.y < b ? 1u : 0u);
+    }
+    if (before_a) atomicAdd(&V.cell_rank[c], before_a);
+    if (before_b) atomicAdd(&V.cell_rank[c + 128u], before_b);
+}
+
+// Item i = level x receivers + receiver; the receiver's sequence key and index
+// go to keys[r], vals[r] (kRanked: its cell's rank to the 32-bit keys).
+template <bool kRanked>
 __device__ __forceinline__ void seed_lookup_item(const ViewDevice &V, const FrameParams &F,
                                                  const float4 *__restrict__ pos, unsigned long long i,
                                                  unsigned long long *keys, uint32_t *vals) {
     if (i >= (unsigned long long)F.receivers * F.levels) return;
-    uint32_t r = (uint32_t)(i / F.levels), level = (uint32_t)(i % F.levels);
+    const uint32_t level = (uint32_t)(i / F.receivers), r = (uint32_t)(i - (unsigned long long)level * F.receivers);
     float4 p = pos[r];
     const f3 q{p.x, p.y, p.z};
     // The variant this receiver's rays deposit into (one trace per
@@ -443,18 +492,23 @@ __device__ __forceinline__ void seed_lookup_item(const ViewDevice &V, const Fram
     if (level == 0u) V.receiver_lod[r] = lod;
     int32_t x, y, z;
     cell_of(F, level, q, x, y, z, lod);
+    const bool absent = F.sparse && p.w == 0.0f;
+    const uint32_t cell = absent ? lux::kEmpty : cell_id(V, F, level, x, y, z, lod);
     if (level == 0u) {
-        keys[r] = F.sparse && p.w == 0.0f ? ~0ull : sequence_key(x, y, z, lod);
+        if (kRanked)  // an absent receiver sorts last
+            reinterpret_cast<uint32_t *>(keys)[r] = cell == lux::kEmpty ? 0xffffffffu : V.cell_rank[cell];
+        else
+            keys[r] = absent ? ~0ull : sequence_key(x, y, z, lod);
         vals[r] = r;
     }
-    V.receiver_cell[(size_t)level * F.receivers + r] =
-        F.sparse && p.w == 0.0f ? lux::kEmpty : cell_id(V, F, level, x, y, z, lod);
+    V.receiver_cell[(size_t)level * F.receivers + r] = cell;
 }
 
+template <bool kRanked>
 __global__ void seed_lookup_kernel(ViewDevice V, FrameParams F, const float4 *__restrict__ pos) {
     size_t n = (size_t)F.receivers * F.levels;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        seed_lookup_item(V, F, pos, i, V.order_keys, V.order_vals);
+        seed_lookup_item<kRanked>(V, F, pos, i, V.order_keys, V.order_vals);
 }
 
 // Per-level record offsets; the entry capacity bounds the whole frame.
@@ -988,7 +1042,10 @@ __global__ void __launch_bounds__(128, kFlat ? LUX_FLAT_SHADOW_MIN_BLOCKS : LUX_
 // Next-event sum in sample order (plus the multi-bounce term with
 // `feedback`); false when the ray's query is unsupported.
 __device__ __forceinline__ bool ray_radiance(const ViewDevice &V, uint32_t ray, f3 &radiance, bool feedback = false) {
-    float4 b = V.ts.ray_base[ray];
+    // A ray's sixteen results are one 16-byte load; contributions are read
+    // for the visible samples only, four loads at a time.
+    const float4 b = V.ts.ray_base[ray];
+    const uint4 results = reinterpret_cast<const uint4 *>(V.ts.queue_result)[ray];
     const uint32_t packed = lux::as_uint(b.w);
     if (packed == lux::kEmpty) return false;
     // The emissive samples (averaged), the environment samples (averaged over
@@ -996,20 +1053,37 @@ __device__ __forceinline__ bool ray_radiance(const ViewDevice &V, uint32_t ray, 
     const uint32_t count = packed & 31u, conventional = (packed >> 5) & 15u;
     const uint32_t environment = ((packed >> 9) & 1u) != 0u ? count : 0u;
     const uint32_t used = packed >> 16;
+    const uint32_t word[4] = {results.x, results.y, results.z, results.w};
+    uint32_t visible = 0, unsupported = 0;  // a bit per sample
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        visible |= (((__vcmpeq4(word[k], 0u) & 0x01010101u) * 0x01020408u) >> 24) << (4 * k);
+        unsupported |= (((__vcmpeq4(word[k], 0x02020202u) & 0x01010101u) * 0x01020408u) >> 24) << (4 * k);
+    }
+    if (unsupported & used) return false;
+    visible &= used;
     f3 sum{0.0f, 0.0f, 0.0f}, esum{0.0f, 0.0f, 0.0f}, csum{0.0f, 0.0f, 0.0f};
-    for (uint32_t s = 0; s < count + environment + conventional && s < lux::kMaxNeeSamples; ++s) {
-        if (!(used & (1u << s))) continue;
-        size_t slot = (size_t)ray * lux::kMaxNeeSamples + s;
-        uint8_t r = V.ts.queue_result[slot];
-        if (r == 2) return false;
-        if (r == 1) continue;
-        float4 c = V.ts.slot_contrib[slot];
-        if (s < count)
-            sum = f3{sum.x + c.x, sum.y + c.y, sum.z + c.z};
-        else if (s < count + environment)
-            esum = f3{esum.x + c.x, esum.y + c.y, esum.z + c.z};
-        else
-            csum = f3{csum.x + c.x, csum.y + c.y, csum.z + c.z};
+    const float4 *contrib = V.ts.slot_contrib + (size_t)ray * lux::kMaxNeeSamples;
+    while (visible) {
+        uint32_t at[4], n = 0;
+        float4 c[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            at[k] = visible ? (uint32_t)__ffs(visible) - 1u : 0u;
+            n += visible ? 1u : 0u;
+            visible &= visible - 1u;
+            c[k] = (uint32_t)k < n ? contrib[at[k]] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if ((uint32_t)k >= n) break;
+            if (at[k] < count)
+                sum = f3{sum.x + c[k].x, sum.y + c[k].y, sum.z + c[k].z};
+            else if (at[k] < count + environment)
+                esum = f3{esum.x + c[k].x, esum.y + c[k].y, esum.z + c[k].z};
+            else
+                csum = f3{csum.x + c[k].x, csum.y + c[k].y, csum.z + c[k].z};
+        }
     }
     float4 e = feedback ? V.ts.ray_extra[ray] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     f3 extra{e.x, e.y, e.z};
@@ -1025,16 +1099,17 @@ __device__ __forceinline__ void deposit_split_ray(const ViewDevice &V, const Fra
                                                   unsigned long long st[7]) {
     uint32_t i = ray / F.rays_per_receiver, k = ray % F.rays_per_receiver;
     if (F.sparse && V.receiver_cell[i] == lux::kEmpty) return;  // absent receiver: no ray
+    // What does not depend on the radiance is loaded before it.
+    const float4 n4 = nrm[i];
+    const float t = V.ts.ray_o[ray].w;
+    f3 dir;
+    float u, v;
+    split_direction(V, F, frame, i, k, f3{n4.x, n4.y, n4.z}, dir, u, v);
     f3 radiance;
     if (!ray_radiance(V, ray, radiance, F.shade.feedback != 0u)) {
         st[kStatUnsupported] += 1;
         return;
     }
-    float4 n4 = nrm[i];
-    f3 dir;
-    float u, v;
-    split_direction(V, F, frame, i, k, f3{n4.x, n4.y, n4.z}, dir, u, v);
-    float t = V.ts.ray_o[ray].w;
     // splitIntervalContainsHit at the receiver's LOD (ends scale by 2^lod,
     // shaders/split.slang:224-236).
     const float ls = F.lod_enabled ? lux::lod_scale(V.receiver_lod[i]) : 1.0f;
@@ -1702,37 +1777,144 @@ __global__ void __launch_bounds__(LUX_MERGE_THREADS, LUX_MERGE_MIN_BLOCKS)
 __global__ void __launch_bounds__(256, LUX_MERGE_OWN_MIN_BLOCKS) merge_own_list_kernel(ViewDevice V, FrameParams F,
                                                                                       HistoryDevice H) {
     if (*V.error_flags) return;
+    // All levels are one range (level bases are consecutive), so a small
+    // frame's levels do not run one latency after another.  A warp whose 32
+    // records straddle two levels appends them level by level.
     const uint32_t lane = threadIdx.x & 31u;
-    for (uint32_t l = 0; l < F.levels; ++l) {
-        const uint32_t dirs = F.dirs[l];
-        const unsigned long long n = (unsigned long long)V.cell_count[l] * dirs, base = V.level_base[l];
-        for (unsigned long long r = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; r < n;
-             r += (unsigned long long)gridDim.x * blockDim.x) {
-            uint32_t cell, d;
-            record_cell(r, dirs, cell, d);
-            MergeOwn own;
-            const bool children = merge_own(V, F, H, l, base, dirs, cell, d, own);
-            if (!children) merge_finish(V, F, l, base, dirs, cell, d, own, false);
-            const unsigned active = __activemask();
-            const unsigned want = __ballot_sync(active, children);
-            if (want) {
-                const uint32_t leader = (uint32_t)__ffs(want) - 1u;
-                uint32_t at = 0;
-                if (lane == leader) at = atomicAdd(&V.pass_count[l], (uint32_t)__popc(want));
-                at = __shfl_sync(active, at, leader);
-                if (children) V.pass_list[base + at + (uint32_t)__popc(want & ((1u << lane) - 1u))] = (uint32_t)r;
-            }
+    uint32_t l = 0;
+    unsigned long long base = 0, end = (unsigned long long)V.cell_count[0] * F.dirs[0];
+    for (unsigned long long e = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;;
+         e += (unsigned long long)gridDim.x * blockDim.x) {
+        while (e >= end) {
+            if (++l >= F.levels) return;
+            base = end;
+            end += (unsigned long long)V.cell_count[l] * F.dirs[l];
+        }
+        const unsigned long long r = e - base;
+        uint32_t cell, d;
+        record_cell(r, F.dirs[l], cell, d);
+        MergeOwn own;
+        const bool children = merge_own(V, F, H, l, base, F.dirs[l], cell, d, own);
+        if (!children) merge_finish(V, F, l, base, F.dirs[l], cell, d, own, false);
+        unsigned want = __ballot_sync(__activemask(), children);
+        if (children) {
+            want = __match_any_sync(want, l);
+            const uint32_t leader = (uint32_t)__ffs(want) - 1u;
+            uint32_t at = 0;
+            if (lane == leader) at = atomicAdd(&V.pass_count[l], (uint32_t)__popc(want));
+            at = __shfl_sync(want, at, leader);
+            V.pass_list[base + at + (uint32_t)__popc(want & ((1u << lane) - 1u))] = (uint32_t)r;
         }
     }
 }
 
-// The children pass of one level over its listed records.
+// merge_children_record by four lanes, one child of the record each: a lane's
+// eight corner records are loaded before any is used, where one lane per
+// record ran through its corners with four loads in flight at a time.  Per
+// child the corners are summed in interpolate_children's order and the four
+// children in merge_finish's, so the record is the same bit for bit.  Every
+// lane of the warp calls it; lanes with !valid have no record.
+__device__ __forceinline__ void merge_children_quad(const ViewDevice &V, const FrameParams &F, uint32_t level,
+                                                    unsigned long long base, uint32_t dirs, uint32_t record,
+                                                    bool valid) {
+    const uint32_t child = threadIdx.x & 3u;
+    const unsigned long long e = base + record;
+    float2 mass = make_float2(0.0f, 0.0f);
+    float4 raw = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float4 v = raw;
+    if (valid) {
+        uint32_t cell, d;
+        record_cell(record, dirs, cell, d);
+        mass = V.mass[e];
+        raw = V.raw[e];
+        const size_t ci = (size_t)level * F.cell_capacity + cell;
+        const uint4 *cid = reinterpret_cast<const uint4 *>(V.corner_ids + ci * 8);  // 32-byte rows
+        const uint4 c0 = __ldg(cid), c1 = __ldg(cid + 1);
+        const float4 frac = __ldg(V.corner_frac + ci);
+        const uint32_t ids[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+        const uint32_t x = d % F.columns[level], y = d / F.columns[level];
+        const uint32_t fine = (x * 2u + (child & 1u)) + (y * 2u + (child >> 1)) * F.columns[level + 1];
+        const unsigned long long child_base = V.level_base[level + 1] + fine;
+        const uint32_t child_dirs = F.dirs[level + 1];
+        float4 s[8];
+#pragma unroll
+        for (uint32_t corner = 0; corner < 8u; ++corner)
+            s[corner] = ids[corner] == lux::kEmpty
+                            ? make_float4(0.0f, 0.0f, 0.0f, 0.0f)
+                            : __ldg(V.merged + child_base + (unsigned long long)ids[corner] * child_dirs);
+        float sx = 0.0f, sy = 0.0f, sz = 0.0f, total = 0.0f, potential = 0.0f;
+#pragma unroll
+        for (uint32_t corner = 0; corner < 8u; ++corner) {
+            const float ax = (corner & 1u) == 0u ? 1.0f - frac.x : frac.x;
+            const float ay = ((corner >> 1) & 1u) == 0u ? 1.0f - frac.y : frac.y;
+            const float az = (corner >> 2) == 0u ? 1.0f - frac.z : frac.z;
+            const float w = (ax * ay) * az;
+            if (!(w > 0.0f)) continue;
+            potential += w;
+            const float4 t = s[corner];  // a missing corner has no support
+            if (t.w > 0.0f && isfinite(t.x) && isfinite(t.y) && isfinite(t.z) && isfinite(t.w)) {
+                const float sw = w * lux::saturate(t.w);
+                sx = sx + t.x * sw;
+                sy = sy + t.y * sw;
+                sz = sz + t.z * sw;
+                total += sw;
+            }
+        }
+        if (total > 0.0f) {
+            const float support = lux::saturate(total / fmaxf(potential, 1e-8f));
+            if (support > 0.0f)
+                v = make_float4((sx / total) * support, (sy / total) * support, (sz / total) * support, support);
+        }
+    }
+    float cx = 0.0f, cy = 0.0f, cz = 0.0f, csup = 0.0f;
+#pragma unroll
+    for (uint32_t k = 0; k < 4u; ++k) {
+        const uint32_t from = (threadIdx.x & 28u) + k;
+        cx = cx + __shfl_sync(0xffffffffu, v.x, from);
+        cy = cy + __shfl_sync(0xffffffffu, v.y, from);
+        cz = cz + __shfl_sync(0xffffffffu, v.z, from);
+        csup = csup + __shfl_sync(0xffffffffu, v.w, from);
+    }
+    const float transmittance = lux::saturate(raw.w);
+    // Listed records pass light on; one that does not was finished before.
+    if (!valid || child != 0u || !(mass.y > 0.0f) || !(transmittance > 0.0f)) return;
+    float support = mass.x > 0.0f ? 1.0f - transmittance : 0.0f;
+    float rx = 0.0f, ry = 0.0f, rz = 0.0f;
+    if (support > 0.0f) {
+        rx = raw.x;
+        ry = raw.y;
+        rz = raw.z;
+    }
+    if (csup > 0.0f) {
+        rx = rx + (transmittance * cx) * 0.25f;
+        ry = ry + (transmittance * cy) * 0.25f;
+        rz = rz + (transmittance * cz) * 0.25f;
+        support = support + (transmittance * csup) * 0.25f;
+    }
+    V.merged[e] = support > 0.0f ? make_float4(rx / support, ry / support, rz / support, lux::saturate(support))
+                                 : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+}
+
+// The children pass of one level over its listed records: four lanes per
+// record while that fits the launch at once (a short list is one chain of
+// loads: 33 -> 19 us for the three levels of a 640x360 frame), else a lane per
+// record, which executes half the instructions (386 us against 448 for the
+// seven levels at 1280x720).
 __global__ void __launch_bounds__(LUX_MERGE_THREADS, LUX_MERGE_MIN_BLOCKS)
     merge_children_list_kernel(ViewDevice V, FrameParams F, uint32_t level) {
     if (*V.error_flags) return;
     const uint32_t dirs = F.dirs[level], n = V.pass_count[level];
     const unsigned long long base = V.level_base[level];
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const uint32_t thread = blockIdx.x * blockDim.x + threadIdx.x, threads = gridDim.x * blockDim.x;
+    if (n <= threads / 4u) {
+        const uint32_t i = thread >> 2;
+        if ((i & ~7u) >= n) return;  // whole warps
+        const bool valid = i < n;
+        const uint32_t record = valid ? __ldg(V.pass_list + base + i) : 0u;
+        merge_children_quad(V, F, level, base, dirs, record, valid);
+        return;
+    }
+    for (uint32_t i = thread; i < n; i += threads) {
         uint32_t cell, d;
         record_cell(__ldg(V.pass_list + base + i), dirs, cell, d);
         merge_children_record(V, F, level, base, dirs, cell, d);
@@ -2310,7 +2492,7 @@ __global__ void batch_seed_lookup_kernel(const BatchJob *__restrict__ jobs, cons
                                          uint32_t n, unsigned long long *keys, uint32_t *vals) {
     const unsigned long long *recv = batch_row(dom, n, kRowRecv);
     for_batch_items(batch_row(dom, n, kRowSeed), n, [&](uint32_t j, unsigned long long i) {
-        seed_lookup_item(jobs[j].V, jobs[j].F, jobs[j].pos, i, keys + recv[j], vals + recv[j]);
+        seed_lookup_item<false>(jobs[j].V, jobs[j].F, jobs[j].pos, i, keys + recv[j], vals + recv[j]);
     });
 }
 
@@ -2908,14 +3090,21 @@ static size_t order_temp_bytes(uint32_t receivers) {
     cub::DeviceRadixSort::SortPairs(nullptr, bytes, (const unsigned long long *)nullptr, (unsigned long long *)nullptr,
                                     (const uint32_t *)nullptr, (uint32_t *)nullptr, (int)std::max(receivers, 1u), 0,
                                     62);
-    return std::max<size_t>(bytes, 16);
+    size_t ranked = 0;
+    cub::DeviceRadixSort::SortPairs(nullptr, ranked, (const uint32_t *)nullptr, (uint32_t *)nullptr,
+                                    (const uint32_t *)nullptr, (uint32_t *)nullptr, (int)std::max(receivers, 1u), 0,
+                                    32);
+    return std::max<size_t>(std::max(bytes, ranked), 16);
 }
 
 static lux_status view_alloc(LuxView *v) {
     LuxContext *ctx = v->ctx;
     const LuxViewDesc &d = v->desc;
     ViewDevice &D = v->dev;
+    // At most half full; small views' directories an eighth, since a frame of a
+    // few thousand receivers waits for the longest probe chain of each pass.
     v->dir_capacity = next_pow2(2ull * d.max_cells);
+    while (v->dir_capacity < kSmallDirectory && v->dir_capacity < 8ull * d.max_cells) v->dir_capacity *= 2u;
     size_t L = LUX_MAX_LEVELS;
     struct A {
         void **p;
@@ -2931,6 +3120,7 @@ static lux_status view_alloc(LuxView *v) {
         {(void **)&D.receiver_ordinal, (size_t)d.max_receivers * sizeof(uint32_t)},
         {(void **)&D.order_keys, 2 * (size_t)d.max_receivers * sizeof(unsigned long long)},
         {(void **)&D.order_vals, 2 * (size_t)d.max_receivers * sizeof(uint32_t)},
+        {(void **)&D.cell_rank, (size_t)d.max_cells * sizeof(uint32_t)},
         {(void **)&D.order_temp, order_temp_bytes(d.max_receivers)},
         {(void **)&D.corner_ids, L * (size_t)d.max_cells * 8 * sizeof(uint32_t)},
         {(void **)&D.corner_frac, L * (size_t)d.max_cells * sizeof(float4)},
@@ -3063,7 +3253,7 @@ extern "C" lux_status lux_view_destroy(LuxView *v) {
     if (!v) return LUX_OK;
     ViewDevice &D = v->dev;
     void *ptrs[] = {D.dir_keys, D.dir_ids, D.cell_keys, D.cell_count, D.level_base, D.receiver_cell, D.receiver_lod,
-                    D.receiver_ordinal, D.order_keys, D.order_vals, D.order_temp,
+                    D.receiver_ordinal, D.order_keys, D.order_vals, D.cell_rank, D.order_temp,
                     D.corner_ids,
                     D.corner_frac, D.accum, D.count, D.merged, D.raw, D.mass, D.hist_cell, D.cell_last,
                     D.retain_hist, D.retain_limit, D.tables, D.error_flags, D.stats,
@@ -3259,12 +3449,27 @@ static void enqueue_seed(LuxView *v, const FrameParams &F, const float4 *pos, cu
     if (F.receivers) {
         seed_insert_kernel<<<blocks_for(places, 256, most), 256, 0, st>>>(D, F, pos);
         seed_assign_kernel<<<blocks_for(slots, 256, most), 256, 0, st>>>(D, F);
-        seed_lookup_kernel<<<blocks_for(places, 256, most), 256, 0, st>>>(D, F, pos);
-        if (F.layout == LUX_LAYOUT_SPLIT) {  // the receivers' places in the sample sequence
+        // Cascade-0 cells the receivers can seed (two LODs in an overlap).
+        const uint64_t cells = std::min<uint64_t>(F.cell_capacity, (uint64_t)F.receivers * (F.lod_enabled ? 2u : 1u));
+        const bool split = F.layout == LUX_LAYOUT_SPLIT, ranked = split && cells <= kRankedCells;
+        if (ranked)
+            cell_rank_kernel<<<dim3((unsigned)((cells + 255) / 256), (unsigned)((cells + kRankChunk - 1) / kRankChunk)), 128,
+                               0, st>>>(D, F);
+        (ranked ? seed_lookup_kernel<true> : seed_lookup_kernel<false>)<<<blocks_for(places, 256, most), 256, 0, st>>>(
+            D, F, pos);
+        if (split) {  // the receivers' places in the sample sequence
             size_t bytes = D.order_temp_bytes;
-            cub::DeviceRadixSort::SortPairs(D.order_temp, bytes, D.order_keys, D.order_keys + v->desc.max_receivers,
-                                            D.order_vals, D.order_vals + v->desc.max_receivers, (int)F.receivers, 0,
-                                            62, st);
+            uint32_t *vals = D.order_vals, *sorted = D.order_vals + v->desc.max_receivers;
+            if (ranked) {
+                int bits = 1;  // ranks below `cells`, and all ones
+                while ((1ull << bits) < cells + 1) ++bits;
+                uint32_t *keys = reinterpret_cast<uint32_t *>(D.order_keys);
+                cub::DeviceRadixSort::SortPairs(D.order_temp, bytes, keys, keys + v->desc.max_receivers, vals, sorted,
+                                                (int)F.receivers, 0, bits, st);
+            } else {
+                cub::DeviceRadixSort::SortPairs(D.order_temp, bytes, D.order_keys, D.order_keys + v->desc.max_receivers,
+                                                vals, sorted, (int)F.receivers, 0, 62, st);
+            }
             ordinal_kernel<<<blocks_for(F.receivers, 256, most), 256, 0, st>>>(D, D.order_vals + v->desc.max_receivers,
                                                                               F.receivers);
         }
@@ -3300,7 +3505,7 @@ static void enqueue_merge(LuxView *v, const FrameParams &F, cudaStream_t st) {
     const HistoryDevice H = history_device(v);
     // Records bound every pass; a view's capacity is usually close to its use.
     const int own_blocks = blocks_for(F.entry_capacity, 256, most * 2);
-    const int child_blocks = blocks_for(F.entry_capacity, LUX_MERGE_THREADS, most * 512 / LUX_MERGE_THREADS);
+    const int child_blocks = blocks_for(4ull * F.entry_capacity, LUX_MERGE_THREADS, most * 512 / LUX_MERGE_THREADS);
     if (F.levels > 1 || F.history)
         merge_prep_kernel<<<blocks_for((uint64_t)F.cell_capacity * F.levels * 8u, 128, most), 128, 0, st>>>(D, F, H);
     // Record indices in the pass list are 32-bit (a level's records).
