@@ -15,8 +15,8 @@
 //  * The weights live in shared memory for the kernel's lifetime, packed by
 //    the Adam step in the same layout, once as W ([out][in]) for the forward
 //    pass and once as W^T for the backward data gradients.
-//  * Weight gradients g^T h are summed on the CUDA cores from the same
-//    shared tiles (fire-and-forget atomics into an FP32 gradient buffer).
+//  * Weight gradients g^T h are summed over a CTA's tiles in tensor memory
+//    and added once per CTA to an FP32 gradient buffer.
 //  * Every wait on the tensor cores is bounded; a wait that gives up sets an
 //    error flag, the CTA leaves its loop, and TMEM is freed.
 #include <cuda_bf16.h>
@@ -142,19 +142,14 @@ __device__ __forceinline__ void mbar_init(uint64_t *bar) {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
 
-// Every thread's view of one tensor-core round: the issuing thread has
-// committed, all threads wait (bounded), the answer is CTA-uniform.
-__device__ __forceinline__ bool wait_round(uint32_t bar, uint32_t &phase) {
-    bool ok = mbar_wait(bar, phase);
-    phase ^= 1u;
-    return __syncthreads_and(ok) != 0;
-}
-
-__device__ __forceinline__ void sync_for_mma() {
+// Operands in shared memory before the next chain, accumulators read before
+// they are overwritten; false (CTA-uniform) when a thread has given up a wait.
+__device__ __forceinline__ bool sync_for_mma(bool ok) {
     proxy_fence();
     tc_fence_before();
-    __syncthreads();
+    ok = __syncthreads_and(ok) != 0;
     tc_fence_after();
+    return ok;
 }
 
 // One layer: D[128 x N] = A[128 x K] * B[N x K]^T from packed shared tiles.
@@ -184,10 +179,6 @@ __device__ __forceinline__ void store_row64(bf16 *tile, uint32_t row, const floa
     }
 }
 
-__device__ __forceinline__ float bf16_at(const bf16 *tile, uint32_t row, uint32_t col) {
-    return __bfloat162float(tile[packed(row, col, kTile)]);
-}
-
 // ---- hash encoding ----------------------------------------------------------
 
 struct GridParams {
@@ -196,11 +187,18 @@ struct GridParams {
     uint32_t res[kLevelsMax];
 };
 
-__device__ __forceinline__ uint32_t grid_index(const GridParams &G, uint32_t level, uint32_t x, uint32_t y, uint32_t z) {
-    uint32_t stride = G.res[level] + 1u;
-    unsigned long long dense = (unsigned long long)stride * stride * stride;
-    if (dense <= G.table) return x + stride * (y + stride * z);
-    return (x * 1u ^ y * 2654435761u ^ z * 805459861u) & (G.table - 1u);
+// A vertex's entry in its level's table: x + stride (y + stride z) where the
+// whole grid fits the table, else the hash x ^ y p ^ z q; the y and z factors
+// are kept so that a cell's eight vertices cost two products.
+struct LevelIndex {
+    uint32_t y, z, mask;
+    bool dense;
+};
+__device__ __forceinline__ LevelIndex level_index(const GridParams &G, uint32_t level) {
+    const uint32_t stride = G.res[level] + 1u;
+    const bool dense = (unsigned long long)stride * stride * stride <= G.table;
+    return dense ? LevelIndex{stride, stride * stride, 0xffffffffu, true}
+                 : LevelIndex{2654435761u, 805459861u, G.table - 1u, false};
 }
 
 struct Corner {
@@ -220,10 +218,13 @@ __device__ __forceinline__ void level_corners(const GridParams &G, uint32_t leve
         i0[a] = (uint32_t)fl;
         f[a] = fminf(fmaxf(p - fl, 0.0f), 1.0f);
     }
+    const LevelIndex L = level_index(G, level);
+    const uint32_t hy = i0[1] * L.y, hz = i0[2] * L.z;
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
         uint32_t dx = k & 1, dy = (k >> 1) & 1, dz = (k >> 2) & 1;
-        c.index[k] = level * G.table + grid_index(G, level, i0[0] + dx, i0[1] + dy, i0[2] + dz);
+        const uint32_t x = i0[0] + dx, y = dy ? hy + L.y : hy, z = dz ? hz + L.z : hz;
+        c.index[k] = L.dense ? x + y + z : (x ^ y ^ z) & L.mask;
         c.weight[k] = (dx ? f[0] : 1.0f - f[0]) * (dy ? f[1] : 1.0f - f[1]) * (dz ? f[2] : 1.0f - f[2]);
     }
 }
@@ -259,69 +260,96 @@ __device__ __forceinline__ void sh16(float x, float y, float z, float *o) {
 // direction's 16 spherical-harmonic coefficients, normal, albedo, a
 // constant 1 (the first layer's bias), zeros.
 // n_dev (optional): a device count that caps n (compacted query lists).
-__global__ void encode_kernel(GridParams G, const LuxCacheSample *__restrict__ samples, uint32_t n,
-                              const uint32_t *__restrict__ n_dev, const __nv_bfloat162 *__restrict__ table,
-                              uint4 *__restrict__ out) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+// Four lanes per sample, four levels and two 16-byte pieces of the row each:
+// a small batch has four times the warps in flight that a thread per sample
+// gave, and a row is written as whole sectors.  Large batches are bound by
+// the L2 sectors of the 128 table reads per sample (69% of the L2's rate at
+// 500,009 random positions, 176 us); a warp per level, and 16-byte loads that
+// take both x neighbours, measured the same or less.
+__device__ __forceinline__ float2 bf16x2_floats(uint32_t v) {
+    return make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u));
+}
+__global__ void __launch_bounds__(128, 8)
+    encode_kernel(GridParams G, const LuxCacheSample *__restrict__ samples, uint32_t n,
+                  const uint32_t *__restrict__ n_dev, const uint32_t *__restrict__ table, uint4 *__restrict__ out) {
+    const unsigned long long t = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
     if (n_dev) n = min(n, *n_dev);
-    if (i >= n) return;
-    LuxCacheSample s = samples[i];
+    if (t >> 2 >= n) return;
+    const uint32_t i = (uint32_t)(t >> 2), q = (uint32_t)t & 3u;
+    const LuxCacheSample &s = samples[i];
     float u[3];
     unit_position(G, s, u);
-    float v[kIn];
+    uint32_t w[4];
 #pragma unroll
-    for (int k = 0; k < kIn; ++k) v[k] = 0.0f;
-    // Unrolled over the maximum level count so v[] stays in registers.
-#pragma unroll
-    for (uint32_t level = 0; level < (uint32_t)kLevelsMax; ++level) {
-        if (level >= G.levels) break;
-        Corner c;
-        level_corners(G, level, u, c);
+    for (uint32_t j = 0; j < 4u; ++j) {
+        const uint32_t level = q * 4u + j;
         float f0 = 0.0f, f1 = 0.0f;
+        if (level < G.levels) {
+            Corner c;
+            level_corners(G, level, u, c);
+            const uint32_t *row = table + (size_t)level * G.table;
+            uint32_t v[8];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            float2 t = __bfloat1622float2(table[c.index[k]]);
-            f0 += c.weight[k] * t.x;
-            f1 += c.weight[k] * t.y;
+            for (int k = 0; k < 8; ++k) v[k] = __ldg(row + c.index[k]);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const float2 f = bf16x2_floats(v[k]);
+                f0 += c.weight[k] * f.x;
+                f1 += c.weight[k] * f.y;
+            }
         }
-        v[2 * level] = f0;
-        v[2 * level + 1] = f1;
+        w[j] = pack_bf16x2(f0, f1);
     }
-    const int base = 2 * kLevelsMax;
-    sh16(s.direction[0], s.direction[1], s.direction[2], v + base);
-    v[base + 16] = s.normal[0];
-    v[base + 17] = s.normal[1];
-    v[base + 18] = s.normal[2];
-    v[base + 19] = s.albedo[0];
-    v[base + 20] = s.albedo[1];
-    v[base + 21] = s.albedo[2];
-    v[base + 22] = 1.0f;
+    uint4 *row = out + (size_t)i * (kIn / 8);
+    row[q] = make_uint4(w[0], w[1], w[2], w[3]);
+    float v[8];
+    if (q < 2u) {
+        float sh[16];
+        sh16(s.direction[0], s.direction[1], s.direction[2], sh);
 #pragma unroll
-    for (int q = 0; q < kIn / 8; ++q) {
-        uint4 w;
-        w.x = pack_bf16x2(v[q * 8 + 0], v[q * 8 + 1]);
-        w.y = pack_bf16x2(v[q * 8 + 2], v[q * 8 + 3]);
-        w.z = pack_bf16x2(v[q * 8 + 4], v[q * 8 + 5]);
-        w.w = pack_bf16x2(v[q * 8 + 6], v[q * 8 + 7]);
-        out[(size_t)i * (kIn / 8) + q] = w;
+        for (int k = 0; k < 8; ++k) v[k] = q ? sh[8 + k] : sh[k];
+    } else {
+        const bool last = q == 3u;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            v[k] = last ? 0.0f : s.normal[k];
+            v[3 + k] = last ? 0.0f : s.albedo[k];
+        }
+        v[6] = last ? 0.0f : 1.0f;
+        v[7] = 0.0f;
     }
+    row[4 + q] = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]),
+                            pack_bf16x2(v[6], v[7]));
 }
 
-// Scatter of the input gradient to the hash table (same corners).
-__global__ void encode_backward_kernel(GridParams G, const LuxCacheSample *__restrict__ samples, uint32_t n,
-                                       const float *__restrict__ dx, float2 *__restrict__ grad) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    LuxCacheSample s = samples[i];
+// Scatter of the input gradient to the hash table (same corners), a lane per
+// sample and level.  Bound by the rate of the atomics, so neighbours in x that
+// share an aligned pair of entries (half of them) go out as one: 16,384
+// samples 24.0 -> 19.5 us.
+__global__ void __launch_bounds__(128) encode_backward_kernel(GridParams G, const LuxCacheSample *__restrict__ samples,
+                                                              uint32_t n, const float2 *__restrict__ dx,
+                                                              float2 *__restrict__ grad) {
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, i = t / kLevelsMax, level = t % kLevelsMax;
+    if (i >= n || level >= G.levels) return;
+    const float2 g = dx[t];
+    if (g.x == 0.0f && g.y == 0.0f) return;
     float u[3];
-    unit_position(G, s, u);
-    for (uint32_t level = 0; level < G.levels; ++level) {
-        float g0 = dx[(size_t)i * 2 * kLevelsMax + 2 * level], g1 = dx[(size_t)i * 2 * kLevelsMax + 2 * level + 1];
-        if (g0 == 0.0f && g1 == 0.0f) continue;
-        Corner c;
-        level_corners(G, level, u, c);
+    unit_position(G, samples[i], u);
+    Corner c;
+    level_corners(G, level, u, c);
+    float2 *row = grad + (size_t)level * G.table;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) atomicAdd(&grad[c.index[k]], make_float2(c.weight[k] * g0, c.weight[k] * g1));
+    for (int k = 0; k < 8; k += 2) {
+        const uint32_t a = c.index[k], b = c.index[k + 1];
+        const float2 ga = make_float2(c.weight[k] * g.x, c.weight[k] * g.y);
+        const float2 gb = make_float2(c.weight[k + 1] * g.x, c.weight[k + 1] * g.y);
+        if ((a ^ b) == 1u) {
+            atomicAdd(reinterpret_cast<float4 *>(row) + (a >> 1), a & 1u ? make_float4(gb.x, gb.y, ga.x, ga.y)
+                                                                         : make_float4(ga.x, ga.y, gb.x, gb.y));
+        } else {
+            atomicAdd(&row[a], ga);
+            atomicAdd(&row[b], gb);
+        }
     }
 }
 
@@ -335,11 +363,31 @@ struct SmemForward {
     static constexpr uint32_t kBytes = kSlot + 8;
 };
 
+// Rows first .. first + 127 of x (zeros past n), to a packed tile.  A warp
+// reads whole rows, four per load, so a load touches 4 lines, not 32.
+__device__ __forceinline__ void load_rows(uint4 q[8], const uint4 *__restrict__ x, uint32_t first, uint32_t n) {
+    const uint32_t kg = threadIdx.x & 7u, r0 = (threadIdx.x & ~31u) + ((threadIdx.x >> 3) & 3u);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const uint32_t r = first + r0 + 4u * j;
+        q[j] = r < n ? x[(size_t)r * 8 + kg] : make_uint4(0, 0, 0, 0);
+    }
+}
+__device__ __forceinline__ void store_rows(bf16 *tile, const uint4 q[8]) {
+    const uint32_t kg = threadIdx.x & 7u, r0 = (threadIdx.x & ~31u) + ((threadIdx.x >> 3) & 3u);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) *reinterpret_cast<uint4 *>(tile + packed(r0 + 4u * j, kg * 8u, kTile)) = q[j];
+}
+
+// A tile is a chain of five rounds, so an SM holds as many CTAs as its shared
+// memory does, and reads the next tile meanwhile: 500,009 rows 67 -> 48 us
+// (2 CTAs per SM 66, 3 57; 8 tiles per SM over shared weights 57).
+constexpr uint32_t kForwardBlocks = 4;
 // Inference: out[row] = MLP(x[row]) (rgb; w = 1).  clamp: rgb >= 0.
-__global__ void __launch_bounds__(kTile) mlp_forward_kernel(const uint4 *__restrict__ x, uint32_t n,
-                                                             const uint32_t *__restrict__ n_dev,
-                                                             const uint4 *__restrict__ weights, float4 *__restrict__ out,
-                                                             int clamp, uint32_t *__restrict__ error) {
+__global__ void __launch_bounds__(kTile, kForwardBlocks)
+    mlp_forward_kernel(const uint4 *__restrict__ x, uint32_t n, const uint32_t *__restrict__ n_dev,
+                       const uint4 *__restrict__ weights, float4 *__restrict__ out, int clamp,
+                       uint32_t *__restrict__ error) {
     if (n_dev) n = min(n, *n_dev);
     extern __shared__ __align__(1024) unsigned char smem[];
     bf16 *W = reinterpret_cast<bf16 *>(smem + SmemForward::kW);
@@ -349,29 +397,36 @@ __global__ void __launch_bounds__(kTile) mlp_forward_kernel(const uint4 *__restr
     const uint32_t tid = threadIdx.x, warp = tid >> 5;
     if (warp == 0) tmem_alloc(slot);
     if (tid == 0) mbar_init(bar);
-    for (uint32_t i = tid; i < kWTotal / 8; i += kTile) reinterpret_cast<uint4 *>(W)[i] = weights[i];
-    sync_for_mma();
+    static_assert(kWTotal / 8 % kTile == 0 && kPackedElems / 8 % kTile == 0, "whole rounds of weight loads");
+#pragma unroll
+    for (uint32_t i = 0; i < kWTotal / 8 / kTile; ++i)
+        reinterpret_cast<uint4 *>(W)[i * kTile + tid] = weights[i * kTile + tid];
+    sync_for_mma(true);
     const uint32_t tmem = *slot;
     const uint32_t lane_addr = tmem + ((warp * 32u) << 16);
     const uint32_t bar_addr = smem_u32(bar), a_addr = smem_u32(A), w_addr = smem_u32(W);
     uint32_t phase = 0;
-    bool ok = true;
-    for (uint32_t tile = blockIdx.x; ok && tile * kTile < n; tile += gridDim.x) {
-        uint32_t row = tile * kTile + tid;
-#pragma unroll
-        for (int kg = 0; kg < 8; ++kg) {
-            uint4 q = row < n ? x[(size_t)row * 8 + kg] : make_uint4(0, 0, 0, 0);
-            *reinterpret_cast<uint4 *>(A + packed(tid, (uint32_t)kg * 8u, kTile)) = q;
-        }
-        for (int l = 0; l <= kHiddenLayers && ok; ++l) {
-            sync_for_mma();
+    uint4 q[8];  // the next tile's rows, read while this one is worked on
+    load_rows(q, x, blockIdx.x * kTile, n);
+    bool ok = true, stop = false;  // ok: this thread's last wait ended; stop: CTA-uniform
+    for (uint32_t tile = blockIdx.x; !stop && tile * kTile < n; tile += gridDim.x) {
+        const uint32_t row = tile * kTile + tid;
+        store_rows(A, q);
+        const unsigned long long next = ((unsigned long long)tile + gridDim.x) * kTile;
+        if (next < n) load_rows(q, x, (uint32_t)next, n);
+        for (int l = 0; l <= kHiddenLayers; ++l) {
+            ok = sync_for_mma(ok);
+            if (!ok) {
+                stop = true;
+                break;
+            }
             const uint32_t N = l < kHiddenLayers ? kHidden : kOut;
             if (tid == 0) {
                 issue_layer(tmem, a_addr, w_addr + fwd_offset(l) * 2u, N, kIn);
                 mma_commit(bar_addr);
             }
-            ok = wait_round(bar_addr, phase);
-            if (!ok) break;
+            ok = mbar_wait(bar_addr, phase);
+            phase ^= 1u;
             tc_fence_after();
             if (l < kHiddenLayers) {
                 float v[64];
@@ -387,7 +442,7 @@ __global__ void __launch_bounds__(kTile) mlp_forward_kernel(const uint4 *__restr
                 float v[16];
                 tmem_load16(lane_addr, v);
                 tmem_wait_load();
-                if (row < n) {
+                if (ok && row < n) {
                     float r = v[0], g = v[1], b = v[2];
                     if (clamp) {
                         r = fmaxf(r, 0.0f);
@@ -399,7 +454,7 @@ __global__ void __launch_bounds__(kTile) mlp_forward_kernel(const uint4 *__restr
             }
         }
     }
-    if (!ok && tid == 0) atomicOr(error, 1u);
+    if (!ok) atomicOr(error, 1u);
     if (!ok) mbar_wait(bar_addr, phase ^ 1u);  // let an in-flight chain finish before freeing TMEM
     tc_fence_before();
     __syncthreads();
@@ -479,8 +534,10 @@ __global__ void __launch_bounds__(kTile) mlp_train_kernel(const uint4 *__restric
     const uint32_t tid = threadIdx.x, warp = tid >> 5;
     if (warp == 0) tmem_alloc(slot, kTrainTmemCols);
     if (tid == 0) mbar_init(bar);
-    for (uint32_t i = tid; i < kPackedElems / 8; i += kTile) reinterpret_cast<uint4 *>(Wf)[i] = weights[i];
-    sync_for_mma();
+#pragma unroll 17
+    for (uint32_t i = 0; i < kPackedElems / 8 / kTile; ++i)
+        reinterpret_cast<uint4 *>(Wf)[i * kTile + tid] = weights[i * kTile + tid];
+    sync_for_mma(true);
     const uint32_t tmem = *slot;
     const uint32_t lane_addr = tmem + ((warp * 32u) << 16);
     const uint32_t bar_addr = smem_u32(bar);
@@ -491,22 +548,23 @@ __global__ void __launch_bounds__(kTile) mlp_train_kernel(const uint4 *__restric
     float loss_sum = 0.0f;
     for (uint32_t tile = blockIdx.x; ok && tile * kTile < n; tile += gridDim.x) {
         const uint32_t row = tile * kTile + tid;
-#pragma unroll
-        for (int kg = 0; kg < 8; ++kg) {
-            uint4 q = row < n ? x[(size_t)row * 8 + kg] : make_uint4(0, 0, 0, 0);
-            *reinterpret_cast<uint4 *>(H + packed(tid, (uint32_t)kg * 8u, kTile)) = q;
-        }
+        uint4 q[8];
+        load_rows(q, x, tile * kTile, n);
+        store_rows(H, q);
+        const float w = row < n ? samples[row].weight : 0.0f;
+        const float4 t = row < n ? target[row] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         // Forward: h_{l+1} = relu(h_l W_l^T), y = h_4 W_4^T.
         float y[16];
-        for (int l = 0; l <= kHiddenLayers && ok; ++l) {
-            sync_for_mma();
+        for (int l = 0; l <= kHiddenLayers; ++l) {
+            ok = sync_for_mma(ok);
+            if (!ok) break;
             const uint32_t N = l < kHiddenLayers ? kHidden : kOut;
             if (tid == 0) {
                 issue_layer(tmem, h_addr + (uint32_t)l * h_elems * 2u, w_addr + fwd_offset(l) * 2u, N, kIn);
                 mma_commit(bar_addr);
             }
-            ok = wait_round(bar_addr, phase);
-            if (!ok) break;
+            ok = mbar_wait(bar_addr, phase);  // the CTA agrees at the next barrier
+            phase ^= 1u;
             tc_fence_after();
             if (l < kHiddenLayers) {
                 float v[64];
@@ -523,14 +581,11 @@ __global__ void __launch_bounds__(kTile) mlp_train_kernel(const uint4 *__restric
                 tmem_wait_load();
             }
         }
-        if (!ok) break;
         // Relative L2 loss and its gradient (weighted; rows past n weigh 0).
         float gout[16];
 #pragma unroll
         for (int c = 0; c < 16; ++c) gout[c] = 0.0f;
         if (row < n) {
-            float w = samples[row].weight;
-            float4 t = target[row];
             float tt[3] = {t.x, t.y, t.z};
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
@@ -551,8 +606,9 @@ __global__ void __launch_bounds__(kTile) mlp_train_kernel(const uint4 *__restric
         }
         // Backward, layer 4 down to 0: dh_l = g_l W_l (from the packed W_l^T)
         // and dW_l^T += h_l^T g_l, both on the tensor cores in one round.
-        for (int l = kHiddenLayers; l >= 0 && ok; --l) {
-            sync_for_mma();
+        for (int l = kHiddenLayers; l >= 0; --l) {
+            ok = sync_for_mma(ok);
+            if (!ok) break;
             const bool out_layer = l == kHiddenLayers;
             if (tid == 0) {
                 const uint32_t grad_tile = out_layer ? d_addr : g_addr;
@@ -563,8 +619,8 @@ __global__ void __launch_bounds__(kTile) mlp_train_kernel(const uint4 *__restric
                 mma_commit(bar_addr);
             }
             const bf16 *h = H + (uint32_t)l * h_elems;
-            ok = wait_round(bar_addr, phase);  // both chains done: G may be overwritten
-            if (!ok) break;
+            ok = mbar_wait(bar_addr, phase);  // both chains done: G may be overwritten
+            phase ^= 1u;
             tc_fence_after();
             float v[64];
             tmem_load16(lane_addr + 0, v);
@@ -573,14 +629,27 @@ __global__ void __launch_bounds__(kTile) mlp_train_kernel(const uint4 *__restric
             tmem_load16(lane_addr + 48, v + 48);
             tmem_wait_load();
             if (l > 0) {
+                // relu's mask from the stored activations, eight per load
 #pragma unroll
-                for (int k = 0; k < 64; ++k) v[k] = bf16_at(h, tid, (uint32_t)k) > 0.0f ? v[k] : 0.0f;
+                for (int kg = 0; kg < 8; ++kg) {
+                    const uint4 q = *reinterpret_cast<const uint4 *>(h + packed(tid, (uint32_t)kg * 8u, kTile));
+                    const uint32_t two[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const float2 a = bf16x2_floats(two[k]);
+                        v[kg * 8 + 2 * k] = a.x > 0.0f ? v[kg * 8 + 2 * k] : 0.0f;
+                        v[kg * 8 + 2 * k + 1] = a.y > 0.0f ? v[kg * 8 + 2 * k + 1] : 0.0f;
+                    }
+                }
                 store_row64(G, tid, v);
             } else if (row < n) {
+                float4 *to = reinterpret_cast<float4 *>(dx + (size_t)row * 2 * kLevelsMax);
 #pragma unroll
-                for (int k = 0; k < 2 * kLevelsMax; ++k) dx[(size_t)row * 2 * kLevelsMax + k] = v[k];
+                for (int k = 0; k < 2 * kLevelsMax / 4; ++k)
+                    to[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
             }
         }
+        ok = sync_for_mma(ok);
         grads = grads || ok;
     }
     // This CTA's weight gradients, once, from TMEM.
@@ -611,22 +680,34 @@ struct AdamParams {
     float lr, beta1, beta2, eps, correction1, correction2;
 };
 
-// Adam on four consecutive parameters per thread (the hash table: n is a
-// multiple of 4), with the BF16 copy written as one 8-byte store.  Sparse
-// ("lazy") Adam: a parameter this step's samples did not reach (zero
-// gradient) keeps its value and moments, so a step reads only the gradients
-// of the untouched entries -- a batch reaches a quarter of a fine level's
-// entries at most.  A parameter's first update is the dense step's.
+// A table entry's Adam state, 32 bytes (one sector): the two features' values,
+// first and second moments.  The entries one step reaches are scattered (its
+// samples reach a quarter of a fine level's entries at most), so with three
+// arrays nearly every sector of all three moved for a quarter of its bytes:
+// 16,384 samples into 16 x 524,288 entries 78 -> 54 us per step, of which the
+// 67 MB of gradients are 10 at the copy rate.
+struct __align__(32) TableEntry {
+    float2 p, m, v, unused;
+};
+constexpr int kAdamThreads = 256, kAdamScan = 4;  // float4 gradients per lane and round
+
+// Sparse ("lazy") Adam on the hash table: an entry this step's samples did not
+// reach (zero gradient) keeps its values and moments, so a step reads only the
+// gradients of the untouched entries.  A parameter's first update is the dense
+// step's.  A warp reads 256 entries' gradients, clears those it found, and
+// lists the reached entries in shared memory; then a lane updates one listed
+// entry, so that no lane waits through the divisions of others'.
 //
 // The same launch also takes the Adam step of the MLP weights (thread e of
 // the grid: weight e, dense Adam, skipping weights whose gradient and first
 // moment are both zero: never touched) and writes each weight's BF16 copy into the forward (W) and
 // backward (W^T) tile layouts, as pack_weights_kernel does: one launch per
 // training step instead of three.
-__global__ void adam4_kernel(AdamParams P, float4 *__restrict__ param, float4 *__restrict__ grad,
-                             float4 *__restrict__ m, float4 *__restrict__ v, size_t n4, uint2 *__restrict__ out,
-                             float *__restrict__ w, float *__restrict__ wg, float *__restrict__ wm,
-                             float *__restrict__ wv, bf16 *__restrict__ w_packed) {
+__global__ void __launch_bounds__(kAdamThreads, 5) adam_kernel(AdamParams P, TableEntry *__restrict__ rows,
+                                                            float4 *__restrict__ grad, size_t entries,
+                                                            uint32_t *__restrict__ out, float *__restrict__ w,
+                                                            float *__restrict__ wg, float *__restrict__ wm,
+                                                            float *__restrict__ wv, bf16 *__restrict__ w_packed) {
     const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
     if (w && e < (uint32_t)kWTotal) {
         float p = w[e];
@@ -649,25 +730,74 @@ __global__ void adam4_kernel(AdamParams P, float4 *__restrict__ param, float4 *_
         w_packed[fwd_offset((int)l) + packed(o, i, N)] = b;
         w_packed[bwd_offset((int)l) + packed(i, o, kIn)] = b;
     }
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n4; i += (size_t)gridDim.x * blockDim.x) {
-        float4 g = grad[i];
-        if (g.x == 0.0f && g.y == 0.0f && g.z == 0.0f && g.w == 0.0f) continue;  // not reached this step
-        grad[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        float4 mi = m[i], vi = v[i], p = param[i];
-        float gs[4] = {g.x, g.y, g.z, g.w}, ms[4] = {mi.x, mi.y, mi.z, mi.w}, vs[4] = {vi.x, vi.y, vi.z, vi.w};
-        float ps[4] = {p.x, p.y, p.z, p.w};
+    constexpr uint32_t kRound = 32u * kAdamScan * 2u;  // entries per warp and round (tables hold whole rounds)
+    __shared__ float2 listed_grad[kAdamThreads / 32][kRound];
+    __shared__ uint16_t listed[kAdamThreads / 32][kRound];
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
+    for (size_t first = (blockIdx.x * (size_t)(kAdamThreads / 32) + warp) * kRound; first < entries;
+         first += (size_t)gridDim.x * (kAdamThreads / 32) * kRound) {
+        float4 *at = grad + first / 2 + lane;
+        float4 g[kAdamScan];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            if (gs[k] == 0.0f) continue;
-            ms[k] = P.beta1 * ms[k] + (1.0f - P.beta1) * gs[k];
-            vs[k] = P.beta2 * vs[k] + (1.0f - P.beta2) * gs[k] * gs[k];
-            ps[k] = ps[k] - P.lr * (ms[k] / P.correction1) / (sqrtf(vs[k] / P.correction2) + P.eps);
+        for (int k = 0; k < kAdamScan; ++k) g[k] = at[k * 32];
+        uint32_t count = 0;
+#pragma unroll
+        for (int k = 0; k < kAdamScan; ++k) {
+            const bool lo = !(g[k].x == 0.0f && g[k].y == 0.0f), hi = !(g[k].z == 0.0f && g[k].w == 0.0f);
+            const unsigned los = __ballot_sync(0xffffffffu, lo), his = __ballot_sync(0xffffffffu, hi);
+            if (lo || hi) at[k * 32] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            const uint32_t entry = (uint32_t)(k * 32 + lane) * 2u;
+            if (lo) {
+                const uint32_t to = count + (uint32_t)__popc(los & below);
+                listed[warp][to] = (uint16_t)entry;
+                listed_grad[warp][to] = make_float2(g[k].x, g[k].y);
+            }
+            count += (uint32_t)__popc(los);
+            if (hi) {
+                const uint32_t to = count + (uint32_t)__popc(his & below);
+                listed[warp][to] = (uint16_t)(entry + 1u);
+                listed_grad[warp][to] = make_float2(g[k].z, g[k].w);
+            }
+            count += (uint32_t)__popc(his);
         }
-        m[i] = make_float4(ms[0], ms[1], ms[2], ms[3]);
-        v[i] = make_float4(vs[0], vs[1], vs[2], vs[3]);
-        param[i] = make_float4(ps[0], ps[1], ps[2], ps[3]);
-        out[i] = make_uint2(pack_bf16x2(ps[0], ps[1]), pack_bf16x2(ps[2], ps[3]));
+        __syncwarp();
+        float4 next_pm = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        float2 next_v = make_float2(0.0f, 0.0f);
+        if (lane < count) {
+            const TableEntry *row = rows + first + listed[warp][lane];
+            next_pm = reinterpret_cast<const float4 *>(row)[0];
+            next_v = row->v;
+        }
+        for (uint32_t i = lane; i < count; i += 32u) {
+            const size_t e = first + listed[warp][i];
+            const float2 gr = listed_grad[warp][i];
+            const float4 pm = next_pm;
+            const float2 v = next_v;
+            if (i + 32u < count) {
+                const TableEntry *row = rows + first + listed[warp][i + 32u];
+                next_pm = reinterpret_cast<const float4 *>(row)[0];
+                next_v = row->v;
+            }
+            const float gs[2] = {gr.x, gr.y};
+            float ps[2] = {pm.x, pm.y}, ms[2] = {pm.z, pm.w}, vs[2] = {v.x, v.y};
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                if (gs[k] == 0.0f) continue;
+                ms[k] = P.beta1 * ms[k] + (1.0f - P.beta1) * gs[k];
+                vs[k] = P.beta2 * vs[k] + (1.0f - P.beta2) * gs[k] * gs[k];
+                ps[k] = ps[k] - P.lr * (ms[k] / P.correction1) / (sqrtf(vs[k] / P.correction2) + P.eps);
+            }
+            reinterpret_cast<float4 *>(rows + e)[0] = make_float4(ps[0], ps[1], ms[0], ms[1]);
+            reinterpret_cast<float4 *>(rows + e)[1] = make_float4(vs[0], vs[1], 0.0f, 0.0f);
+            out[e] = pack_bf16x2(ps[0], ps[1]);
+        }
+        __syncwarp();
     }
+}
+
+__global__ void read_rows_kernel(const TableEntry *__restrict__ rows, size_t n, float2 *__restrict__ out) {
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+        out[i] = rows[i].p;
 }
 
 // Packs the FP32 master weights into the forward (W) and backward (W^T)
@@ -684,12 +814,14 @@ __global__ void pack_weights_kernel(const float *__restrict__ w, bf16 *__restric
     out[bwd_offset((int)l) + packed(i, o, kIn)] = b;
 }
 
-__global__ void init_uniform_kernel(float *__restrict__ p, size_t n, float scale, uint32_t seed, bf16 *__restrict__ out) {
+// Value i goes to p[(i / 2) pitch + i % 2].
+__global__ void init_uniform_kernel(float *__restrict__ p, size_t n, uint32_t pitch, float scale, uint32_t seed,
+                                    bf16 *__restrict__ out) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         uint32_t h = lux::transport_hash((uint32_t)i * 0x9E3779B9u ^ lux::transport_hash(seed + (uint32_t)(i >> 32)));
         float u = (float)(h >> 8) / 16777216.0f;
         float val = (2.0f * u - 1.0f) * scale;
-        p[i] = val;
+        p[(i >> 1) * pitch + (i & 1u)] = val;
         if (out) out[i] = __float2bfloat16_rn(val);
     }
 }
@@ -701,7 +833,8 @@ struct LuxCache {
     LuxCacheDesc desc{};
     GridParams grid{};
     size_t table_params = 0;  // levels * table * 2
-    float *table_master = nullptr, *table_grad = nullptr, *table_m = nullptr, *table_v = nullptr;
+    TableEntry *table_rows = nullptr;  // values and moments, levels x table
+    float *table_grad = nullptr;
     bf16 *table = nullptr;
     float *w_master = nullptr, *w_grad = nullptr, *w_m = nullptr, *w_v = nullptr;
     bf16 *w_packed = nullptr;
@@ -716,8 +849,8 @@ struct LuxCache {
 namespace {
 
 void cache_free(LuxCache *c) {
-    void *ptrs[] = {c->table_master, c->table_grad, c->table_m, c->table_v, c->table, c->w_master, c->w_grad,
-                    c->w_m,          c->w_v,        c->w_packed, c->x,      c->dx,    c->loss,     c->error};
+    void *ptrs[] = {c->table_rows, c->table_grad, c->table, c->w_master, c->w_grad, c->w_m, c->w_v, c->w_packed,
+                    c->x,          c->dx,         c->loss,  c->error};
     for (void *p : ptrs)
         if (p) cudaFree(p);
 }
@@ -790,10 +923,8 @@ extern "C" lux_status lux_cache_create(LuxContext *ctx, const LuxCacheDesc *desc
     c->table_params = (size_t)d.levels * G.table * 2;
     cudaSetDevice(ctx->device);
     size_t tp = c->table_params;
-    bool ok = cudaMalloc((void **)&c->table_master, tp * 4) == cudaSuccess &&
+    bool ok = cudaMalloc((void **)&c->table_rows, tp / 2 * sizeof(TableEntry)) == cudaSuccess &&
               cudaMalloc((void **)&c->table_grad, tp * 4) == cudaSuccess &&
-              cudaMalloc((void **)&c->table_m, tp * 4) == cudaSuccess &&
-              cudaMalloc((void **)&c->table_v, tp * 4) == cudaSuccess &&
               cudaMalloc((void **)&c->table, tp * 2) == cudaSuccess &&
               cudaMalloc((void **)&c->w_master, kWTotal * 4) == cudaSuccess &&
               cudaMalloc((void **)&c->w_grad, kWTotal * 4) == cudaSuccess &&
@@ -810,19 +941,19 @@ extern "C" lux_status lux_cache_create(LuxContext *ctx, const LuxCacheDesc *desc
     }
     cudaStream_t st = ctx->stream;
     cudaMemsetAsync(c->table_grad, 0, tp * 4, st);
-    cudaMemsetAsync(c->table_m, 0, tp * 4, st);
-    cudaMemsetAsync(c->table_v, 0, tp * 4, st);
+    cudaMemsetAsync(c->table_rows, 0, tp / 2 * sizeof(TableEntry), st);
     cudaMemsetAsync(c->w_grad, 0, kWTotal * 4, st);
     cudaMemsetAsync(c->w_m, 0, kWTotal * 4, st);
     cudaMemsetAsync(c->w_v, 0, kWTotal * 4, st);
     cudaMemsetAsync(c->w_packed, 0, kPackedElems * 2, st);
     cudaMemsetAsync(c->error, 0, 16, st);
     const int grid = ctx->sm_count * 8;
-    init_uniform_kernel<<<grid, 256, 0, st>>>(c->table_master, tp, 1e-4f, d.seed, c->table);
+    init_uniform_kernel<<<grid, 256, 0, st>>>((float *)c->table_rows, tp, sizeof(TableEntry) / 4, 1e-4f, d.seed,
+                                              c->table);
     // Hidden layers: uniform +-sqrt(6 / fan_in) (ReLU); output layer a tenth.
-    init_uniform_kernel<<<grid, 256, 0, st>>>(c->w_master, (size_t)kHiddenLayers * kWHidden,
+    init_uniform_kernel<<<grid, 256, 0, st>>>(c->w_master, (size_t)kHiddenLayers * kWHidden, 2,
                                               std::sqrt(6.0f / kIn), d.seed ^ 0x5bd1e995u, nullptr);
-    init_uniform_kernel<<<grid, 256, 0, st>>>(c->w_master + kHiddenLayers * kWHidden, (size_t)kOut * kIn,
+    init_uniform_kernel<<<grid, 256, 0, st>>>(c->w_master + kHiddenLayers * kWHidden, (size_t)kOut * kIn, 2,
                                               0.1f * std::sqrt(6.0f / kIn), d.seed ^ 0x27d4eb2fu, nullptr);
     pack_weights_kernel<<<(kWTotal + 255) / 256, 256, 0, st>>>(c->w_master, c->w_packed);
     cudaFuncSetAttribute(mlp_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kForwardSmem);
@@ -855,11 +986,16 @@ extern "C" lux_status lux_cache_set_bounds(LuxCache *c, const float lo[3], const
     return LUX_OK;
 }
 
+// Blocks of 128 threads for `lanes` lanes per sample.
+static unsigned encode_blocks(uint32_t samples, uint32_t lanes = 4u) {
+    return (unsigned)(((uint64_t)samples * lanes + 127) / 128);
+}
+
 static lux_status cache_forward(LuxCache *c, const uint4 *x, uint32_t count, const uint32_t *count_dev, float *out,
                                 int clamp) {
     LuxContext *ctx = c->ctx;
     uint32_t tiles = (count + kTile - 1) / kTile;
-    uint32_t grid = std::min<uint32_t>(tiles, (uint32_t)ctx->sm_count * 2u);
+    uint32_t grid = std::min<uint32_t>(tiles, (uint32_t)ctx->sm_count * kForwardBlocks);
     mlp_forward_kernel<<<grid, kTile, kForwardSmem, ctx->stream>>>(x, count, count_dev, (const uint4 *)c->w_packed,
                                                                    (float4 *)out, clamp, c->error);
     return lux_cuda_check(ctx, (int)cudaGetLastError(), "cache: forward launch");
@@ -869,8 +1005,8 @@ extern "C" lux_status lux_cache_encode(LuxCache *c, const LuxCacheSample *sample
     if (!c || (count && (!samples || !out))) return LUX_ERR_INVALID_ARGUMENT;
     if (count == 0) return LUX_OK;
     cudaSetDevice(c->ctx->device);
-    encode_kernel<<<(count + 127) / 128, 128, 0, c->ctx->stream>>>(
-        c->grid, samples, count, nullptr, (const __nv_bfloat162 *)c->table, (uint4 *)out);
+    encode_kernel<<<encode_blocks(count), 128, 0, c->ctx->stream>>>(
+        c->grid, samples, count, nullptr, (const uint32_t *)c->table, (uint4 *)out);
     return lux_cuda_check(c->ctx, (int)cudaGetLastError(), "cache: encode launch");
 }
 
@@ -887,8 +1023,8 @@ extern "C" lux_status lux_cache_query(LuxCache *c, const LuxCacheSample *queries
     cudaSetDevice(c->ctx->device);
     lux_status rc = ensure_rows(c, count);
     if (rc != LUX_OK) return rc;
-    encode_kernel<<<(count + 127) / 128, 128, 0, c->ctx->stream>>>(c->grid, queries, count, nullptr,
-                                                                   (const __nv_bfloat162 *)c->table, c->x);
+    encode_kernel<<<encode_blocks(count), 128, 0, c->ctx->stream>>>(c->grid, queries, count, nullptr,
+                                                                   (const uint32_t *)c->table, c->x);
     return cache_forward(c, c->x, count, nullptr, out, 1);
 }
 
@@ -898,8 +1034,8 @@ lux_status lux_cache_query_device_count(LuxCache *c, const LuxCacheSample *queri
     if (max_count == 0) return LUX_OK;
     lux_status rc = ensure_rows(c, max_count);
     if (rc != LUX_OK) return rc;
-    encode_kernel<<<(max_count + 127) / 128, 128, 0, c->ctx->stream>>>(c->grid, queries, max_count, count,
-                                                                       (const __nv_bfloat162 *)c->table, c->x);
+    encode_kernel<<<encode_blocks(max_count), 128, 0, c->ctx->stream>>>(c->grid, queries, max_count, count,
+                                                                       (const uint32_t *)c->table, c->x);
     return cache_forward(c, c->x, max_count, count, out, 1);
 }
 
@@ -912,18 +1048,17 @@ extern "C" lux_status lux_cache_train(LuxCache *c, const LuxCacheSample *samples
     lux_status rc = ensure_rows(c, batch);
     if (rc != LUX_OK) return rc;
     cudaStream_t st = ctx->stream;
-    const int grid = ctx->sm_count * 8;
     for (uint32_t s0 = 0; s0 < count; s0 += batch) {
         uint32_t nb = std::min(batch, count - s0);
         const LuxCacheSample *sb = samples + s0;
-        encode_kernel<<<(nb + 127) / 128, 128, 0, st>>>(c->grid, sb, nb, nullptr, (const __nv_bfloat162 *)c->table,
+        encode_kernel<<<encode_blocks(nb), 128, 0, st>>>(c->grid, sb, nb, nullptr, (const uint32_t *)c->table,
                                                         c->x);
         cudaMemsetAsync(c->loss, 0, 4, st);
         uint32_t tiles = (nb + kTile - 1) / kTile;
         mlp_train_kernel<<<std::min<uint32_t>(tiles, (uint32_t)ctx->sm_count), kTile, kTrainSmem, st>>>(
             c->x, (const float4 *)targets + s0, sb, nb, 1.0f / (3.0f * (float)nb), (const uint4 *)c->w_packed,
             c->w_grad, c->dx, c->loss, c->error);
-        encode_backward_kernel<<<(nb + 127) / 128, 128, 0, st>>>(c->grid, sb, nb, c->dx, (float2 *)c->table_grad);
+        encode_backward_kernel<<<encode_blocks(nb, kLevelsMax), 128, 0, st>>>(c->grid, sb, nb, (const float2 *)c->dx, (float2 *)c->table_grad);
         ++c->steps;
         AdamParams P;
         P.lr = c->desc.learning_rate;
@@ -932,9 +1067,12 @@ extern "C" lux_status lux_cache_train(LuxCache *c, const LuxCacheSample *samples
         P.eps = 1e-10f;
         P.correction1 = 1.0f - (float)std::pow(0.9, (double)c->steps);
         P.correction2 = 1.0f - (float)std::pow(0.99, (double)c->steps);
-        adam4_kernel<<<std::max(grid, (kWTotal + 255) / 256), 256, 0, st>>>(
-            P, (float4 *)c->table_master, (float4 *)c->table_grad, (float4 *)c->table_m, (float4 *)c->table_v,
-            c->table_params / 4, (uint2 *)c->table, c->w_master, c->w_grad, c->w_m, c->w_v, c->w_packed);
+        // A round per block, so that the blocks balance; at least the weights' threads.
+        const size_t rounds = std::max<size_t>(c->table_params / 2 / (kAdamThreads * kAdamScan * 2),
+                                               (kWTotal + kAdamThreads - 1) / kAdamThreads);
+        adam_kernel<<<(unsigned)std::min<size_t>(rounds, 1u << 20), kAdamThreads, 0, st>>>(
+            P, c->table_rows, (float4 *)c->table_grad, c->table_params / 2, (uint32_t *)c->table, c->w_master, c->w_grad,
+            c->w_m, c->w_v, c->w_packed);
         c->samples += nb;
         rc = lux_cuda_check(ctx, (int)cudaGetLastError(), "cache: train launch");
         if (rc != LUX_OK) return rc;
@@ -973,15 +1111,15 @@ extern "C" lux_status lux_cache_gradients(LuxCache *c, const LuxCacheSample *sam
     lux_status rc = ensure_rows(c, c->desc.batch);
     if (rc != LUX_OK) return rc;
     cudaStream_t st = ctx->stream;
-    encode_kernel<<<(count + 127) / 128, 128, 0, st>>>(c->grid, samples, count, nullptr,
-                                                       (const __nv_bfloat162 *)c->table, c->x);
+    encode_kernel<<<encode_blocks(count), 128, 0, st>>>(c->grid, samples, count, nullptr,
+                                                       (const uint32_t *)c->table, c->x);
     cudaMemsetAsync(c->loss, 0, 4, st);
     uint32_t tiles = (count + kTile - 1) / kTile;
     mlp_train_kernel<<<std::min<uint32_t>(tiles, (uint32_t)ctx->sm_count), kTile, kTrainSmem, st>>>(
         c->x, (const float4 *)targets, samples, count, 1.0f / (3.0f * (float)count), (const uint4 *)c->w_packed,
         c->w_grad, c->dx, c->loss, c->error);
-    encode_backward_kernel<<<(count + 127) / 128, 128, 0, st>>>(c->grid, samples, count, c->dx,
-                                                                (float2 *)c->table_grad);
+    encode_backward_kernel<<<encode_blocks(count, kLevelsMax), 128, 0, st>>>(c->grid, samples, count,
+                                                                                 (const float2 *)c->dx, (float2 *)c->table_grad);
     rc = lux_cuda_check(ctx, (int)cudaStreamSynchronize(st), "cache: gradients");
     if (rc != LUX_OK) return rc;
     bool ok = cudaMemcpy(grad_weights, c->w_grad, kWTotal * 4, cudaMemcpyDeviceToHost) == cudaSuccess &&
@@ -998,8 +1136,22 @@ extern "C" lux_status lux_cache_read_table(LuxCache *c, float *out) {
     cudaSetDevice(c->ctx->device);
     lux_status rc = lux_cuda_check(c->ctx, (int)cudaStreamSynchronize(c->ctx->stream), "cache: table");
     if (rc != LUX_OK) return rc;
-    return lux_cuda_check(c->ctx, (int)cudaMemcpy(out, c->table_master, c->table_params * 4, cudaMemcpyDeviceToHost),
-                          "cache: table copy");
+    // Through a device buffer of one piece: the values lie 32 bytes apart.
+    const size_t n = c->table_params / 2, piece = std::min<size_t>(n, 1u << 20);
+    float2 *packed_rows = nullptr;
+    if (cudaMalloc((void **)&packed_rows, piece * sizeof(float2)) != cudaSuccess) {
+        cudaGetLastError();
+        return lux_fail(c->ctx, LUX_ERR_OUT_OF_MEMORY, "cache: table copy buffer allocation failed");
+    }
+    cudaError_t e = cudaSuccess;
+    for (size_t i = 0; i < n && e == cudaSuccess; i += piece) {
+        const size_t take = std::min(piece, n - i);
+        read_rows_kernel<<<c->ctx->sm_count * 4, 256, 0, c->ctx->stream>>>(c->table_rows + i, take, packed_rows);
+        e = cudaMemcpyAsync(out + 2 * i, packed_rows, take * sizeof(float2), cudaMemcpyDeviceToHost, c->ctx->stream);
+    }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c->ctx->stream);
+    cudaFree(packed_rows);
+    return lux_cuda_check(c->ctx, (int)e, "cache: table copy");
 }
 
 extern "C" lux_status lux_cache_read_weights(LuxCache *c, float *out) {
