@@ -56,7 +56,7 @@
 #endif
 // The batched trace kernels keep a job's scene pointers per warp as well.
 #ifndef LUX_BATCH_MIN_BLOCKS
-#define LUX_BATCH_MIN_BLOCKS 6
+#define LUX_BATCH_MIN_BLOCKS 7
 #endif
 #ifndef LUX_SMALL_DIRECTORY
 #define LUX_SMALL_DIRECTORY 32768u
@@ -2305,7 +2305,10 @@ __global__ void __launch_bounds__(128, LUX_BATCH_MIN_BLOCKS)
     closest_batch_phase<kFlat>(jobs, begin, n, total, *frame, counter, tile, &scratch[threadIdx.x >> 5]);
 }
 
-__global__ void __launch_bounds__(128, LUX_SHADE_MIN_BLOCKS) shade_batch_kernel(const BatchJob *__restrict__ jobs,
+// Four blocks per SM, not shade_kernel's six: the job's pointers are loaded, not
+// parameters, and at six 310 bytes of them spilled (448 us for twelve views of
+// 640x360; four 368, three 459).
+__global__ void __launch_bounds__(128, 4) shade_batch_kernel(const BatchJob *__restrict__ jobs,
                                                           const uint32_t *__restrict__ begin, uint32_t n,
                                                           uint32_t total, const uint32_t *__restrict__ frame) {
     __shared__ ShadeScratch scratch[4];
@@ -2459,6 +2462,41 @@ __device__ __forceinline__ const unsigned long long *batch_row(const unsigned lo
     return dom + (size_t)row * (n + 1);
 }
 
+// fn(job, j, first, last) for the items of a padded domain row in block-sized
+// spans of one job each.  The record passes do little per record, and their
+// job's fields are shared memory here: read from the job table for each record
+// behind a search and the error word, they were a chain of twenty loads.
+// Every thread of the block calls it, and fn is called by all of them.
+constexpr uint32_t kSpanMost = 4096;  // items per span, fewer when the row is short
+template <typename Fn>
+__device__ __forceinline__ void for_batch_spans(const BatchJob *__restrict__ jobs,
+                                                const unsigned long long *__restrict__ begin, uint32_t n, Fn &&fn) {
+    static_assert(sizeof(BatchJob) % 16 == 0, "copied in 16-byte words");
+    __shared__ uint4 copy[sizeof(BatchJob) / 16];
+    const BatchJob &J = *reinterpret_cast<const BatchJob *>(copy);
+    const unsigned long long total = begin[n], share = total / (gridDim.x * 4ull);
+    const uint32_t span = share >= kSpanMost ? kSpanMost
+                                             : (((uint32_t)share + blockDim.x) / blockDim.x) * blockDim.x;
+    uint32_t cur = lux::kEmpty;
+    for (unsigned long long x = blockIdx.x * (unsigned long long)span; x < total;
+         x += gridDim.x * (unsigned long long)span) {
+        const unsigned long long end = min(x + span, total);
+        for (unsigned long long at = x; at < end;) {
+            const uint32_t j = find_job64(begin, n, at);
+            const unsigned long long first = begin[j], stop = min(end, begin[j + 1u]);
+            if (j != cur) {
+                __syncthreads();  // the previous job is no longer read
+                for (uint32_t k = threadIdx.x; k < sizeof(BatchJob) / 16; k += blockDim.x)
+                    copy[k] = reinterpret_cast<const uint4 *>(jobs + j)[k];
+                __syncthreads();
+                cur = j;
+            }
+            fn(J, j, at - first, stop - first);
+            at = stop;
+        }
+    }
+}
+
 // The directory clear, and the retain age histograms of the jobs that
 // blend history.
 __global__ void batch_clear_kernel(const BatchJob *__restrict__ jobs, const unsigned long long *__restrict__ dom,
@@ -2586,9 +2624,11 @@ __global__ void __launch_bounds__(1024) batch_layout_kernel(const BatchJob *__re
 __global__ void batch_clear_entries_kernel(const BatchJob *__restrict__ jobs,
                                            const unsigned long long *__restrict__ dom, uint32_t n,
                                            const unsigned long long *__restrict__ count) {
-    for_batch_items(batch_row(dom, n, kRowEntries), n, [&](uint32_t j, unsigned long long i) {
-        if (i < count[j]) clear_entry(jobs[j].V, i);
-    });
+    for_batch_spans(jobs, batch_row(dom, n, kRowEntries), n,
+                    [&](const BatchJob &J, uint32_t j, unsigned long long first, unsigned long long last) {
+                        const unsigned long long stop = min(last, count[j]);
+                        for (unsigned long long i = first + threadIdx.x; i < stop; i += blockDim.x) clear_entry(J.V, i);
+                    });
 }
 
 // Before the merge, one launch for all levels and jobs: each cell's corners
@@ -2623,33 +2663,41 @@ __global__ void __launch_bounds__(256) batch_merge_own_kernel(const BatchJob *__
 
 // The listing own pass over all jobs (merge_own_list_kernel's list for each
 // job's view): a warp chunk belongs to one job; lanes with records of one
-// level that pass light on append them together.
-__global__ void __launch_bounds__(256) batch_merge_own_list_kernel(const BatchJob *__restrict__ jobs,
+// level that pass light on append them together.  Twelve views of 640x360: 842
+// -> 695 us; the same rate per record as merge_own_list_kernel's.
+__global__ void __launch_bounds__(256, 6) batch_merge_own_list_kernel(const BatchJob *__restrict__ jobs,
                                                                    const unsigned long long *__restrict__ dom,
                                                                    uint32_t n,
                                                                    const unsigned long long *__restrict__ count) {
     const uint32_t lane = threadIdx.x & 31u;
-    for_batch_items(batch_row(dom, n, kRowEntries), n, [&](uint32_t j, unsigned long long e) {
-        const BatchJob &J = jobs[j];
-        if (e >= count[j] || *J.V.error_flags) return;
-        uint32_t level = 0;
-        while (level + 1u < J.F.levels && e >= J.V.level_base[level + 1u]) ++level;
-        const unsigned long long base = J.V.level_base[level];
-        const uint32_t dirs = J.F.dirs[level];
-        const unsigned long long r = e - base;
-        uint32_t cell, d;
-        record_cell(r, dirs, cell, d);
-        MergeOwn own;
-        if (!merge_own(J.V, J.F, J.H, level, base, dirs, cell, d, own)) {
-            merge_finish(J.V, J.F, level, base, dirs, cell, d, own, false);
-            return;
+    for_batch_spans(jobs, batch_row(dom, n, kRowEntries), n,
+                    [&](const BatchJob &J, uint32_t j, unsigned long long first, unsigned long long last) {
+        const unsigned long long stop = min(last, count[j]);
+        if (*J.V.error_flags) return;
+        uint32_t level = 0, dirs = J.F.dirs[0];
+        unsigned long long base = 0, end = J.F.levels > 1u ? J.V.level_base[1] : ~0ull;
+        for (unsigned long long e = first + threadIdx.x; e < stop; e += blockDim.x) {
+            while (e >= end) {
+                dirs = J.F.dirs[++level];
+                base = end;
+                end = level + 1u < J.F.levels ? J.V.level_base[level + 1u] : ~0ull;
+            }
+            const unsigned long long r = e - base;
+            uint32_t cell, d;
+            record_cell(r, dirs, cell, d);
+            MergeOwn own;
+            const bool children = merge_own(J.V, J.F, J.H, level, base, dirs, cell, d, own);
+            if (!children) merge_finish(J.V, J.F, level, base, dirs, cell, d, own, false);
+            unsigned want = __ballot_sync(__activemask(), children);
+            if (children) {
+                want = __match_any_sync(want, level);
+                const uint32_t leader = (uint32_t)__ffs(want) - 1u;
+                uint32_t at = 0;
+                if (lane == leader) at = atomicAdd(&J.V.pass_count[level], (uint32_t)__popc(want));
+                at = __shfl_sync(want, at, leader);
+                J.V.pass_list[base + at + (uint32_t)__popc(want & ((1u << lane) - 1u))] = (uint32_t)r;
+            }
         }
-        const unsigned group = __match_any_sync(__activemask(), level);
-        const uint32_t leader = (uint32_t)__ffs(group) - 1u;
-        uint32_t at = 0;
-        if (lane == leader) at = atomicAdd(&J.V.pass_count[level], (uint32_t)__popc(group));
-        at = __shfl_sync(group, at, leader);
-        J.V.pass_list[base + at + (uint32_t)__popc(group & ((1u << lane) - 1u))] = (uint32_t)r;
     });
 }
 
