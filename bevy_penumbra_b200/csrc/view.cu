@@ -33,6 +33,7 @@
 #include "lux_internal.h"
 #include "lux_math.cuh"
 #include "shade.cuh"
+#include "launch.cuh"
 #include "traverse.cuh"
 
 // Resident 128-thread blocks per SM the trace kernels are compiled for: the
@@ -332,6 +333,7 @@ __device__ __forceinline__ void clear_item(const ViewDevice &V, const FrameParam
 }
 
 __global__ void clear_kernel(ViewDevice V, FrameParams F) {
+    lux::after_previous();
     size_t n = (size_t)F.levels * F.dir_capacity;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
         clear_item(V, F, i);
@@ -383,6 +385,7 @@ __device__ __forceinline__ void seed_insert_item(const ViewDevice &V, const Fram
 }
 
 __global__ void seed_insert_kernel(ViewDevice V, FrameParams F, const float4 *__restrict__ pos) {
+    lux::after_previous();
     size_t n = (size_t)F.receivers * F.levels;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
         seed_insert_item(V, F, pos, i);
@@ -410,6 +413,7 @@ __device__ __forceinline__ void seed_assign_item(const ViewDevice &V, const Fram
 }
 
 __global__ void seed_assign_kernel(ViewDevice V, FrameParams F) {
+    lux::after_previous();
     size_t n = (size_t)F.levels * F.dir_capacity;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
         seed_assign_item(V, F, i);
@@ -435,6 +439,7 @@ __device__ __forceinline__ unsigned long long sequence_key(int32_t x, int32_t y,
 
 // sorted: the receiver indices in sequence order (the sort's output half).
 __global__ void ordinal_kernel(ViewDevice V, const uint32_t *__restrict__ sorted, uint32_t receivers) {
+    lux::after_previous();
     for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < receivers; j += gridDim.x * blockDim.x)
         V.receiver_ordinal[sorted[j]] = j;
 }
@@ -449,6 +454,7 @@ __global__ void ordinal_kernel(ViewDevice V, const uint32_t *__restrict__ sorted
 // 256.
 constexpr uint32_t kRankedCells = 16384, kRankChunk = 256;
 __global__ void __launch_bounds__(128) cell_rank_kernel(ViewDevice V, FrameParams F) {
+    lux::after_previous();
     __shared__ __align__(16) unsigned long long key[kRankChunk];
     const uint32_t cells = min(V.cell_count[0], F.cell_capacity);
     const uint32_t c = blockIdx.x * 256u + threadIdx.x, first = blockIdx.y * kRankChunk;
@@ -506,6 +512,7 @@ __device__ __forceinline__ void seed_lookup_item(const ViewDevice &V, const Fram
 
 template <bool kRanked>
 __global__ void seed_lookup_kernel(ViewDevice V, FrameParams F, const float4 *__restrict__ pos) {
+    lux::after_previous();
     size_t n = (size_t)F.receivers * F.levels;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
         seed_lookup_item<kRanked>(V, F, pos, i, V.order_keys, V.order_vals);
@@ -525,6 +532,7 @@ __device__ __forceinline__ void layout_view(const ViewDevice &V, const FramePara
 }
 
 __global__ void layout_kernel(ViewDevice V, FrameParams F) {
+    lux::after_previous();
     if (threadIdx.x == 0 && blockIdx.x == 0) layout_view(V, F);
 }
 
@@ -540,6 +548,7 @@ __device__ __forceinline__ void clear_entry(const ViewDevice &V, unsigned long l
 }
 
 __global__ void clear_entries_kernel(ViewDevice V, FrameParams F) {
+    lux::after_previous();
     if (*V.error_flags) return;
     unsigned long long n = total_entries(V, F);
     for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; i < n;
@@ -725,6 +734,7 @@ __global__ void __launch_bounds__(128, kFlat ? LUX_FLAT_CLOSEST_MIN_BLOCKS : LUX
                                                             const float4 *__restrict__ pos,
                                                             const float4 *__restrict__ nrm, uint32_t ray_count,
                                                             uint32_t tile) {
+    lux::after_previous();
     if (*V.error_flags) return;
     __shared__ lux::LeafScratch scratch[4];
     lux::LeafScratch *L = &scratch[threadIdx.x >> 5];
@@ -748,6 +758,7 @@ __global__ void __launch_bounds__(128, kFlat ? LUX_FLAT_CLOSEST_MIN_BLOCKS : LUX
 template <bool kFlat>
 __global__ void __launch_bounds__(128, kFlat ? LUX_FLAT_CLOSEST_MIN_BLOCKS : LUX_CLOSEST_MIN_BLOCKS)
     closest_dense_kernel(ViewDevice V, FrameParams F, const __grid_constant__ SceneView S) {
+    lux::after_previous();
     if (*V.error_flags) return;
     __shared__ lux::LeafScratch scratch[4];
     lux::LeafScratch *L = &scratch[threadIdx.x >> 5];
@@ -812,6 +823,7 @@ __global__ void sort_scatter_kernel(ViewDevice V, uint32_t n) {
 
 // The queries' slots in key order (counted by hit shading).
 __global__ void query_scatter_kernel(ViewDevice V, uint32_t capacity) {
+    lux::after_previous();
     const uint32_t n = min(*V.ts.queue_count, capacity);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint32_t slot = V.ts.query_slot[i];
@@ -974,6 +986,7 @@ __device__ __forceinline__ void shade_warp(const ViewDevice &V, const FrameParam
 __global__ void __launch_bounds__(128, LUX_SHADE_MIN_BLOCKS) shade_kernel(ViewDevice V, FrameParams F,
                                                     const __grid_constant__ SceneView S, uint32_t ray_count,
                                                     bool dense, uint32_t per_warp) {
+    lux::after_previous();
     if (*V.error_flags) return;
     __shared__ ShadeScratch scratch[4];
     const uint32_t lane = threadIdx.x & 31u, warps = gridDim.x * 4u;
@@ -1039,6 +1052,7 @@ template <int kDepth, bool kFlat>
 __global__ void __launch_bounds__(128, kFlat ? LUX_FLAT_SHADOW_MIN_BLOCKS : LUX_SHADOW_MIN_BLOCKS)
     shadow_kernel(ViewDevice V, FrameParams F, const __grid_constant__ SceneView S,
                                                                              uint32_t tile) {
+    lux::after_previous();
     if (*V.error_flags) return;
     __shared__ lux::LeafScratch scratch[4];
     lux::LeafScratch *L = &scratch[threadIdx.x >> 5];
@@ -1154,6 +1168,7 @@ __device__ __forceinline__ void deposit_split_ray(const ViewDevice &V, const Fra
 
 __global__ void __launch_bounds__(128) deposit_split_kernel(ViewDevice V, FrameParams F,
                                                             const float4 *__restrict__ nrm, uint32_t ray_count) {
+    lux::after_previous();
     unsigned long long st[7] = {0, 0, 0, 0, 0, 0, 0};
     uint32_t ray = blockIdx.x * blockDim.x + threadIdx.x;
     if (*V.error_flags == 0u && ray < ray_count) deposit_split_ray(V, F, F.shade.frame, nrm, ray, st);
@@ -1161,6 +1176,7 @@ __global__ void __launch_bounds__(128) deposit_split_kernel(ViewDevice V, FrameP
 }
 
 __global__ void __launch_bounds__(128) deposit_dense_kernel(ViewDevice V, FrameParams F) {
+    lux::after_previous();
     if (*V.error_flags) return;
     unsigned long long n = total_entries(V, F);
     for (unsigned long long e = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
@@ -1373,6 +1389,7 @@ __device__ __forceinline__ void for_level_cells(const uint32_t *__restrict__ cel
 // Before the merge, one launch for every level: each cell's corners in the
 // next level, and with history its previous frame's id.
 __global__ void merge_prep_kernel(ViewDevice V, FrameParams F, HistoryDevice H) {
+    lux::after_previous();
     if (*V.error_flags) return;
     if (blockIdx.x == 0 && threadIdx.x < F.levels) V.pass_count[threadIdx.x] = 0u;
     // Eight threads per cell, one corner each; the history map goes to the
@@ -1427,6 +1444,7 @@ __device__ __forceinline__ uint32_t retain_bin(const ViewDevice &V, const FrameP
 }
 
 __global__ void retain_count_kernel(ViewDevice V, FrameParams F, HistoryDevice H) {
+    lux::after_previous();
     for_level_cells(H.cell_count, F, 1u, [&](uint32_t l, uint32_t c) {
         int4 key;
         uint32_t bin = retain_bin(V, F, H, l, c, key);
@@ -1478,6 +1496,7 @@ __device__ __forceinline__ void retain_limit_block(const ViewDevice &V, const Fr
 }
 
 __global__ void __launch_bounds__(kRetainBins) retain_limit_kernel(ViewDevice V, FrameParams F) {
+    lux::after_previous();
     retain_limit_block(V, F);
 }
 
@@ -1505,6 +1524,7 @@ __device__ __forceinline__ void retain_cell(const ViewDevice &V, const FramePara
 }
 
 __global__ void retain_insert_kernel(ViewDevice V, FrameParams F, HistoryDevice H) {
+    lux::after_previous();
     for_level_cells(H.cell_count, F, 1u, [&](uint32_t l, uint32_t c) {
         int4 key;
         if (retain_bin(V, F, H, l, c, key) < V.retain_limit[l]) retain_cell(V, F, H, l, c, key);
@@ -1764,6 +1784,7 @@ __device__ __forceinline__ void merge_children_record(const ViewDevice &V, const
 }
 
 __global__ void __launch_bounds__(256, LUX_MERGE_OWN_MIN_BLOCKS) merge_own_kernel(ViewDevice V, FrameParams F, HistoryDevice H) {
+    lux::after_previous();
     if (*V.error_flags) return;
     for (uint32_t l = 0; l < F.levels; ++l) {
         const uint32_t dirs = F.dirs[l];
@@ -1776,6 +1797,7 @@ __global__ void __launch_bounds__(256, LUX_MERGE_OWN_MIN_BLOCKS) merge_own_kerne
 
 __global__ void __launch_bounds__(LUX_MERGE_THREADS, LUX_MERGE_MIN_BLOCKS)
     merge_children_kernel(ViewDevice V, FrameParams F, uint32_t level) {
+    lux::after_previous();
     if (*V.error_flags) return;
     const uint32_t dirs = F.dirs[level], cells = V.cell_count[level];
     const unsigned long long n = (unsigned long long)cells * dirs;
@@ -1795,6 +1817,7 @@ __global__ void __launch_bounds__(LUX_MERGE_THREADS, LUX_MERGE_MIN_BLOCKS)
 // Levels hold fewer than 2^32 records (checked on the host).
 __global__ void __launch_bounds__(256, LUX_MERGE_OWN_MIN_BLOCKS) merge_own_list_kernel(ViewDevice V, FrameParams F,
                                                                                       HistoryDevice H) {
+    lux::after_previous();
     if (*V.error_flags) return;
     // All levels are one range (level bases are consecutive), so a small
     // frame's levels do not run one latency after another.  A warp whose 32
@@ -1921,6 +1944,7 @@ __device__ __forceinline__ void merge_children_quad(const ViewDevice &V, const F
 // seven levels at 1280x720).
 __global__ void __launch_bounds__(LUX_MERGE_THREADS, LUX_MERGE_MIN_BLOCKS)
     merge_children_list_kernel(ViewDevice V, FrameParams F, uint32_t level) {
+    lux::after_previous();
     if (*V.error_flags) return;
     const uint32_t dirs = F.dirs[level], n = V.pass_count[level];
     const unsigned long long base = V.level_base[level];
@@ -1990,6 +2014,7 @@ __device__ __forceinline__ void pack_cell(const ViewDevice &V, const FrameParams
 }
 
 __global__ void __launch_bounds__(64) pack_kernel(ViewDevice V, FrameParams F) {
+    lux::after_previous();
     if (*V.error_flags) return;
     extern __shared__ float4 smem[];
     float4 *val = smem;            // [dirs]
@@ -2082,9 +2107,9 @@ __device__ __forceinline__ void diffuse_at_lod(const ViewDevice &V, const FrameP
 }
 
 // worldResolve, shaders/world_resolve.slang:96-196, :281-313.
-__global__ void __launch_bounds__(128) resolve_kernel(ViewDevice V, FrameParams F, const float4 *__restrict__ pos,
-                                                      const float4 *__restrict__ nrm, uint32_t count,
-                                                      float4 *__restrict__ out) {
+__global__ void __launch_bounds__(128) resolve_kernel(ViewDevice V, FrameParams F, const float4 *pos,
+                                                      const float4 *nrm, uint32_t count, float4 *out) {
+    lux::after_previous();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
     float4 p = pos[i], n4 = nrm[i];
@@ -3093,7 +3118,7 @@ struct LuxView {
     cudaEvent_t stage_ready = nullptr;
     // Unbatched Split frames: retain, layout and record clearing run on this
     // stream during the closest-hit pass (`seeded` forks it after the seed,
-    // `laid_out` joins it before hit shading).
+    // `laid_out` joins it before the deposit).
     cudaStream_t setup_stream = nullptr;
     cudaEvent_t seeded = nullptr, laid_out = nullptr;
     FrameParams last{};
@@ -3504,7 +3529,7 @@ static void launch_shade(const LuxContext *ctx, const ViewDevice &D, const Frame
     uint32_t per_warp = 32;
     while (per_warp > 4u && (uint64_t)rays < (uint64_t)per_warp * ctx->sm_count * 8u) per_warp /= 2u;
     const int blocks = blocks_for(rays, 4u * per_warp, dense ? ctx->sm_count * 16 : INT32_MAX);
-    shade_kernel<<<blocks, 128, 0, st>>>(D, F, scene->view, rays, dense, per_warp);
+    lux::launch(shade_kernel, blocks, 128, 0, st, D, F, scene->view, rays, dense, per_warp);
 }
 
 // seed: clear, the receivers' cells and dense ids, the sample-sequence order.
@@ -3512,18 +3537,19 @@ static void enqueue_seed(LuxView *v, const FrameParams &F, const float4 *pos, cu
     const ViewDevice &D = v->dev;
     const int most = v->ctx->sm_count * 8;
     const uint64_t slots = (uint64_t)F.levels * F.dir_capacity, places = (uint64_t)F.receivers * F.levels;
-    clear_kernel<<<blocks_for(slots, 256, most), 256, 0, st>>>(D, F);
+    lux::launch(clear_kernel, blocks_for(slots, 256, most), 256, 0, st, D, F);
     if (F.receivers) {
-        seed_insert_kernel<<<blocks_for(places, 256, most), 256, 0, st>>>(D, F, pos);
-        seed_assign_kernel<<<blocks_for(slots, 256, most), 256, 0, st>>>(D, F);
+        lux::launch(seed_insert_kernel, blocks_for(places, 256, most), 256, 0, st, D, F, pos);
+        lux::launch(seed_assign_kernel, blocks_for(slots, 256, most), 256, 0, st, D, F);
         // Cascade-0 cells the receivers can seed (two LODs in an overlap).
         const uint64_t cells = std::min<uint64_t>(F.cell_capacity, (uint64_t)F.receivers * (F.lod_enabled ? 2u : 1u));
         const bool split = F.layout == LUX_LAYOUT_SPLIT, ranked = split && cells <= kRankedCells;
         if (ranked)
-            cell_rank_kernel<<<dim3((unsigned)((cells + 255) / 256), (unsigned)((cells + kRankChunk - 1) / kRankChunk)), 128,
-                               0, st>>>(D, F);
-        (ranked ? seed_lookup_kernel<true> : seed_lookup_kernel<false>)<<<blocks_for(places, 256, most), 256, 0, st>>>(
-            D, F, pos);
+            lux::launch(cell_rank_kernel,
+                        dim3((unsigned)((cells + 255) / 256), (unsigned)((cells + kRankChunk - 1) / kRankChunk)), 128,
+                        0, st, D, F);
+        lux::launch((ranked ? seed_lookup_kernel<true> : seed_lookup_kernel<false>), blocks_for(places, 256, most),
+                    256, 0, st, D, F, pos);
         if (split) {  // the receivers' places in the sample sequence
             size_t bytes = D.order_temp_bytes;
             uint32_t *vals = D.order_vals, *sorted = D.order_vals + v->desc.max_receivers;
@@ -3537,8 +3563,8 @@ static void enqueue_seed(LuxView *v, const FrameParams &F, const float4 *pos, cu
                 cub::DeviceRadixSort::SortPairs(D.order_temp, bytes, D.order_keys, D.order_keys + v->desc.max_receivers,
                                                 vals, sorted, (int)F.receivers, 0, 62, st);
             }
-            ordinal_kernel<<<blocks_for(F.receivers, 256, most), 256, 0, st>>>(D, D.order_vals + v->desc.max_receivers,
-                                                                              F.receivers);
+            lux::launch(ordinal_kernel, blocks_for(F.receivers, 256, most), 256, 0, st, D,
+                        D.order_vals + v->desc.max_receivers, F.receivers);
         }
     }
 }
@@ -3551,12 +3577,12 @@ static void enqueue_layout(LuxView *v, const FrameParams &F, cudaStream_t st) {
         const HistoryDevice H = history_device(v);
         cudaMemsetAsync(D.retain_hist, 0, (size_t)LUX_MAX_LEVELS * kRetainBins * sizeof(uint32_t), st);
         const int blocks = blocks_for((uint64_t)F.cell_capacity * F.levels, 256, most);
-        retain_count_kernel<<<blocks, 256, 0, st>>>(D, F, H);
-        retain_limit_kernel<<<1, kRetainBins, 0, st>>>(D, F);
-        retain_insert_kernel<<<blocks, 256, 0, st>>>(D, F, H);
+        lux::launch(retain_count_kernel, blocks, 256, 0, st, D, F, H);
+        lux::launch(retain_limit_kernel, 1, kRetainBins, 0, st, D, F);
+        lux::launch(retain_insert_kernel, blocks, 256, 0, st, D, F, H);
     }
-    layout_kernel<<<1, 32, 0, st>>>(D, F);
-    clear_entries_kernel<<<blocks_for(F.entry_capacity, 256, most), 256, 0, st>>>(D, F);
+    lux::launch(layout_kernel, 1, 32, 0, st, D, F);
+    lux::launch(clear_entries_kernel, blocks_for(F.entry_capacity, 256, most), 256, 0, st, D, F);
 }
 
 static void enqueue_setup(LuxView *v, const FrameParams &F, const float4 *pos, cudaStream_t st) {
@@ -3574,18 +3600,19 @@ static void enqueue_merge(LuxView *v, const FrameParams &F, cudaStream_t st) {
     const int own_blocks = blocks_for(F.entry_capacity, 256, most * 2);
     const int child_blocks = blocks_for(4ull * F.entry_capacity, LUX_MERGE_THREADS, most * 512 / LUX_MERGE_THREADS);
     if (F.levels > 1 || F.history)
-        merge_prep_kernel<<<blocks_for((uint64_t)F.cell_capacity * F.levels * 8u, 128, most), 128, 0, st>>>(D, F, H);
+        lux::launch(merge_prep_kernel, blocks_for((uint64_t)F.cell_capacity * F.levels * 8u, 128, most), 128, 0, st,
+                    D, F, H);
     // Record indices in the pass list are 32-bit (a level's records).
     const bool listed = LUX_MERGE_COMPACT && F.levels > 1 && v->desc.max_entries <= 0xffffffffull;
     if (listed) {
-        merge_own_list_kernel<<<own_blocks, 256, 0, st>>>(D, F, H);
+        lux::launch(merge_own_list_kernel, own_blocks, 256, 0, st, D, F, H);
         for (int l = (int)F.levels - 2; l >= 0; --l)
-            merge_children_list_kernel<<<child_blocks, LUX_MERGE_THREADS, 0, st>>>(D, F, (uint32_t)l);
+            lux::launch(merge_children_list_kernel, child_blocks, LUX_MERGE_THREADS, 0, st, D, F, (uint32_t)l);
         return;
     }
-    merge_own_kernel<<<own_blocks, 256, 0, st>>>(D, F, H);
+    lux::launch(merge_own_kernel, own_blocks, 256, 0, st, D, F, H);
     for (int l = (int)F.levels - 2; l >= 0; --l)
-        merge_children_kernel<<<child_blocks, LUX_MERGE_THREADS, 0, st>>>(D, F, (uint32_t)l);
+        lux::launch(merge_children_kernel, child_blocks, LUX_MERGE_THREADS, 0, st, D, F, (uint32_t)l);
 }
 
 // Start of an unbatched frame: the last frame's records become the history
@@ -3631,7 +3658,7 @@ static void end_history(LuxView *v, const FrameParams &F) {
 // checked by make_params.
 static void enqueue_pack(LuxView *v, const FrameParams &F, cudaStream_t st) {
     size_t smem = (size_t)F.dirs[0] * 2 * sizeof(float4);
-    pack_kernel<<<blocks_for(F.cell_capacity, 1, v->ctx->sm_count * 8), 64, smem, st>>>(v->dev, F);
+    lux::launch(pack_kernel, blocks_for(F.cell_capacity, 1, v->ctx->sm_count * 8), 64, smem, st, v->dev, F);
 }
 
 // Next-event slots of one hit: the emissive samples (max(1, n / 2)), as many
@@ -3901,10 +3928,14 @@ static lux_status view_frame(LuxView *v, const LuxScene *scene, const LuxSetting
                 auto kernel = flat ? closest_split_kernel<64, true>
                                    : (T.stack_depth == 32 ? closest_split_kernel<32, false>
                                                           : closest_split_kernel<64, false>);
-                kernel<<<trace_blocks(ctx, T.closest_blocks_per_sm, tile_of(T), rays), 128, 0, st>>>(
-                    Dr, F, scene->view, pos, nrm, rays, tile_of(T));
+                lux::launch(kernel, trace_blocks(ctx, T.closest_blocks_per_sm, tile_of(T), rays), 128, 0, st, Dr, F,
+                            scene->view, pos, nrm, rays, tile_of(T));
             }
-            if (forked) cudaStreamWaitEvent(st, v->laid_out, 0);  // join the setup stream
+            // The setup stream joins where it is needed: its cleared query bins
+            // by shading, the records' layout by the deposit (in a short frame
+            // the retained cells take longer than the closest hits: shading
+            // began 12 us later in a 385-ray frame).
+            if (forked && query_bits) cudaStreamWaitEvent(st, v->laid_out, 0);
             ViewDevice Dq = D;  // query pass view: keys counted by shade, optional order
             Dq.query_bits = query_bits;
             if (query_bits && (!forked || T.sort_rays))
@@ -3913,7 +3944,7 @@ static lux_status view_frame(LuxView *v, const LuxScene *scene, const LuxSetting
             const uint64_t queries = most_queries(F, scene, rays);
             if (query_bits) {
                 enqueue_sort_scan(D, query_bins(query_bits), st);
-                query_scatter_kernel<<<blocks_for(queries, 256, most), 256, 0, st>>>(D, F.queue_capacity);
+                lux::launch(query_scatter_kernel, blocks_for(queries, 256, most), 256, 0, st, D, F.queue_capacity);
                 Dq.query_order = D.sort_perm;
             }
             if (T.shadow_mode == 1)
@@ -3922,8 +3953,8 @@ static lux_status view_frame(LuxView *v, const LuxScene *scene, const LuxSetting
             else {
                 auto kernel = flat ? shadow_kernel<64, true>
                                    : (T.stack_depth == 32 ? shadow_kernel<32, false> : shadow_kernel<64, false>);
-                kernel<<<trace_blocks(ctx, T.shadow_blocks_per_sm, tile_of(T), queries), 128, 0, st>>>(Dq, F, scene->view,
-                                                                                                     tile_of(T));
+                lux::launch(kernel, trace_blocks(ctx, T.shadow_blocks_per_sm, tile_of(T), queries), 128, 0, st, Dq, F,
+                            scene->view, tile_of(T));
             }
             if (cached) {
                 const int g = ctx->sm_count * 8;
@@ -3932,7 +3963,8 @@ static lux_status view_frame(LuxView *v, const LuxScene *scene, const LuxSetting
                 if (qrc != LUX_OK) return qrc;
                 cache_apply_kernel<<<g, 256, 0, st>>>(D, F, rays, C);
             }
-            deposit_split_kernel<<<(rays + 127) / 128, 128, 0, st>>>(D, F, nrm, rays);
+            if (forked) cudaStreamWaitEvent(st, v->laid_out, 0);
+            lux::launch(deposit_split_kernel, (rays + 127) / 128, 128, 0, st, D, F, nrm, rays);
             if (cached) {
                 const int g = ctx->sm_count * 8;
                 cache_count_kernel<<<g, 256, 0, st>>>(D, F, rays, C);
@@ -3947,12 +3979,13 @@ static lux_status view_frame(LuxView *v, const LuxScene *scene, const LuxSetting
         const bool flat = scene->view.flat_nodes != nullptr;
         const uint64_t rays = std::min<uint64_t>(F.ray_capacity, F.entry_capacity);  // one per record
         const int blocks = blocks_for(rays, 128, ctx->sm_count * 16);
-        (flat ? closest_dense_kernel<true> : closest_dense_kernel<false>)<<<blocks, 128, 0, st>>>(D, F, scene->view);
+        lux::launch((flat ? closest_dense_kernel<true> : closest_dense_kernel<false>), blocks, 128, 0, st, D, F,
+                    scene->view);
         launch_shade(ctx, D, F, scene, (uint32_t)rays, true, st);
-        (flat ? shadow_kernel<64, true> : shadow_kernel<64, false>)
-            <<<trace_blocks(ctx, v->tuning.shadow_blocks_per_sm, tile_of(v->tuning), most_queries(F, scene, rays)), 128, 0,
-               st>>>(D, F, scene->view, tile_of(v->tuning));
-        deposit_dense_kernel<<<blocks, 128, 0, st>>>(D, F);
+        lux::launch((flat ? shadow_kernel<64, true> : shadow_kernel<64, false>),
+                    trace_blocks(ctx, v->tuning.shadow_blocks_per_sm, tile_of(v->tuning), most_queries(F, scene, rays)),
+                    128, 0, st, D, F, scene->view, tile_of(v->tuning));
+        lux::launch(deposit_dense_kernel, blocks, 128, 0, st, D, F);
     }
     mark(2);
     enqueue_merge(v, F, st);
@@ -3993,8 +4026,8 @@ extern "C" lux_status lux_view_resolve(LuxView *v, const LuxSettings *settings, 
     if (!v->has_frame) return lux_fail(v->ctx, LUX_ERR_INVALID_ARGUMENT, "resolve: no frame traced yet");
     if (count == 0) return LUX_OK;
     if (v->timing) cudaEventRecord(v->ev[5], v->ctx->stream);
-    resolve_kernel<<<(count + 127) / 128, 128, 0, v->ctx->stream>>>(v->dev, v->last, (const float4 *)ppos,
-                                                                      (const float4 *)pnrm, count, (float4 *)out);
+    lux::launch(resolve_kernel, (count + 127) / 128, 128, 0, v->ctx->stream, v->dev, v->last, (const float4 *)ppos,
+           (const float4 *)pnrm, count, (float4 *)out);
     if (v->timing) cudaEventRecord(v->ev[6], v->ctx->stream);
     return lux_cuda_check(v->ctx, (int)cudaGetLastError(), "resolve launch");
 }
@@ -4195,6 +4228,7 @@ extern "C" lux_status lux_view_get_tuning(const LuxView *v, LuxTuning *t) {
 namespace {
 
 __global__ void scratch_clear_kernel(ViewDevice V) {
+    lux::after_previous();
     if (threadIdx.x == 0 && blockIdx.x == 0) {
         *V.error_flags = 0;
         *V.ts.queue_count = 0;
@@ -4208,6 +4242,7 @@ template <bool kFlat>
 __global__ void __launch_bounds__(128, kFlat ? LUX_FLAT_CLOSEST_MIN_BLOCKS : LUX_CLOSEST_MIN_BLOCKS)
     closest_rays_kernel(ViewDevice V, const __grid_constant__ SceneView S, const LuxRay *__restrict__ rays,
                         uint32_t count) {
+    lux::after_previous();
     __shared__ lux::LeafScratch scratch[4];
     lux::LeafScratch *L = &scratch[threadIdx.x >> 5];
     uint32_t traced = 0;
@@ -4231,6 +4266,7 @@ __global__ void __launch_bounds__(128, kFlat ? LUX_FLAT_CLOSEST_MIN_BLOCKS : LUX
 
 // out[i] = (radiance rgb, hit distance) or (0, 0, 0, -1) when unsupported.
 __global__ void radiance_out_kernel(ViewDevice V, uint32_t count, float4 *__restrict__ out) {
+    lux::after_previous();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
     f3 radiance;
@@ -4258,15 +4294,15 @@ lux_status launch_interval_radiance(LuxContext *ctx, const LuxScene *scene, cons
     F.shade.frame = s.frame_index;
     F.shade.environment = f3{s.environment[0], s.environment[1], s.environment[2]};
     cudaStream_t st = ctx->stream;
-    scratch_clear_kernel<<<1, 32, 0, st>>>(V);
+    lux::launch(scratch_clear_kernel, 1, 32, 0, st, V);
     if (count) {
         const bool flat = scene->view.flat_nodes != nullptr;
-        (flat ? closest_rays_kernel<true> : closest_rays_kernel<false>)<<<trace_blocks(ctx, 16u, 32u, count), 128, 0, st>>>(
-            V, scene->view, rays, count);
+        lux::launch((flat ? closest_rays_kernel<true> : closest_rays_kernel<false>),
+                    trace_blocks(ctx, 16u, 32u, count), 128, 0, st, V, scene->view, rays, count);
         launch_shade(ctx, V, F, scene, count, false, st);
-        (flat ? shadow_kernel<64, true> : shadow_kernel<64, false>)
-            <<<trace_blocks(ctx, 16u, 32u, most_queries(F, scene, count)), 128, 0, st>>>(V, F, scene->view, 32u);
-        radiance_out_kernel<<<(count + 127) / 128, 128, 0, st>>>(V, count, (float4 *)out);
+        lux::launch((flat ? shadow_kernel<64, true> : shadow_kernel<64, false>),
+                    trace_blocks(ctx, 16u, 32u, most_queries(F, scene, count)), 128, 0, st, V, F, scene->view, 32u);
+        lux::launch(radiance_out_kernel, (count + 127) / 128, 128, 0, st, V, count, (float4 *)out);
     }
     return lux_cuda_check(ctx, (int)cudaGetLastError(), "interval_radiance launch");
 }
