@@ -438,7 +438,7 @@ __device__ __forceinline__ unsigned long long sequence_key(int32_t x, int32_t y,
 }
 
 // sorted: the receiver indices in sequence order (the sort's output half).
-__global__ void ordinal_kernel(ViewDevice V, const uint32_t *__restrict__ sorted, uint32_t receivers) {
+__global__ void ordinal_kernel(ViewDevice V, const uint32_t *sorted, uint32_t receivers) {
     lux::after_previous();
     for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < receivers; j += gridDim.x * blockDim.x)
         V.receiver_ordinal[sorted[j]] = j;
