@@ -27,18 +27,18 @@ __device__ __forceinline__ void after_previous() {
 // kernel<<<grid, block, smem, st>>>(args...) for a kernel that begins with
 // after_previous.  After anything but a kernel it is an ordinary launch.
 template <typename... P, typename... A>
-inline void launch(void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t st, A &&...args) {
+inline void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A &&...args) {
     cudaLaunchAttribute early[1];
     early[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     early[0].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
-    cfg.blockDim = dim3(block);
+    cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cfg.attrs = early;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
 }  // namespace lux

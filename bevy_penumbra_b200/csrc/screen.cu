@@ -25,6 +25,7 @@
 #include <cmath>
 #include <cstring>
 
+#include "launch.cuh"
 #include "lux_internal.h"
 #include "lux_math.cuh"
 
@@ -128,6 +129,7 @@ __device__ __forceinline__ float lerpf(float a, float b, float t) { return a + t
 constexpr int kTemporalTile = 16, kTemporalSpan = kTemporalTile + 2;
 __global__ void __launch_bounds__(256, LUX_TEMPORAL_BLOCKS) temporal_kernel(ScreenParams P, Input in, History H,
                                                                             History out) {
+    lux::after_previous();
     __shared__ float4 s_irr[kTemporalSpan * kTemporalSpan], s_pos[kTemporalSpan * kTemporalSpan];
     __shared__ float4 s_nrm[kTemporalSpan * kTemporalSpan];
     __shared__ uint2 s_id[kTemporalSpan * kTemporalSpan];
@@ -361,6 +363,7 @@ __device__ __forceinline__ float power32(float c) {
 // output's own (meta.z).  dst_mask: nullptr when no pass follows.
 __global__ void __launch_bounds__(256, LUX_DENOISE_BLOCKS) denoise_kernel(ScreenParams P, Input in, History T, const float4 *src,
                                                       const float *src_mask, float4 *dst, float *dst_mask) {
+    lux::after_previous();
     __shared__ float4 s_value[kDenoiseSpan * kDenoiseSpan], s_nrm[kDenoiseSpan * kDenoiseSpan];
     __shared__ float4 s_pos[kDenoiseSpan * kDenoiseSpan];
     __shared__ uint2 s_id[kDenoiseSpan * kDenoiseSpan];
@@ -551,7 +554,7 @@ extern "C" lux_status lux_screen_filter(LuxScreen *s, const LuxSettings *setting
     cudaStream_t stream = ctx->stream;
     dim3 block(16, 16), grid((s->width + 15) / 16, (s->height + 15) / 16);
     History &prev = s->h[s->cur], &next = s->h[1 - s->cur];
-    temporal_kernel<<<grid, block, 0, stream>>>(P, in, prev, next);
+    lux::launch(temporal_kernel, grid, block, 0, stream, P, in, prev, next);
     s->cur = 1 - s->cur;
     s->valid = true;
     const History &T = s->h[s->cur];
@@ -572,7 +575,7 @@ extern "C" lux_status lux_screen_filter(LuxScreen *s, const LuxSettings *setting
         // Blocks of 16 x 16 pixels of one lattice phase, step x step phases.
         const uint32_t lu = (s->width + P.step - 1) / P.step, lv = (s->height + P.step - 1) / P.step;
         dim3 lattice(P.step * ((lu + kDenoiseTile - 1) / kDenoiseTile), P.step * ((lv + kDenoiseTile - 1) / kDenoiseTile));
-        denoise_kernel<<<lattice, block, 0, stream>>>(P, in, T, src, src_mask, dst, dst_mask);
+        lux::launch(denoise_kernel, lattice, block, 0, stream, P, in, T, src, src_mask, dst, dst_mask);
         src = dst;
         src_mask = dst_mask;
     }
