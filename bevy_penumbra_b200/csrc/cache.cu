@@ -271,9 +271,11 @@ __device__ __forceinline__ float2 bf16x2_floats(uint32_t v) {
 }
 __global__ void __launch_bounds__(128, 8)
     encode_kernel(GridParams G, const LuxCacheSample *__restrict__ samples, uint32_t n,
-                  const uint32_t *__restrict__ n_dev, const uint32_t *__restrict__ table, uint4 *__restrict__ out) {
+                  const uint32_t *__restrict__ n_dev, const uint32_t *__restrict__ table, uint4 *__restrict__ out,
+                  float *__restrict__ loss) {
     const unsigned long long t = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
     if (n_dev) n = min(n, *n_dev);
+    if (t == 0 && loss) *loss = 0.0f;  // of the training pass that follows
     if (t >> 2 >= n) return;
     const uint32_t i = (uint32_t)(t >> 2), q = (uint32_t)t & 3u;
     const LuxCacheSample &s = samples[i];
@@ -1006,7 +1008,7 @@ extern "C" lux_status lux_cache_encode(LuxCache *c, const LuxCacheSample *sample
     if (count == 0) return LUX_OK;
     cudaSetDevice(c->ctx->device);
     encode_kernel<<<encode_blocks(count), 128, 0, c->ctx->stream>>>(
-        c->grid, samples, count, nullptr, (const uint32_t *)c->table, (uint4 *)out);
+        c->grid, samples, count, nullptr, (const uint32_t *)c->table, (uint4 *)out, nullptr);
     return lux_cuda_check(c->ctx, (int)cudaGetLastError(), "cache: encode launch");
 }
 
@@ -1024,7 +1026,7 @@ extern "C" lux_status lux_cache_query(LuxCache *c, const LuxCacheSample *queries
     lux_status rc = ensure_rows(c, count);
     if (rc != LUX_OK) return rc;
     encode_kernel<<<encode_blocks(count), 128, 0, c->ctx->stream>>>(c->grid, queries, count, nullptr,
-                                                                   (const uint32_t *)c->table, c->x);
+                                                                   (const uint32_t *)c->table, c->x, nullptr);
     return cache_forward(c, c->x, count, nullptr, out, 1);
 }
 
@@ -1035,7 +1037,7 @@ lux_status lux_cache_query_device_count(LuxCache *c, const LuxCacheSample *queri
     lux_status rc = ensure_rows(c, max_count);
     if (rc != LUX_OK) return rc;
     encode_kernel<<<encode_blocks(max_count), 128, 0, c->ctx->stream>>>(c->grid, queries, max_count, count,
-                                                                       (const uint32_t *)c->table, c->x);
+                                                                       (const uint32_t *)c->table, c->x, nullptr);
     return cache_forward(c, c->x, max_count, count, out, 1);
 }
 
@@ -1052,8 +1054,7 @@ extern "C" lux_status lux_cache_train(LuxCache *c, const LuxCacheSample *samples
         uint32_t nb = std::min(batch, count - s0);
         const LuxCacheSample *sb = samples + s0;
         encode_kernel<<<encode_blocks(nb), 128, 0, st>>>(c->grid, sb, nb, nullptr, (const uint32_t *)c->table,
-                                                        c->x);
-        cudaMemsetAsync(c->loss, 0, 4, st);
+                                                        c->x, c->loss);
         uint32_t tiles = (nb + kTile - 1) / kTile;
         mlp_train_kernel<<<std::min<uint32_t>(tiles, (uint32_t)ctx->sm_count), kTile, kTrainSmem, st>>>(
             c->x, (const float4 *)targets + s0, sb, nb, 1.0f / (3.0f * (float)nb), (const uint4 *)c->w_packed,
@@ -1112,8 +1113,7 @@ extern "C" lux_status lux_cache_gradients(LuxCache *c, const LuxCacheSample *sam
     if (rc != LUX_OK) return rc;
     cudaStream_t st = ctx->stream;
     encode_kernel<<<encode_blocks(count), 128, 0, st>>>(c->grid, samples, count, nullptr,
-                                                       (const uint32_t *)c->table, c->x);
-    cudaMemsetAsync(c->loss, 0, 4, st);
+                                                       (const uint32_t *)c->table, c->x, c->loss);
     uint32_t tiles = (count + kTile - 1) / kTile;
     mlp_train_kernel<<<std::min<uint32_t>(tiles, (uint32_t)ctx->sm_count), kTile, kTrainSmem, st>>>(
         c->x, (const float4 *)targets, samples, count, 1.0f / (3.0f * (float)count), (const uint4 *)c->w_packed,
