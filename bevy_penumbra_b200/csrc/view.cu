@@ -169,6 +169,7 @@ struct ViewDevice {
     uint32_t *receiver_ordinal;     // [max_receivers] the receiver's place in the sample sequence
     unsigned long long *order_keys; // [2][max_receivers] sequence-order sort keys (in, out; 32-bit when ranked)
     uint32_t *cell_rank;            // [max_cells] place of each cascade-0 cell in the sequence order
+    unsigned long long *rank_keys;  // [ranked cells, whole pieces] their sequence keys, sorted piece by piece
     uint32_t *order_vals;           // [2][max_receivers] receiver indices (in, out)
     void *order_temp;               // radix-sort scratch
     size_t order_temp_bytes;
@@ -447,36 +448,81 @@ __global__ void ordinal_kernel(ViewDevice V, const uint32_t *sorted, uint32_t re
 // The sequence order by cells: receivers of one cell are consecutive and in
 // index order, so a receiver's key can be its cell's place among the frame's
 // cascade-0 cells, a number of few bits, instead of the cell's 62-bit key: the
-// radix sort then takes 2 passes where it took 8 (14,400 receivers: 100 us with
-// its clears, 30 now with the ranking).  The place is a count over all pairs
-// of cells, which is cheap while the cells are few (kRankedCells); above that
-// the 62-bit keys are sorted.  Block (x, y): 256 cells, two per thread, against
-// 256.
-constexpr uint32_t kRankedCells = 16384, kRankChunk = 256;
-__global__ void __launch_bounds__(128) cell_rank_kernel(ViewDevice V, FrameParams F) {
+// radix sort then takes 2 or 3 passes where it took 8, at some 11 us per pass
+// and its clears (14,400 receivers 100 -> 30 us, 61,050 in 40,000 places for
+// cells 105 -> 42, ranking included).  Pieces of 256 cells (1024 where there may be
+// many) are sorted in shared memory, then each cell's place is the sum of its places in all pieces;
+// that grows with the square of the cells, so above kRankedCells the 62-bit keys
+// are sorted.
+constexpr uint32_t kRankedCells = 1u << 17, kRankTile = 512;
+constexpr uint32_t kSmallPiece = 256, kLargePiece = 1024, kSmallPieceCells = 16384;
+__device__ __forceinline__ unsigned long long cell_sequence_key(const ViewDevice &V, uint32_t cell) {
+    const int4 q = V.cell_keys[cell];
+    return sequence_key(q.x, q.y, q.z, lux::key_lod(q.w));
+}
+template <uint32_t kPiece>
+__global__ void __launch_bounds__(kPiece / 2) cell_piece_kernel(ViewDevice V, FrameParams F) {
     lux::after_previous();
-    __shared__ __align__(16) unsigned long long key[kRankChunk];
-    const uint32_t cells = min(V.cell_count[0], F.cell_capacity);
-    const uint32_t c = blockIdx.x * 256u + threadIdx.x, first = blockIdx.y * kRankChunk;
-    if (blockIdx.x * 256u >= cells || first >= cells) return;
-    const uint32_t n = min(kRankChunk, cells - first);
-    auto key_of = [&](uint32_t cell) {
-        const int4 q = V.cell_keys[cell];
-        return sequence_key(q.x, q.y, q.z, lux::key_lod(q.w));
-    };
-    for (uint32_t k = threadIdx.x; k < kRankChunk; k += 128u) key[k] = k < n ? key_of(first + k) : ~0ull;  // before no cell
-    __syncthreads();
-    if (c >= cells) return;
-    const unsigned long long a = key_of(c), b = c + 128u < cells ? key_of(c + 128u) : 0ull;
-    uint32_t before_a = 0, before_b = 0;
-#pragma unroll 8
-    for (uint32_t k = 0; k < kRankChunk; k += 2u) {
-        const ulonglong2 two = *reinterpret_cast<const ulonglong2 *>(&key[k]);
-        before_a += (two.x < a ? 1u : 0u) + (two.y < a ? 1u : 0u);
-        before_b += (two.x < b ? 1u : 0u) + (two.y < b ? 1u : 0u);
+    __shared__ ulonglong2 pair[kPiece / 2];
+    const uint32_t cells = min(V.cell_count[0], F.cell_capacity), first = blockIdx.x * kPiece, t = threadIdx.x;
+    if (first >= cells) return;
+    // Thread t holds elements 2 t and 2 t + 1; those after every cell are ones.
+    // Bitonic: partners within a warp exchange by shuffles, others through
+    // shared memory (of 1024 elements, all stages there took 13 us, not 5).
+    const uint32_t e = first + 2u * t;
+    unsigned long long x = e < cells ? cell_sequence_key(V, e) : ~0ull;
+    unsigned long long y = e + 1u < cells ? cell_sequence_key(V, e + 1u) : ~0ull;
+#pragma unroll
+    for (uint32_t size = 2; size <= kPiece; size <<= 1) {
+        const bool up = ((2u * t) & size) == 0u;
+#pragma unroll
+        for (uint32_t stride = size >> 1; stride >= 2u; stride >>= 1) {
+            unsigned long long ox, oy;
+            if (stride >= 64u) {
+                __syncthreads();
+                pair[t] = make_ulonglong2(x, y);
+                __syncthreads();
+                const ulonglong2 o = pair[t ^ (stride >> 1)];
+                ox = o.x;
+                oy = o.y;
+            } else {
+                ox = __shfl_xor_sync(0xffffffffu, x, stride >> 1);
+                oy = __shfl_xor_sync(0xffffffffu, y, stride >> 1);
+            }
+            const bool low = ((t & (stride >> 1)) == 0u) == up;
+            x = low ? min(x, ox) : max(x, ox);
+            y = low ? min(y, oy) : max(y, oy);
+        }
+        const unsigned long long least = min(x, y), most = max(x, y);
+        x = up ? least : most;
+        y = up ? most : least;
     }
-    if (before_a) atomicAdd(&V.cell_rank[c], before_a);
-    if (before_b) atomicAdd(&V.cell_rank[c + 128u], before_b);
+    reinterpret_cast<ulonglong2 *>(V.rank_keys + first)[t] = make_ulonglong2(x, y);
+}
+template <uint32_t kPiece>
+__global__ void __launch_bounds__(256) cell_rank_kernel(ViewDevice V, FrameParams F) {
+    lux::after_previous();
+    __shared__ __align__(16) unsigned long long key[kPiece];
+    const uint32_t cells = min(V.cell_count[0], F.cell_capacity);
+    const uint32_t pieces = (cells + kPiece - 1u) / kPiece, tiles = (cells + kRankTile - 1u) / kRankTile;
+    for (uint32_t at = blockIdx.x; at < pieces * tiles; at += gridDim.x) {
+        const ulonglong2 *piece = reinterpret_cast<const ulonglong2 *>(V.rank_keys + (size_t)(at / tiles) * kPiece);
+        __syncthreads();  // the previous piece is no longer read
+        for (uint32_t k = threadIdx.x; k < kPiece / 2u; k += 256u) reinterpret_cast<ulonglong2 *>(key)[k] = piece[k];
+        __syncthreads();
+#pragma unroll
+        for (uint32_t half = 0; half < kRankTile; half += 256u) {
+            const uint32_t c = (at % tiles) * kRankTile + half + threadIdx.x;
+            if (c >= cells) continue;
+            const unsigned long long mine = cell_sequence_key(V, c);
+            uint32_t before = 0;
+#pragma unroll
+            for (uint32_t step = kPiece / 2u; step; step >>= 1)
+                if (key[before + step - 1u] < mine) before += step;
+            if (key[before] < mine) ++before;  // all of the piece
+            if (before) atomicAdd(&V.cell_rank[c], before);
+        }
+    }
 }
 
 // Item i = level x receivers + receiver; the receiver's sequence key and index
@@ -708,13 +754,18 @@ __device__ __forceinline__ uint32_t warp_fetch(uint32_t *counter, uint32_t tile 
 // 16 in half the warps (27k queries 57 -> 48 us).  Warps past the items fetch
 // nothing.
 constexpr uint32_t kFewestLanes = 4;
-template <uint32_t kShare, uint32_t kMostFew, typename Fn>
-__device__ __forceinline__ void for_warp_items(uint32_t *counter, uint32_t n, uint32_t tile, Fn &&fn) {
-    const uint32_t lane = threadIdx.x & 31u, warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+template <uint32_t kShare, uint32_t kMostFew>
+__device__ __forceinline__ uint32_t walks_per_warp(uint32_t n) {
     const uint32_t warps = gridDim.x * (blockDim.x >> 5) / kShare;
     uint32_t lanes = 32u;
     if ((unsigned long long)warps * kMostFew >= n)
         for (lanes = kMostFew; lanes > kFewestLanes && (unsigned long long)warps * (lanes >> 1) >= n;) lanes >>= 1;
+    return lanes;
+}
+template <uint32_t kShare, uint32_t kMostFew, typename Fn>
+__device__ __forceinline__ void for_warp_items(uint32_t *counter, uint32_t n, uint32_t tile, Fn &&fn) {
+    const uint32_t lane = threadIdx.x & 31u, warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t lanes = walks_per_warp<kShare, kMostFew>(n);
     if (lanes < 32u) {
         const uint32_t slot = warp * lanes + lane;
         if (slot - lane < n) fn(slot, lane < lanes && slot < n);
@@ -2165,7 +2216,7 @@ uint32_t next_pow2(uint64_t v) {
 // warp-sized chunk lies inside one job: the job is warp-uniform, per-view
 // warp aggregation (query append, stats) works unchanged, and a warp reads
 // its job's parameters as broadcasts.
-struct BatchJob {
+struct alignas(16) BatchJob {
     ViewDevice V;
     FrameParams F;
     SceneView S;
@@ -2212,10 +2263,13 @@ __device__ __forceinline__ void closest_batch_phase(const BatchJob *__restrict__
     uint32_t cur = lux::kEmpty;
     unsigned long long st[7] = {0, 0, 0, 0, 0, 0, 0};
     lux::TraceCounters cn{0, 0, 0};
-    while (true) {
-        const uint32_t first = warp_fetch(counter, tile);
-        if (first >= total) break;
-        for (uint32_t base = first; base < first + tile && base < total; base += 32u) {
+    // Few walks per warp in small batches, as for_warp_items; 4, 8 or 16 items of
+    // the 32-padded rows belong to one job too.
+    const uint32_t lanes = walks_per_warp<1u, 8u>(total), size = lanes < 32u ? lanes : tile;
+    const uint32_t own = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * lanes;
+    for (uint32_t first = lanes < 32u ? own : warp_fetch(counter, tile); first < total;
+         first = lanes < 32u ? total : warp_fetch(counter, tile)) {
+        for (uint32_t base = first; base < first + size && base < total; base += 32u) {
             uint32_t j = find_job(begin, n, base);
             const BatchJob &J = jobs[j];
             if (j != cur) {
@@ -2223,9 +2277,10 @@ __device__ __forceinline__ void closest_batch_phase(const BatchJob *__restrict__
                 cur = j;
             }
             if (__shfl_sync(0xffffffffu, *J.V.error_flags, 0)) continue;  // one value for the warp
-            uint32_t slot = base - __ldg(begin + j) + lane;
-            closest_split_ray_warp<lux::kStack, kFlat>(J.V, J.F, fr, J.S, J.pos, J.nrm, slot, slot < J.rays, cn, L);
-            if (slot < J.rays) st[kStatInterval] += 1;
+            const uint32_t slot = base - __ldg(begin + j) + lane;
+            const bool valid = lane < lanes && slot < J.rays;
+            closest_split_ray_warp<lux::kStack, kFlat>(J.V, J.F, fr, J.S, J.pos, J.nrm, slot, valid, cn, L);
+            if (valid) st[kStatInterval] += 1;
         }
     }
     if (cur != lux::kEmpty) flush_stats(jobs[cur].V.stats, st, cn, false);
@@ -2305,10 +2360,13 @@ __device__ __forceinline__ void shadow_batch_phase(const BatchJob *__restrict__ 
     uint32_t cur = lux::kEmpty;
     unsigned long long st[7] = {0, 0, 0, 0, 0, 0, 0};
     lux::TraceCounters cn{0, 0, 0};
-    while (true) {
-        const uint32_t first = warp_fetch(counter, tile);
-        if (first >= total) break;
-        for (uint32_t base = first; base < first + tile && base < total; base += 32u) {
+    // Few walks per warp in small batches, as for_warp_items; 4, 8 or 16 items of
+    // the 32-padded rows belong to one job too.
+    const uint32_t lanes = walks_per_warp<2u, 16u>(total), size = lanes < 32u ? lanes : tile;
+    const uint32_t own = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * lanes;
+    for (uint32_t first = lanes < 32u ? own : warp_fetch(counter, tile); first < total;
+         first = lanes < 32u ? total : warp_fetch(counter, tile)) {
+        for (uint32_t base = first; base < first + size && base < total; base += 32u) {
             uint32_t j = find_query_job(qbegin, n, base);
             const BatchJob &J = jobs[j];
             if (j != cur) {
@@ -2316,7 +2374,7 @@ __device__ __forceinline__ void shadow_batch_phase(const BatchJob *__restrict__ 
                 cur = j;
             }
             uint32_t i = base - qbegin[j] + lane;
-            const bool valid = i < job_queries(J);
+            const bool valid = lane < lanes && i < job_queries(J);
             shadow_query_warp<lux::kStack, kFlat>(J.V, J.S, i, valid, cn, L);
             if (valid) st[kStatShadow] += 1;
         }
@@ -2680,9 +2738,12 @@ __global__ void batch_clear_entries_kernel(const BatchJob *__restrict__ jobs,
 __global__ void batch_merge_prep_kernel(const BatchJob *__restrict__ jobs, const unsigned long long *__restrict__ dom,
                                         uint32_t n, const unsigned long long *__restrict__ count, uint32_t levels) {
     // Every job's list lengths start at zero (the listing own pass follows).
-    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n * LUX_MAX_LEVELS; k += gridDim.x * blockDim.x)
-        jobs[k / LUX_MAX_LEVELS].V.pass_count[k % LUX_MAX_LEVELS] = 0u;
-    for (uint32_t l = 0; l < levels; ++l) {
+    if (blockIdx.y == 0u)
+        for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n * LUX_MAX_LEVELS; k += gridDim.x * blockDim.x)
+            jobs[k / LUX_MAX_LEVELS].V.pass_count[k % LUX_MAX_LEVELS] = 0u;
+    // A row of blocks per level: small views' levels run beside one another
+    // instead of one latency after another (six views of 427x240: 42 -> 13 us).
+    for (uint32_t l = blockIdx.y; l < levels; l += gridDim.y) {
         const unsigned long long *cells = count + (size_t)(kRowCells - kRowEntries + l) * n;
         for_batch_items(batch_row(dom, n, kRowCells + l), n, [&](uint32_t j, unsigned long long c) {
             const BatchJob &J = jobs[j];
@@ -3213,6 +3274,7 @@ static lux_status view_alloc(LuxView *v) {
         {(void **)&D.order_keys, 2 * (size_t)d.max_receivers * sizeof(unsigned long long)},
         {(void **)&D.order_vals, 2 * (size_t)d.max_receivers * sizeof(uint32_t)},
         {(void **)&D.cell_rank, (size_t)d.max_cells * sizeof(uint32_t)},
+        {(void **)&D.rank_keys, ((size_t)std::min(d.max_cells, kRankedCells) + kLargePiece) * sizeof(unsigned long long)},
         {(void **)&D.order_temp, order_temp_bytes(d.max_receivers)},
         {(void **)&D.corner_ids, L * (size_t)d.max_cells * 8 * sizeof(uint32_t)},
         {(void **)&D.corner_frac, L * (size_t)d.max_cells * sizeof(float4)},
@@ -3345,7 +3407,7 @@ extern "C" lux_status lux_view_destroy(LuxView *v) {
     if (!v) return LUX_OK;
     ViewDevice &D = v->dev;
     void *ptrs[] = {D.dir_keys, D.dir_ids, D.cell_keys, D.cell_count, D.level_base, D.receiver_cell, D.receiver_lod,
-                    D.receiver_ordinal, D.order_keys, D.order_vals, D.cell_rank, D.order_temp,
+                    D.receiver_ordinal, D.order_keys, D.order_vals, D.cell_rank, D.rank_keys, D.order_temp,
                     D.corner_ids,
                     D.corner_frac, D.accum, D.count, D.merged, D.raw, D.mass, D.hist_cell, D.cell_last,
                     D.retain_hist, D.retain_limit, D.tables, D.error_flags, D.stats,
@@ -3544,10 +3606,17 @@ static void enqueue_seed(LuxView *v, const FrameParams &F, const float4 *pos, cu
         // Cascade-0 cells the receivers can seed (two LODs in an overlap).
         const uint64_t cells = std::min<uint64_t>(F.cell_capacity, (uint64_t)F.receivers * (F.lod_enabled ? 2u : 1u));
         const bool split = F.layout == LUX_LAYOUT_SPLIT, ranked = split && cells <= kRankedCells;
-        if (ranked)
-            lux::launch(cell_rank_kernel,
-                        dim3((unsigned)((cells + 255) / 256), (unsigned)((cells + kRankChunk - 1) / kRankChunk)), 128,
-                        0, st, D, F);
+        if (ranked) {
+            // A piece of 256 is sorted in half the time of 1024, but four times
+            // the pieces are searched for each cell.
+            const bool small = cells <= kSmallPieceCells;
+            const uint32_t piece = small ? kSmallPiece : kLargePiece;
+            const uint64_t pieces = (cells + piece - 1) / piece, tiles = pieces * ((cells + kRankTile - 1) / kRankTile);
+            lux::launch(small ? cell_piece_kernel<kSmallPiece> : cell_piece_kernel<kLargePiece>, (unsigned)pieces,
+                        piece / 2, 0, st, D, F);
+            lux::launch(small ? cell_rank_kernel<kSmallPiece> : cell_rank_kernel<kLargePiece>,
+                        (unsigned)std::min<uint64_t>(tiles, (uint64_t)most), 256, 0, st, D, F);
+        }
         lux::launch((ranked ? seed_lookup_kernel<true> : seed_lookup_kernel<false>), blocks_for(places, 256, most),
                     256, 0, st, D, F, pos);
         if (split) {  // the receivers' places in the sample sequence
@@ -3868,8 +3937,10 @@ static lux_status view_frame(LuxView *v, const LuxScene *scene, const LuxSetting
     // rest of the setup runs beside it on the setup stream.
     bool forked = false;
     if (F.layout == LUX_LAYOUT_SPLIT && rc->count && !cached_frame) {
+        int setup_priority = 0;  // the highest: its few blocks start between those of the trace kernels
+        if (!v->setup_stream) cudaDeviceGetStreamPriorityRange(nullptr, &setup_priority);
         if (!v->setup_stream &&
-            (cudaStreamCreateWithFlags(&v->setup_stream, cudaStreamNonBlocking) != cudaSuccess ||
+            (cudaStreamCreateWithPriority(&v->setup_stream, cudaStreamNonBlocking, setup_priority) != cudaSuccess ||
              cudaEventCreateWithFlags(&v->seeded, cudaEventDisableTiming) != cudaSuccess ||
              cudaEventCreateWithFlags(&v->laid_out, cudaEventDisableTiming) != cudaSuccess)) {
             cudaGetLastError();
@@ -4658,7 +4729,8 @@ static void batch_enqueue(LuxBatch *b, cudaStream_t st) {
         deposit_batch_kernel<<<grid, 128, 0, st>>>(b->d_jobs, b->d_begin, n, b->total, b->d_frame);
     }
     if (b->levels > 1 || b->history)
-        batch_merge_prep_kernel<<<grid, 128, 0, st>>>(b->d_jobs, b->d_dom, n, b->d_count, b->levels);
+        batch_merge_prep_kernel<<<dim3(std::max(1, grid / (int)b->levels), b->levels), 128, 0, st>>>(
+            b->d_jobs, b->d_dom, n, b->d_count, b->levels);
     // The children passes over each job's list of the records that pass
     // light on (32-bit record indices: every view's records fit them).
     bool listed = LUX_MERGE_COMPACT && b->levels > 1;
