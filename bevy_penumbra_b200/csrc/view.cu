@@ -3177,6 +3177,7 @@ struct LuxView {
     // while the frame traces; `stage_ready` orders the resolve after it.
     cudaStream_t stage_stream = nullptr;
     cudaEvent_t stage_ready = nullptr;
+    uint32_t *stage_flags = nullptr;  // pinned: the frame's error word
     // Unbatched Split frames: retain, layout and record clearing run on this
     // stream during the closest-hit pass (`seeded` forks it after the seed,
     // `laid_out` joins it before the deposit).
@@ -3419,6 +3420,7 @@ extern "C" lux_status lux_view_destroy(LuxView *v) {
     if (v->stage_stream) cudaStreamSynchronize(v->stage_stream);
     for (void *p : ptrs)
         if (p) cudaFree(p);
+    if (v->stage_flags) cudaFreeHost(v->stage_flags);
     if (v->stage_ready) cudaEventDestroy(v->stage_ready);
     if (v->stage_stream) cudaStreamDestroy(v->stage_stream);
     if (v->setup_stream) cudaStreamSynchronize(v->setup_stream);
@@ -4111,6 +4113,11 @@ static lux_status ensure_stage(LuxView *v, uint32_t receivers, uint32_t points) 
             return lux_fail(v->ctx, LUX_ERR_CUDA, "frame_host: staging stream creation failed");
         }
     }
+    if (!v->stage_flags && cudaMallocHost((void **)&v->stage_flags, sizeof(uint32_t)) != cudaSuccess) {
+        cudaGetLastError();
+        v->stage_flags = nullptr;
+        return lux_fail(v->ctx, LUX_ERR_OUT_OF_MEMORY, "frame_host: staging allocation failed");
+    }
     if (receivers > v->stage_receivers) {
         cudaFree(v->stage_pos);
         cudaFree(v->stage_nrm);
@@ -4168,11 +4175,13 @@ extern "C" lux_status lux_view_frame_host(LuxView *v, const LuxScene *scene, con
     s = lux_view_resolve(v, settings, (const float *)v->stage_ppos, (const float *)v->stage_pnrm, points,
                          (float *)v->stage_out);
     if (s != LUX_OK) return s;
+    // The error word comes back on the frame's stream, beside the image; a copy
+    // of its own after the synchronize cost 13 us more.
+    cudaMemcpyAsync(v->stage_flags, v->dev.error_flags, 4, cudaMemcpyDeviceToHost, st);
     cudaMemcpyAsync(out, v->stage_out, (size_t)points * 16, cudaMemcpyDeviceToHost, st);
     s = lux_cuda_check(v->ctx, (int)cudaStreamSynchronize(st), "frame_host");
     if (s != LUX_OK) return s;
-    uint32_t flags = 0;
-    cudaMemcpy(&flags, v->dev.error_flags, 4, cudaMemcpyDeviceToHost);
+    const uint32_t flags = *v->stage_flags;
     if (flags) return lux_fail(v->ctx, LUX_ERR_CAPACITY, "frame_host: view capacity exceeded (see lux_view_stats)");
     return LUX_OK;
 }
