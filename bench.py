@@ -47,18 +47,18 @@ DRAM_BYTES_PER_SHADOW_RAY = (54.969600e6 + 2.205952e6) / 1237295
 LEARNED_CUTOFF = 1
 LEARNED_WARMUP = 200
 # Kernels of one plain Split frame with world history: clear, 3 seed, the
-# sample-sequence sort (radix-sort histogram, exclusive sum, 8 one-sweep passes
-# over 62-bit keys, ordinal), 3 retain, layout, clear entries, closest, shade,
-# shadow, deposit, the corners and history maps of every level, pack; then a
-# merge per level; 4 more when visibility queries are sorted (histogram, scan
-# init and scan, scatter).
-LAUNCHES_PER_FRAME_FIXED = 26
+# sample-sequence sort (cell pieces and ranks, radix-sort histogram, exclusive
+# sum, 2 one-sweep passes over ranks of at most 16 bits, ordinal), 3 retain,
+# layout, clear entries, closest, shade, shadow, deposit, the corners and history
+# maps of every level, pack; then a merge per level; 3 more when visibility
+# queries are sorted (scan init and scan, scatter).
+LAUNCHES_PER_FRAME_FIXED = 22
 
 
 def launches_per_frame(levels: int, sort_queries: bool, sort_rays: bool = False) -> int:
     """Kernels of one plain frame; sorting the interval rays adds the key
-    pass to the four counting-sort launches."""
-    return LAUNCHES_PER_FRAME_FIXED + levels + (4 if sort_queries else 0) + (5 if sort_rays else 0)
+    and histogram passes to the three counting-sort launches."""
+    return LAUNCHES_PER_FRAME_FIXED + levels + (3 if sort_queries else 0) + (5 if sort_rays else 0)
 
 
 def settings_for_workload(sanitize: bool = True):
