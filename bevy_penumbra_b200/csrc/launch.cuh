@@ -16,9 +16,12 @@ namespace lux {
 // threads: waits for the end of the kernel before it in the stream, whose
 // results are visible from here on, then lets the next kernel start (to wait in
 // its turn; so at most one waiting kernel shares the chip).  What the kernel
-// before it may have written is not read through a pointer parameter that
-// promises constant memory, at an address known before this statement: the
-// compiler may move such a load up.
+// before it may have written is read by ordinary loads: neither by __ldg nor
+// through a const __restrict__ pointer parameter.  Those promise memory that is
+// constant while this kernel lives, and it lives while that kernel still
+// writes, so such a load may be moved up or take a line read too early.  What
+// was complete when the kernel before it began (scene data, the cell
+// directories in a resolve, the corners in a children pass) may be read so.
 __device__ __forceinline__ void after_previous() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -1301,9 +1301,9 @@ __device__ __forceinline__ float4 interpolate(const ViewDevice &V, const FramePa
     float4 corner_value[8];
 #pragma unroll
     for (uint32_t corner = 0; corner < 8u; ++corner)
-        corner_value[corner] = __ldg(V.merged + (ids[corner] == lux::kEmpty
-                                                     ? 0ull
-                                                     : base + (unsigned long long)ids[corner] * dirs + dir));
+        corner_value[corner] = V.merged[ids[corner] == lux::kEmpty
+                                            ? 0ull
+                                            : base + (unsigned long long)ids[corner] * dirs + dir];
 #pragma unroll
     for (uint32_t corner = 0; corner < 8u; ++corner) {
         float ax = (corner & 1u) == 0u ? 1.0f - frac.x : frac.x;
@@ -1355,7 +1355,7 @@ __device__ __forceinline__ void interpolate_children(const ViewDevice &V, const 
         const float4 *rec = V.merged + base + (unsigned long long)ids[corner] * dirs;
         float4 s[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) s[k] = __ldg(rec + offset[k]);
+        for (int k = 0; k < 4; ++k) s[k] = rec[offset[k]];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             if (s[k].w > 0.0f && isfinite(s[k].x) && isfinite(s[k].y) && isfinite(s[k].z) && isfinite(s[k].w)) {
@@ -1934,7 +1934,7 @@ __device__ __forceinline__ void merge_children_quad(const ViewDevice &V, const F
         for (uint32_t corner = 0; corner < 8u; ++corner)
             s[corner] = ids[corner] == lux::kEmpty
                             ? make_float4(0.0f, 0.0f, 0.0f, 0.0f)
-                            : __ldg(V.merged + child_base + (unsigned long long)ids[corner] * child_dirs);
+                            : V.merged[child_base + (unsigned long long)ids[corner] * child_dirs];
         float sx = 0.0f, sy = 0.0f, sz = 0.0f, total = 0.0f, potential = 0.0f;
 #pragma unroll
         for (uint32_t corner = 0; corner < 8u; ++corner) {
@@ -2004,13 +2004,13 @@ __global__ void __launch_bounds__(LUX_MERGE_THREADS, LUX_MERGE_MIN_BLOCKS)
         const uint32_t i = thread >> 2;
         if ((i & ~7u) >= n) return;  // whole warps
         const bool valid = i < n;
-        const uint32_t record = valid ? __ldg(V.pass_list + base + i) : 0u;
+        const uint32_t record = valid ? V.pass_list[base + i] : 0u;
         merge_children_quad(V, F, level, base, dirs, record, valid);
         return;
     }
     for (uint32_t i = thread; i < n; i += threads) {
         uint32_t cell, d;
-        record_cell(__ldg(V.pass_list + base + i), dirs, cell, d);
+        record_cell(V.pass_list[base + i], dirs, cell, d);
         merge_children_record(V, F, level, base, dirs, cell, d);
     }
 }
@@ -2122,7 +2122,7 @@ __device__ __forceinline__ void diffuse_at_lod(const ViewDevice &V, const FrameP
         if (cell[corner] == lux::kEmpty) continue;
         float4 texels[4];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) texels[c] = __ldg(V.tables + (size_t)cell[corner] * 36 + texel[c]);
+        for (int c = 0; c < 4; ++c) texels[c] = V.tables[(size_t)cell[corner] * 36 + texel[c]];
         float px = 0.0f, py = 0.0f, pz = 0.0f, pobs = 0.0f;
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
@@ -2844,7 +2844,7 @@ __global__ void __launch_bounds__(LUX_MERGE_THREADS, LUX_MERGE_MIN_BLOCKS)
         const uint32_t dirs = J.F.dirs[level];
         const unsigned long long base = J.V.level_base[level];
         uint32_t cell, d;
-        record_cell(__ldg(J.V.pass_list + base + i), dirs, cell, d);
+        record_cell(J.V.pass_list[base + i], dirs, cell, d);
         merge_children_record(J.V, J.F, level, base, dirs, cell, d);
     });
 }
