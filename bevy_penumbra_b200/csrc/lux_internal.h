@@ -74,7 +74,7 @@ struct TraceScratch {
     float4 *queue_d;        // per (ray, sample): query direction, coherence sort key bits
     uint8_t *queue_result;  // per (ray, sample): 0 visible, 1 blocked, 2 unsupported
     uint32_t *queue_count;
-    uint32_t *work_counter; // [2] persistent-warp ray fetch: closest, shadow
+    uint32_t *work_counter; // [3] persistent-warp ray fetch: closest, shadow; caller rays: some are far
 };
 
 struct LuxContext {
@@ -160,5 +160,10 @@ LuxContext *lux_cache_context(const LuxCache *cache);
 lux_status lux_cache_query_device_count(LuxCache *cache, const LuxCacheSample *queries, const uint32_t *count,
                                         uint32_t max_count, float *out);
 
+// The far ones of caller rays that a closest-hit pass left (ray_h errors),
+// their work added to the three counters.
+void lux_launch_far_rays(LuxContext *ctx, const LuxScene *scene, const TraceScratch &T, const LuxRay *rays,
+                         uint32_t count, unsigned long long *nodes, unsigned long long *triangles,
+                         unsigned long long *instances);
 lux_status lux_fail(LuxContext *ctx, lux_status status, const std::string &message);
 lux_status lux_cuda_check(LuxContext *ctx, int err, const char *what);

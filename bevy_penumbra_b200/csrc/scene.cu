@@ -15,6 +15,7 @@
 #include <unordered_map>
 #include <vector>
 
+#include "launch.cuh"
 #include "lux_internal.h"
 #include "lux_math.cuh"
 #include "traverse.cuh"
@@ -187,6 +188,33 @@ struct Collapser {
     }
 };
 
+__device__ __forceinline__ LuxHit ray_hit(const lux::Hit &h, uint32_t visited) {
+    LuxHit out;
+    out.distance = h.t;
+    out.triangle = h.tri;
+    out.instance = h.inst;
+    out.errors = h.errors;
+    out.barycentric[0] = (1.0f - h.b1) - h.b2;
+    out.barycentric[1] = h.b1;
+    out.barycentric[2] = h.b2;
+    out.visited = visited;
+    return out;
+}
+
+// A ray that starts far outside the scene: not inlined, and the ray and its hit
+// in memory, or the walk beside it would lose registers (3% of a call).
+template <bool kAnyHit>
+__device__ __noinline__ lux::TraceCounters trace_far_ray(const SceneView &S, const LuxRay *ray, LuxHit *hit) {
+    const LuxRay r = *ray;
+    lux::Hit h;
+    lux::TraceCounters cn{0, 0, 0};
+    lux::trace<kAnyHit, lux::kStack, lux::FarSlabRay>(S, lux::f3{r.origin[0], r.origin[1], r.origin[2]},
+                                                     lux::f3{r.direction[0], r.direction[1], r.direction[2]},
+                                                     kAnyHit ? 0.0f : r.tmin, r.limit, h, cn);
+    *hit = ray_hit(h, cn.nodes);
+    return cn;
+}
+
 // 128 threads per block; every lane of a warp walks together (whole-warp
 // leaf tests), lanes past `count` without a query.  One kernel per query kind
 // and tree, so each is compiled for its own walk's registers.
@@ -206,22 +234,14 @@ __global__ void __launch_bounds__(128, kFlat ? (kAnyHit ? 8 : 7) : 5)
     lux::LeafScratch *L = &scratch[threadIdx.x >> 5];
     const float tmin = kAnyHit ? 0.0f : r.tmin;
     if (kFlat) {
-        lux::trace_warp_flat<kAnyHit>(S, active, o, d, tmin, r.limit, h, cn, L);
+        lux::trace_warp_flat<kAnyHit, true>(S, active, o, d, tmin, r.limit, h, cn, L);
     } else {
-        lux::trace_warp<kAnyHit>(S, active, o, d, tmin, r.limit, h, cn, L);
+        lux::trace_warp<kAnyHit, lux::kStack, true>(S, active, o, d, tmin, r.limit, h, cn, L);
     }
-    if (active) {
-        LuxHit out;
-        out.distance = h.t;
-        out.triangle = h.tri;
-        out.instance = h.inst;
-        out.errors = h.errors;
-        out.barycentric[0] = (1.0f - h.b1) - h.b2;
-        out.barycentric[1] = h.b1;
-        out.barycentric[2] = h.b2;
-        out.visited = cn.nodes;
-        hits[i] = out;
-    }
+    if (h.errors == lux::kFarRay)
+        cn = trace_far_ray<kAnyHit>(S, rays + i, hits + i);
+    else if (active)
+        hits[i] = ray_hit(h, cn.nodes);
     if (counters) {
         unsigned long long n = cn.nodes, t = cn.triangles, in = cn.instances;
         for (int off = 16; off > 0; off >>= 1) {
@@ -335,6 +355,34 @@ __global__ void __launch_bounds__(1024) refit_kernel(uint4 *__restrict__ sw, uin
         n.hi_x[c] = mx[0];
         n.hi_y[c] = mx[1];
         n.hi_z[c] = mx[2];
+    }
+}
+
+// The caller rays of a trace scratch that start far outside the scene (noted in
+// work_counter[2], marked in ray_h), a thread each.  A kernel of its own, nearly
+// always empty (4099 rays 118.5 -> 120.5 us; as a function called from the walk's
+// kernel 400,000 rays took 1.8% more), and in this file: in the one of the
+// frame's kernels the second walk made the compiler spill more there.
+__global__ void __launch_bounds__(128) far_rays_kernel(const __grid_constant__ SceneView S, TraceScratch T,
+                                                       const LuxRay *__restrict__ rays, uint32_t count,
+                                                       unsigned long long *nodes, unsigned long long *triangles,
+                                                       unsigned long long *instances) {
+    lux::after_previous();
+    if (T.work_counter[2] == 0u) return;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
+        if (T.ray_h[i].z != lux::kFarRay) continue;
+        const LuxRay r = rays[i];
+        lux::Hit h;
+        lux::TraceCounters cn{0, 0, 0};
+        lux::trace<false, lux::kStack, lux::FarSlabRay>(S, lux::f3{r.origin[0], r.origin[1], r.origin[2]},
+                                                        lux::f3{r.direction[0], r.direction[1], r.direction[2]},
+                                                        r.tmin, r.limit, h, cn);
+        T.ray_o[i].w = h.t;
+        T.ray_d[i].w = h.b1;
+        T.ray_h[i] = make_uint4(h.tri, h.inst, h.errors, lux::as_uint(h.b2));
+        atomicAdd(nodes, (unsigned long long)cn.nodes);
+        atomicAdd(triangles, (unsigned long long)cn.triangles);
+        atomicAdd(instances, (unsigned long long)cn.instances);
     }
 }
 
@@ -965,4 +1013,11 @@ extern "C" lux_status lux_trace_rays(LuxContext *ctx, const LuxScene *scene, con
                                      uint32_t any_hit, LuxHit *hits) {
     if (!ctx || !scene || (count && (!rays || !hits))) return LUX_ERR_INVALID_ARGUMENT;
     return lux_launch_trace_rays(ctx, scene, rays, count, any_hit, hits, nullptr);
+}
+
+void lux_launch_far_rays(LuxContext *ctx, const LuxScene *scene, const TraceScratch &T, const LuxRay *rays,
+                         uint32_t count, unsigned long long *nodes, unsigned long long *triangles,
+                         unsigned long long *instances) {
+    const uint32_t blocks = std::min<uint32_t>((count + 127u) / 128u, (uint32_t)ctx->sm_count);
+    lux::launch(far_rays_kernel, blocks, 128, 0, ctx->stream, scene->view, T, rays, count, nodes, triangles, instances);
 }

@@ -125,15 +125,16 @@ __device__ __forceinline__ void slab_special(float o, float d, float pad, bool t
     }
 }
 
-// pad: kSlabPad x M.
+// pad: kSlabPad x M; with kEven the whole padding, the same on every axis.
+template <bool kEven = false>
 __device__ __forceinline__ SlabRay slab_ray(f3 o, f3 d, float pad) {
     SlabRay r;
     r.ix = rcp_approx(d.x);
     r.iy = rcp_approx(d.y);
     r.iz = rcp_approx(d.z);
-    const float cx = o.x * r.ix, ex = __fmaf_rn(fabsf(o.x), kSlabPad, pad) * fabsf(r.ix);
-    const float cy = o.y * r.iy, ey = __fmaf_rn(fabsf(o.y), kSlabPad, pad) * fabsf(r.iy);
-    const float cz = o.z * r.iz, ez = __fmaf_rn(fabsf(o.z), kSlabPad, pad) * fabsf(r.iz);
+    const float cx = o.x * r.ix, ex = (kEven ? pad : __fmaf_rn(fabsf(o.x), kSlabPad, pad)) * fabsf(r.ix);
+    const float cy = o.y * r.iy, ey = (kEven ? pad : __fmaf_rn(fabsf(o.y), kSlabPad, pad)) * fabsf(r.iy);
+    const float cz = o.z * r.iz, ez = (kEven ? pad : __fmaf_rn(fabsf(o.z), kSlabPad, pad)) * fabsf(r.iz);
     r.nx = -cx - ex;
     r.fx = ex - cx;
     r.ny = -cy - ey;
@@ -184,6 +185,54 @@ __device__ __forceinline__ uint32_t node_test(const Bvh4Node *__restrict__ nodes
     }
     return mask;
 }
+
+// Slab tests of rays from far outside the scene: t = (plane - o) * inv with
+// the correctly rounded reciprocal carries under 2 ulp, and the interval grows
+// by 7.2e-7 relative on both ends.  SlabRay's padding is a part of the origin's
+// magnitude on every axis; where that is many times the boxes, a walk meets so
+// many of them that it runs into its step budget (2e5 units from a scene of 2
+// units and 131,072 triangles: 790 nodes per ray and 16% of the rays abandoned;
+// so 180 and none).  A zero direction component gives an infinite reciprocal:
+// planes on either side of the origin give -inf/+inf (no constraint), a box
+// wholly on one side misses, and a plane through the origin gives NaN, which
+// fmaxf/fminf ignore.
+struct FarSlabRay {
+    float ox, oy, oz;
+    float ix, iy, iz;
+};
+__device__ __forceinline__ void make_slab(FarSlabRay &r, f3 o, f3 d, float) {
+    r = FarSlabRay{o.x, o.y, o.z, __frcp_rn(d.x), __frcp_rn(d.y), __frcp_rn(d.z)};
+}
+__device__ __forceinline__ void make_slab(SlabRay &r, f3 o, f3 d, float pad) { r = slab_ray(o, d, pad); }
+__device__ __forceinline__ uint32_t node_test(const Bvh4Node *__restrict__ nodes, uint32_t index, const FarSlabRay &r,
+                                              float limit, float tmin, float entry[4], uint32_t child[4]) {
+    const Bvh4Node &n = nodes[index];
+    const bool sx = as_uint(r.ix) >> 31, sy = as_uint(r.iy) >> 31, sz = as_uint(r.iz) >> 31;
+    uint32_t mask = 0;
+    for (int i = 0; i < 4; ++i) {
+        child[i] = n.child[i];
+        const float lx = (n.lo_x[i] - r.ox) * r.ix, hx = (n.hi_x[i] - r.ox) * r.ix;
+        const float ly = (n.lo_y[i] - r.oy) * r.iy, hy = (n.hi_y[i] - r.oy) * r.iy;
+        const float lz = (n.lo_z[i] - r.oz) * r.iz, hz = (n.hi_z[i] - r.oz) * r.iz;
+        float near_t = fmaxf(fmaxf(sx ? hx : lx, sy ? hy : ly), fmaxf(sz ? hz : lz, 0.0f));
+        float far_t = fminf(fminf(sx ? lx : hx, sy ? ly : hy), sz ? lz : hz);
+        near_t = near_t - fabsf(near_t) * 7.2e-7f;
+        far_t = far_t + fabsf(far_t) * 7.2e-7f;
+        // An empty slot's inverted infinities come out NaN: every comparison fails.
+        const bool hit = near_t <= far_t && near_t <= limit && far_t >= tmin;
+        entry[i] = hit ? near_t : 0.0f;
+        mask |= hit ? (1u << i) : 0u;
+    }
+    return mask;
+}
+
+// Whether a caller's ray starts so far outside (more than 8 times the scene
+// box's largest coordinate magnitude M) that its padding would be large against
+// the triangles: it is traced by itself then, by FarSlabRay.
+constexpr float kFarOrigin = 8.0f;
+__device__ __forceinline__ float largest_component(f3 v) { return max3(fabsf(v.x), fabsf(v.y), fabsf(v.z)); }
+constexpr uint32_t kFarSteps = 0xffffffffu;  // `steps` of such a ray's walker
+constexpr uint32_t kFarRay = 0x80000000u;    // and the errors it returns
 
 struct TriRay {
     uint32_t kx, ky, kz;
@@ -489,13 +538,13 @@ __device__ __forceinline__ bool leaf_pass(const SceneView &S, LeafScratch *L, ui
 // (per TLAS walk and per instance walk), 2 / 1 when the stack is exhausted in
 // the TLAS / a BLAS, after which the walk continues over every instance / every
 // triangle of the instance in order (shaders/traversal.slang:498-517, :729-745).
-template <bool kAnyHit, int kDepth = kStack>
+template <bool kAnyHit, int kDepth = kStack, typename Slab = SlabRay>
 struct Walker {
     Hit hit;
     f3 o, d, lo, ld;  // world ray; the current instance's local ray
     float tmin;       // at least 0
     float pad;        // kSlabPad x the largest coordinate magnitude of the TLAS root box
-    SlabRay r;        // slab constants of the current space's ray
+    Slab r;           // slab constants of the current space's ray
     uint32_t inst, inst_flags, inst_first;
     int blas_base;        // stack depth at instance entry; -1 = TLAS space
     uint32_t tlas_next;   // TLAS fallback: next instance to scan in order
@@ -508,7 +557,9 @@ struct Walker {
 
     // Returns false when the query is already complete (no instances, the ray
     // misses the TLAS root box: traceRayTracked's early exits; or a ray that
-    // is not finite, which no triangle test accepts).
+    // is not finite, which no triangle test accepts).  kLeaveFar: so do far
+    // rays, with `steps` kFarSteps.
+    template <bool kLeaveFar = false>
     __device__ __forceinline__ bool start(const SceneView &S, f3 origin, f3 direction, float t_min, float limit) {
         hit.t = limit;
         hit.tri = kEmpty;
@@ -524,11 +575,16 @@ struct Walker {
         uint4 ra = __ldg(S.scene_words + 1), rb = __ldg(S.scene_words + 2);
         const f3 rl{as_float(ra.x), as_float(ra.y), as_float(ra.z)}, rh{as_float(rb.x), as_float(rb.y), as_float(rb.z)};
         if (!box_interval(origin, direction, rl.x, rl.y, rl.z, rh.x, rh.y, rh.z, limit, re, rx)) return false;
-        pad = box_magnitude(rl, rh) * kSlabPad;
+        const float magnitude = box_magnitude(rl, rh);
+        if (kLeaveFar && largest_component(origin) > kFarOrigin * magnitude) {
+            steps = kFarSteps;
+            return false;
+        }
+        pad = magnitude * kSlabPad;
         o = origin;
         d = direction;
         tmin = fmaxf(t_min, 0.0f);
-        r = slab_ray(o, d, pad);
+        make_slab(r, o, d, pad);
         lo = o;
         ld = d;
         inst = kEmpty;
@@ -633,7 +689,7 @@ struct Walker {
         cn.instances++;
         if (!isfinite(((fabsf(lo.x) + fabsf(lo.y)) + fabsf(lo.z)) + ((fabsf(ld.x) + fabsf(ld.y)) + fabsf(ld.z))))
             return;  // no triangle test accepts such a ray
-        r = slab_ray(lo, ld, I.extent * kSlabPad);
+        make_slab(r, lo, ld, I.extent * kSlabPad);
         inst = first;
         inst_flags = I.flags;
         inst_first = I.first;
@@ -722,7 +778,7 @@ struct Walker {
                 }
                 blas_base = -1;
                 steps = tlas_steps;
-                r = slab_ray(o, d, pad);
+                make_slab(r, o, d, pad);
                 inst = kEmpty;
                 continue;
             }
@@ -773,9 +829,9 @@ struct Walker {
 // Closest hit (kAnyHit = false) or any hit of one ray.  kDepth is the stack
 // depth: a shallower stack uses less local memory per thread, and a walk that
 // overflows it continues with the reference's ordered scan (same answers).
-template <bool kAnyHit, int kDepth = kStack>
+template <bool kAnyHit, int kDepth = kStack, typename Slab = SlabRay>
 __device__ void trace(const SceneView &S, f3 o, f3 d, float tmin, float limit, Hit &hit, TraceCounters &cn) {
-    Walker<kAnyHit, kDepth> w;
+    Walker<kAnyHit, kDepth, Slab> w;
     uint2 stack[kDepth];
     if (w.start(S, o, d, tmin, limit))
         while (!w.step(S, stack, cn)) {
@@ -791,7 +847,15 @@ __device__ void trace(const SceneView &S, f3 o, f3 d, float tmin, float limit, H
 // (a transform and two sets of slab constants, run by a few lanes of a warp at
 // a time), the rounds that end at an instance, and the registers of the second
 // ray.  Hits are the same: the triangles are tested in the instance's local
-// space from the same local ray, and the copies' boxes are padded (scene.cu).
+// space from the same local ray, the copies' boxes are padded (scene.cu), and
+// so is the ray, by kFlatPad (max|o| + M) on every axis, since a rotated
+// instance's local ray mixes the axes and rounds by the largest.  With u =
+// 2^-24 and sum_j |M_ij| sum_k |R_jk| <= 4 (flat_conditioned): the local
+// origin rounds by 3.5 u, the direction by 3 u over the distance, the matrix
+// itself by u, the triangle test's differences by u and its shear by 2 u, each
+// at most four times that in world space, 42 u of max|o|; the hit distance
+// takes 4 u and the slab constants 6 u: 52 u, and less of M.  (With |o| of the
+// axis alone, rays along an axis lost hits from 1,000 scene sizes on.)
 // Measured at the 1280x720 frame (262,144 triangles, 1.97 M interval rays, 8.8 M
 // visibility queries): closest hits 1.73 -> 1.20 ms, visibility 3.53 -> 2.59
 // ms; 1920x1080 and 1,048,576 triangles: whole frame 20.7 -> 15.7 ms.
@@ -802,6 +866,8 @@ __device__ void trace(const SceneView &S, f3 o, f3 d, float tmin, float limit, H
 // in all; a query that gets there starts over with the two-level walk's
 // accounting (careful_step), whose state lives behind the stack in local
 // memory so that the common walk keeps no register for it.
+constexpr float kFlatPad = 3.814697265625e-6f;  // 64 u
+
 template <bool kAnyHit>
 struct FlatWalker {
     // A pending child: its payload, and for closest hits its entry distance.
@@ -830,6 +896,7 @@ struct FlatWalker {
     uint32_t cur;
     bool have;
 
+    template <bool kLeaveFar = false>
     __device__ __forceinline__ bool start(const SceneView &S, Entry *stack, f3 origin, f3 direction, float t_min,
                                           float limit) {
         if (!(finite3(origin) && finite3(direction))) return false;
@@ -837,10 +904,15 @@ struct FlatWalker {
         uint4 ra = __ldg(S.scene_words + 1), rb = __ldg(S.scene_words + 2);
         const f3 rl{as_float(ra.x), as_float(ra.y), as_float(ra.z)}, rh{as_float(rb.x), as_float(rb.y), as_float(rb.z)};
         if (!box_interval(origin, direction, rl.x, rl.y, rl.z, rh.x, rh.y, rh.z, limit, re, rx)) return false;
+        const float magnitude = box_magnitude(rl, rh), out = largest_component(origin);
+        if (kLeaveFar && out > kFarOrigin * magnitude) {
+            steps = kFarSteps;
+            return false;
+        }
         o = origin;
         d = direction;
         tmin = fmaxf(t_min, 0.0f);
-        r = slab_ray(o, d, box_magnitude(rl, rh) * kSlabPad);
+        r = slab_ray<true>(o, d, (out + magnitude) * kFlatPad);
         if (!kAnyHit) stack[kLimit].set(as_uint(limit), 0u);
         sp = 0;
         cur = S.tlas_root;
@@ -995,17 +1067,22 @@ struct FlatWalker {
 // trace() for a whole warp: every lane of the warp calls it (active: the lane
 // has a query), and the BLAS leaves reached in each round are tested by the
 // whole warp (leaf_pass).  A lane without a query returns no hit.
-template <bool kAnyHit, int kDepth = kStack>
+// kFar: the rays are a caller's and may start far outside the scene; one that
+// does returns no hit and errors = kFarRay, and is traced by itself (trace with
+// FarSlabRay) where that costs the walk beside it least.
+template <bool kAnyHit, int kDepth = kStack, bool kFar = false>
 __device__ __forceinline__ void trace_warp(const SceneView &S, bool active, f3 o, f3 d, float tmin, float limit,
                                            Hit &hit, TraceCounters &cn, LeafScratch *L) {
     Walker<kAnyHit, kDepth> w;
     w.hit = Hit{limit, kEmpty, kEmpty, 0u, 0.0f, 0.0f};
+    w.steps = 0;
     uint2 stack[kDepth];
-    bool alive = active && w.start(S, o, d, tmin, limit);
+    bool alive = active && w.template start<kFar>(S, o, d, tmin, limit);
     while (__any_sync(0xffffffffu, alive)) {
         const bool complete = w.step_warp(S, stack, cn, L, alive);
         alive = alive && !complete;
     }
+    if (kFar && w.steps == kFarSteps) w.hit.errors = kFarRay;
     hit = w.hit;
     if (!kAnyHit) hit_barycentrics(S, o, d, hit);
 }
@@ -1013,19 +1090,22 @@ __device__ __forceinline__ void trace_warp(const SceneView &S, bool active, f3 o
 // trace_warp over the flattened tree.  (The two-level walk is in kernels of its
 // own: the flattened walk loses its registers to a second walk in the same
 // loop, even one that is hardly ever called: closest hits 1.51 ms against 1.26.)
-template <bool kAnyHit>
+template <bool kAnyHit, bool kFar = false>
 __device__ __forceinline__ void trace_warp_flat(const SceneView &S, bool active, f3 o, f3 d, float tmin, float limit,
                                                 Hit &hit, TraceCounters &cn, LeafScratch *L) {
     FlatWalker<kAnyHit> w;
     w.hit = Hit{limit, kEmpty, kEmpty, 0u, 0.0f, 0.0f};
     w.steps = 0;
     typename FlatWalker<kAnyHit>::Entry stack[FlatWalker<kAnyHit>::kEntries];
-    bool alive = active && w.start(S, stack, o, d, tmin, limit);
+    bool alive = active && w.template start<kFar>(S, stack, o, d, tmin, limit);
     while (__any_sync(0xffffffffu, alive)) {
         const bool complete = w.step_warp(S, stack, cn, L, alive);
         alive = alive && !complete;
     }
-    w.finish(stack);
+    if (kFar && w.steps == kFarSteps)
+        w.hit.errors = kFarRay;
+    else
+        w.finish(stack);
     hit = w.hit;
     if (!kAnyHit) hit_barycentrics(S, o, d, hit);
 }

@@ -687,17 +687,19 @@ __global__ void __launch_bounds__(128, LUX_REFILL_MIN_BLOCKS) closest_split_refi
 
 // The closest hits of a warp's rays, stored for shading (every lane calls it;
 // active: the lane has ray `ray`).  kFlat: over the flattened tree, which takes
-// no stack depth.
-template <int kDepth, bool kFlat>
+// no stack depth.  kFar: as trace_warp; that there are far rays is noted for
+// lux_launch_far_rays.
+template <int kDepth, bool kFlat, bool kFar = false>
 __device__ __forceinline__ void closest_ray_warp(const ViewDevice &V, const SceneView &S, uint32_t ray, bool active,
                                                  f3 origin, f3 dir, float tmin, float limit, lux::TraceCounters &cn,
                                                  lux::LeafScratch *L) {
     lux::Hit hit;
     if (kFlat)
-        lux::trace_warp_flat<false>(S, active, origin, dir, tmin, limit, hit, cn, L);
+        lux::trace_warp_flat<false, kFar>(S, active, origin, dir, tmin, limit, hit, cn, L);
     else
-        lux::trace_warp<false, kDepth>(S, active, origin, dir, tmin, limit, hit, cn, L);
+        lux::trace_warp<false, kDepth, kFar>(S, active, origin, dir, tmin, limit, hit, cn, L);
     if (active) store_ray(V, ray, origin, dir, hit);
+    if (kFar && hit.errors == lux::kFarRay) V.ts.work_counter[2] = 1u;
 }
 
 // Split interval rays (traceTransport, shaders/split.slang:1122-1163) of a
@@ -4350,6 +4352,7 @@ __global__ void scratch_clear_kernel(ViewDevice V) {
         *V.ts.queue_count = 0;
         V.ts.work_counter[0] = 0;
         V.ts.work_counter[1] = 0;
+        V.ts.work_counter[2] = 0;
     }
     if (blockIdx.x == 0 && threadIdx.x < 16) V.stats[threadIdx.x] = 0;
 }
@@ -4369,8 +4372,9 @@ __global__ void __launch_bounds__(128, kFlat ? LUX_FLAT_CLOSEST_MIN_BLOCKS : LUX
             r = rays[i];
             ++traced;
         }
-        closest_ray_warp<lux::kStack, kFlat>(V, S, i, active, f3{r.origin[0], r.origin[1], r.origin[2]},
-                                             f3{r.direction[0], r.direction[1], r.direction[2]}, r.tmin, r.limit, cn, L);
+        closest_ray_warp<lux::kStack, kFlat, true>(V, S, i, active, f3{r.origin[0], r.origin[1], r.origin[2]},
+                                                   f3{r.direction[0], r.direction[1], r.direction[2]}, r.tmin, r.limit,
+                                                   cn, L);
     });
     unsigned long long st[7] = {0, 0, 0, 0, 0, 0, 0};
     st[kStatInterval] = traced;
@@ -4415,6 +4419,8 @@ lux_status launch_interval_radiance(LuxContext *ctx, const LuxScene *scene, cons
         const bool flat = scene->view.flat_nodes != nullptr;
         lux::launch((flat ? closest_rays_kernel<true> : closest_rays_kernel<false>),
                     trace_blocks(ctx, 16u, 32u, count), 128, 0, st, V, scene->view, rays, count);
+        lux_launch_far_rays(ctx, scene, V.ts, rays, count, V.stats + kStatNodes, V.stats + kStatTris,
+                            V.stats + kStatInst);
         launch_shade(ctx, V, F, scene, count, false, st);
         lux::launch((flat ? shadow_kernel<64, true> : shadow_kernel<64, false>),
                     trace_blocks(ctx, 16u, 32u, most_queries(F, scene, count)), 128, 0, st, V, F, scene->view, 32u);
