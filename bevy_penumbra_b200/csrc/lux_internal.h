@@ -122,6 +122,13 @@ inline size_t carved_scratch_bytes(uint32_t rays) {
     return 4 * up(r * 16) + up(q * 4) + 3 * up(q * 16) + up(q) + 3 * up(16) + up(128);
 }
 
+// An instance's BLAS root box (local) and how many nodes its copy in the
+// flattened tree has.
+struct FlatBox {
+    float center[3], half[3];
+    uint32_t nodes;
+};
+
 struct LuxScene {
     LuxContext *ctx = nullptr;
     SceneView view{};
@@ -146,6 +153,7 @@ struct LuxScene {
     Bvh4Node *d_flat_nodes = nullptr;
     uint2 *d_flat_leaves = nullptr;
     uint32_t flat_count = 0, flat_tlas = 0;     // flat nodes; of them the TLAS's
+    std::vector<FlatBox> flat_boxes;            // per instance (empty without a flattened tree)
 };
 
 // local_from_world of a 3x4 world_from_local (row-major), inverted in f64

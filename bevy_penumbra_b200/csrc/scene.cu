@@ -481,6 +481,7 @@ struct HostScene {
     // Flattened tree (flat_count 0: none): per instance (first flat node,
     // first leaf record, first BLAS node, BLAS root node).
     std::vector<uint4> flat_inst;
+    std::vector<FlatBox> flat_boxes;
     uint32_t flat_count = 0, flat_leaves = 0, flat_tlas = 0;
 };
 
@@ -522,6 +523,33 @@ static bool flat_conditioned(const float *lfw, const float *wfl) {
         worst = std::max(worst, sum);
     }
     return std::isfinite(worst);
+}
+
+// Whether the flattened walk's padding, 2^-17 of the scene's coordinate
+// magnitude and more for rays from outside, stays small against the instances:
+// world space does not resolve a detailed mesh that is tiny against its
+// distance from the origin, and a walk would meet so many of its boxes that it
+// runs into the step budget (131,072 triangles in 2 units at 1e5: every ray
+// abandoned).  An instance of more than kFlatCoarse nodes needs 2^-10 of the
+// magnitude, else the scene keeps the two-level walk, whose tests are local.
+// wfl: world_from_local rows, `stride` floats apart.
+constexpr uint32_t kFlatCoarse = 64;
+static bool flat_placed(const std::vector<FlatBox> &boxes, const float *wfl, size_t stride) {
+    float magnitude = 0.0f, least = INFINITY;
+    for (size_t i = 0; i < boxes.size(); ++i) {
+        const FlatBox &b = boxes[i];
+        float extent = 0.0f;
+        for (int r = 0; r < 3; ++r) {
+            const float *m = wfl + i * stride + 4 * r;
+            const float c = m[0] * b.center[0] + m[1] * b.center[1] + m[2] * b.center[2] + m[3];
+            const float h = std::fabs(m[0]) * b.half[0] + std::fabs(m[1]) * b.half[1] + std::fabs(m[2]) * b.half[2];
+            if (!std::isfinite(c) || !std::isfinite(h)) return false;
+            magnitude = std::max(magnitude, std::fabs(c) + h);
+            extent = std::max(extent, 2.0f * h);
+        }
+        if (b.nodes > kFlatCoarse) least = std::min(least, extent);
+    }
+    return least >= magnitude * 0.0009765625f;
 }
 
 static lux_status prepare_scene(const uint32_t *sw, size_t sn, const uint32_t *gw, size_t gn, const LuxLight *lights,
@@ -603,6 +631,12 @@ static lux_status prepare_scene(const uint32_t *sw, size_t sn, const uint32_t *g
         const BinNode &box = bin[inst[i].root];
         for (int r = 0; r < 3; ++r)
             inst[i].extent = std::max({inst[i].extent, std::fabs(box.mn[r]), std::fabs(box.mx[r])});
+        FlatBox fb{};
+        for (int r = 0; r < 3; ++r) {
+            fb.center[r] = 0.5f * (box.mn[r] + box.mx[r]);
+            fb.half[r] = 0.5f * (box.mx[r] - box.mn[r]);
+        }
+        H.flat_boxes.push_back(fb);
     }
     // World box of every instance: the eight corners of its BLAS root box
     // through world_from_local (instance rows 3-5) in f64, padded by 2^-17
@@ -702,6 +736,7 @@ static lux_status prepare_scene(const uint32_t *sw, size_t sn, const uint32_t *g
         }
         const Blas &b = it->second;
         inst[i].root = b.root;
+        H.flat_boxes[i].nodes = b.nodes;
         if (!flat_ok) continue;
         const uint32_t *w = sw + 4 * (size_t)(inst_base + 9 * i);
         float lfw[12], wfl[12];
@@ -713,6 +748,11 @@ static lux_status prepare_scene(const uint32_t *sw, size_t sn, const uint32_t *g
         flat_leaves += b.leaves;
         flat_ok = flat_nodes <= kFlatMaxNodes && flat_leaves <= kLeafFirstMask &&
                   3u * (tlas_depth + b.depth) <= (uint32_t)lux::kFlatStack && flat_conditioned(lfw, wfl);
+    }
+    if (flat_ok) {  // world_from_local rows as floats, 36 words per instance
+        std::vector<float> words(36 * (size_t)inst_count);
+        std::memcpy(words.data(), sw + 4 * (size_t)inst_base, words.size() * 4);
+        flat_ok = flat_placed(H.flat_boxes, words.data() + 12, 36);
     }
     if (flat_ok) {
         H.flat_count = (uint32_t)flat_nodes;
@@ -858,6 +898,7 @@ extern "C" lux_status lux_scene_upload(LuxContext *ctx, const uint32_t *sw, size
                        cudaMemcpyHostToDevice) == cudaSuccess) {
             S->flat_count = H.flat_count;
             S->flat_tlas = H.flat_tlas;
+            S->flat_boxes = H.flat_boxes;
         } else {
             cudaGetLastError();
             flat_free(S);
@@ -945,6 +986,7 @@ extern "C" lux_status lux_scene_refit(LuxScene *S, const float *wfl, uint32_t co
             for (int c = 0; c < 4; ++c) inst[i].row[r][c] = lfw[4 * r + c];
         if (S->flat_count) conditioned = conditioned && flat_conditioned(lfw, m);
     }
+    if (S->flat_count) conditioned = conditioned && flat_placed(S->flat_boxes, wfl, 12);
     cudaStream_t st = ctx->stream;
     cudaSetDevice(ctx->device);
     uint4 *sw = (uint4 *)S->d_sw;

@@ -1,6 +1,7 @@
 """Rays from far outside a scene: closest hits are the smallest (distance,
 instance, triangle) over all triangles, bit for bit, and any hit agrees, also
-where the rounding of the world coordinates is larger than the triangles."""
+where the rounding of the world coordinates is larger than the triangles; and
+scenes far from the origin."""
 import ctypes as C
 
 import numpy as np
@@ -88,3 +89,27 @@ def check(packed, rays):
 def test_rays_from_outside(distance):
     packed, m = grid_scene()
     check(packed, rays_to(m, distance, 700, int(distance)))
+
+
+@pytest.mark.parametrize("place", [60.0, 300.0, 1e4, 1e5])
+def test_scene_far_from_the_origin(place):
+    packed, m = grid_scene((place, -0.5 * place, 0.25 * place))
+    check(packed, rays_to(m, 3.0, 400, int(place)))
+
+
+def test_refit_far_from_the_origin_and_back():
+    """A refit that takes a detailed scene far from the origin leaves the
+    flattened tree, one that brings it back returns to it."""
+    near, m0 = grid_scene()
+    far, m1 = grid_scene((1e5, 0.0, -2e4))
+    ctx = bp.LuxContext()
+    scene = bp.GpuScene(ctx, near)
+    for packed, m in ((far, m1), (near, m0)):
+        scene.refit(m[None])
+        rays = rays_to(m, 3.0, 300, 8)
+        d_rays, d_hits = to_device(rays), empty_device(len(rays) * bp.HIT_DTYPE.itemsize)
+        bp.trace_rays(ctx, scene, d_rays.data_ptr(), len(rays), d_hits.data_ptr())
+        got, want = from_device(d_hits, bp.HIT_DTYPE, (len(rays),)), brute(packed, rays)
+        np.testing.assert_array_equal(got["errors"], 0)
+        np.testing.assert_array_equal(got["triangle"], want["triangle"])
+        np.testing.assert_array_equal(got["distance"].view(np.uint32), want["distance"].view(np.uint32))
