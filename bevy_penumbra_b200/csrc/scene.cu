@@ -509,20 +509,30 @@ static uint32_t tree_depth(const std::vector<Bvh4Node> &nodes, uint32_t root) {
 // same few units of the world coordinates when max_i sum_j |M_ij| sum_k
 // |R_jk| is small (at most 3 for rotations with any scale per axis), which the
 // slab and box padding covers; sheared, ill-conditioned poses are left to the
-// two-level walk.
+// two-level walk.  So are words whose local_from_world rows are not the inverse
+// of the world_from_local rows: the walk follows the former, the copies' boxes
+// the latter.  The inverse in double precision, rounded, leaves rows of M R - I
+// within 4 x 2^-24; 12 x 2^-24 of the ray's padding and 2^-19 of the boxes' (the
+// translation) are kept for others.
 static bool flat_conditioned(const float *lfw, const float *wfl) {
-    double worst = 0.0;
     for (int i = 0; i < 3; ++i) {
-        double sum = 0.0;
+        double sum = 0.0, off = wfl[4 * i + 3], terms = std::fabs(off), residual[3] = {};
         for (int j = 0; j < 3; ++j) {
+            const double m = wfl[4 * i + j];
             double row = 0.0;
-            for (int k = 0; k < 3; ++k) row += std::fabs((double)lfw[4 * j + k]);
-            sum += std::fabs((double)wfl[4 * i + j]) * row;
+            for (int k = 0; k < 3; ++k) {
+                row += std::fabs((double)lfw[4 * j + k]);
+                residual[k] += m * lfw[4 * j + k];
+            }
+            sum += std::fabs(m) * row;
+            off += m * lfw[4 * j + 3];
+            terms += std::fabs(m * lfw[4 * j + 3]);
         }
-        if (!(sum <= 4.0)) return false;
-        worst = std::max(worst, sum);
+        residual[i] -= 1.0;
+        const double apart = std::fabs(residual[0]) + std::fabs(residual[1]) + std::fabs(residual[2]);
+        if (!(sum <= 4.0 && apart <= 12.0 * 0x1p-24 && std::fabs(off) <= 0x1p-19 * terms)) return false;
     }
-    return std::isfinite(worst);
+    return true;
 }
 
 // Whether the flattened walk's padding, 2^-17 of the scene's coordinate
