@@ -3203,6 +3203,8 @@ constexpr int kTimingEvents = 7;
 struct LuxView {
     LuxContext *ctx = nullptr;
     uint32_t sort_bins = 0;  // bins of the coherence-sort buffers
+    bool tuned = false;      // the host has set the tuning: sort_queries says whether queries are ordered
+    bool no_order = false;   // no room was found for ordering them without being asked
     LuxTuning tuning{0, 0, 16, 16, 0, 0, 64, 0, 32, 0};
     bool timing = false;
     cudaEvent_t ev[kTimingEvents] = {};
@@ -3367,56 +3369,74 @@ static lux_status view_alloc(LuxView *v) {
 
 // Coherence-sort buffers: the processing order (4 bytes per ray and sample),
 // ray keys (4 per ray), and two arrays of `bins` counters with the scan
-// scratch, allocated when a frame of the view first needs them.
-static lux_status ensure_sort_buffers(LuxView *v, uint32_t bins) {
+// scratch.  All of them or none: without room the view keeps what it had.
+static bool sort_ready(const LuxView *v, uint32_t bins) { return v->dev.sort_hist && bins <= v->sort_bins; }
+static bool make_sort_buffers(LuxView *v, uint32_t bins) {
     ViewDevice &D = v->dev;
-    if (D.sort_hist && bins <= v->sort_bins) return LUX_OK;
-    if (D.sort_hist) {  // a finer grid than before
+    if (sort_ready(v, bins)) return true;
+    const bool first = !D.sort_hist;  // else: more bins than before
+    const size_t rays = v->desc.max_rays, scan_bytes = scan_temp_bytes(bins);
+    const size_t bytes[5] = {first ? rays * sizeof(uint32_t) : 0, first ? rays * lux::kMaxNeeSamples * sizeof(uint32_t) : 0,
+                             (size_t)bins * sizeof(uint32_t), (size_t)bins * sizeof(uint32_t), scan_bytes};
+    void *p[5] = {};
+    for (int k = 0; k < 5; ++k) {
+        if (!bytes[k] || cudaMalloc(&p[k], std::max<size_t>(bytes[k], 16)) == cudaSuccess) continue;
+        cudaGetLastError();
+        for (int j = 0; j < k; ++j) cudaFree(p[j]);
+        return false;
+    }
+    if (first) {
+        D.sort_keys = (uint32_t *)p[0];
+        D.sort_perm = (uint32_t *)p[1];
+    } else {
         cudaStreamSynchronize(v->ctx->stream);
         if (v->setup_stream) cudaStreamSynchronize(v->setup_stream);
         cudaFree(D.sort_hist);
         cudaFree(D.sort_offs);
         cudaFree(D.scan_temp);
-        D.sort_hist = D.sort_offs = nullptr;
-        D.scan_temp = nullptr;
     }
-    D.scan_temp_bytes = scan_temp_bytes(bins);
-    struct A {
-        void **p;
-        size_t bytes;
-    } allocs[] = {
-        {(void **)&D.sort_keys, (size_t)v->desc.max_rays * sizeof(uint32_t)},
-        {(void **)&D.sort_perm, (size_t)v->desc.max_rays * lux::kMaxNeeSamples * sizeof(uint32_t)},
-        {(void **)&D.sort_offs, (size_t)bins * sizeof(uint32_t)},
-        {(void **)&D.scan_temp, D.scan_temp_bytes},
-        {(void **)&D.sort_hist, (size_t)bins * sizeof(uint32_t)},  // last: marks the set complete
-    };
-    for (auto &a : allocs) {
-        if (*a.p) continue;
-        if (cudaMalloc(a.p, std::max<size_t>(a.bytes, 16)) != cudaSuccess) {
-            cudaGetLastError();
-            *a.p = nullptr;
-            cudaFree(D.sort_offs);
-            cudaFree(D.scan_temp);
-            D.sort_offs = nullptr;
-            D.scan_temp = nullptr;
-            return lux_fail(v->ctx, LUX_ERR_OUT_OF_MEMORY, "view: coherence-sort buffer allocation failed");
-        }
-    }
+    D.sort_hist = (uint32_t *)p[2];
+    D.sort_offs = (uint32_t *)p[3];
+    D.scan_temp = p[4];
+    D.scan_temp_bytes = scan_bytes;
     v->sort_bins = bins;
-    return LUX_OK;
+    return true;
+}
+static lux_status ensure_sort_buffers(LuxView *v, uint32_t bins) {
+    if (make_sort_buffers(v, bins)) return LUX_OK;
+    return lux_fail(v->ctx, LUX_ERR_OUT_OF_MEMORY, "view: coherence-sort buffer allocation failed");
 }
 
 // Bits per axis of the origin grid the frame's visibility queries are ordered
 // on, 0 for none: about a bin per two queries, since finer bins than queries
 // order nothing and the bins themselves cost their clearing and their scan.
-// Without the tuning's flag only frames that can queue kOrderQueries or more
+// In a view without a tuning only frames that can queue kOrderQueries or more
 // are ordered: below it the order's launches cost what the walks gain (961x541,
 // 130,000 rays, at most 1.4 M queries: 1189 us ordered, 1179 not; 1920x1080, 4.4 M
 // rays: 12.8 ms ordered, 15.4 not).
 static uint32_t query_order_bits(uint64_t queries, bool asked) {
     if (queries < kOrderQueries && !asked) return 0u;
     return queries >= (6u << 20) ? 7u : (queries >= (1u << 20) ? 6u : 5u);
+}
+// The bins of the largest frame that the view can hold.
+static uint32_t most_query_bins(const LuxView *v) {
+    return query_bins(query_order_bits((uint64_t)v->desc.max_rays * lux::kMaxNeeSamples, true));
+}
+
+// Room for the order that a frame takes without being asked: made once, for the
+// view's largest frame, so that no later frame allocates; not while the stream
+// is being captured, where an allocation would end the capture, and not again
+// after it failed.
+static bool room_for_order(LuxView *v, uint32_t bins) {
+    if (sort_ready(v, bins)) return true;
+    if (v->no_order) return false;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(v->ctx->stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return false;
+    }
+    v->no_order = !make_sort_buffers(v, most_query_bins(v));
+    return !v->no_order;
 }
 
 extern "C" lux_status lux_view_create(LuxContext *ctx, const LuxViewDesc *desc, LuxView **out) {
@@ -3876,6 +3896,7 @@ extern "C" lux_status lux_view_trace_merge(LuxView *v, const LuxScene *scene, co
     LuxTuning t = v->tuning;
     t.closest_mode = 0;
     sec->tuning = t;
+    sec->tuned = v->tuned;
     LuxSettings s2 = s;
     s2.multi_bounce = 0;
     s2.probe_spacing = s.probe_spacing * 4.0f;
@@ -3944,12 +3965,13 @@ static lux_status view_frame(LuxView *v, const LuxScene *scene, const LuxSetting
     uint32_t query_bits = 0;
     if (F.layout == LUX_LAYOUT_SPLIT) {  // before any work of the frame is queued
         const bool asked = v->tuning.sort_queries != 0u;
-        query_bits = query_order_bits(most_queries(F, scene, (uint64_t)rc->count * F.rays_per_receiver), asked);
+        if (asked || !v->tuned)
+            query_bits = query_order_bits(most_queries(F, scene, (uint64_t)rc->count * F.rays_per_receiver), asked);
+        if (query_bits && !asked && !room_for_order(v, query_bins(query_bits))) query_bits = 0;  // as they come
         const uint32_t bins = std::max(query_bits ? query_bins(query_bits) : 0u, v->tuning.sort_rays ? kRaySortBins : 0u);
         if (bins) {
             lux_status sb = ensure_sort_buffers(v, bins);
-            if (sb != LUX_OK && (asked || v->tuning.sort_rays)) return sb;
-            if (sb != LUX_OK) query_bits = 0;  // no room: in the order they come
+            if (sb != LUX_OK) return sb;
         }
     }
     const ViewDevice &D = v->dev;
@@ -4325,9 +4347,8 @@ extern "C" lux_status lux_view_set_tuning(LuxView *v, const LuxTuning *t) {
         t->fused_trace > 1)
         return lux_fail(v->ctx, LUX_ERR_INVALID_ARGUMENT, "set_tuning: value out of range");
     v->tuning = *t;
-    const uint64_t queries = (uint64_t)v->desc.max_rays * lux::kMaxNeeSamples;  // of the view's largest frame
-    const uint32_t bins = std::max(t->sort_queries ? query_bins(query_order_bits(queries, true)) : 0u,
-                                   t->sort_rays ? kRaySortBins : 0u);
+    v->tuned = true;
+    const uint32_t bins = std::max(t->sort_queries ? most_query_bins(v) : 0u, t->sort_rays ? kRaySortBins : 0u);
     return bins ? ensure_sort_buffers(v, bins) : LUX_OK;
 }
 

@@ -374,10 +374,12 @@ typedef struct LuxTuning {
     uint32_t closest_blocks_per_sm;
     uint32_t shadow_blocks_per_sm;
     uint32_t sort_queries;        /* 1: order visibility queries by (emitter bucket of 8, origin cell of a 32^3 to
-                                     128^3 grid over the scene box, by the frame's size) before tracing;
-                                     0: only in Split frames that can queue 2^21 of them or more (the order takes
-                                     68 device bytes per ray of max_rays and up to 128 MiB, from the first such
-                                     frame on; without room the queries are traced in the order they come) */
+                                     128^3 grid over the scene box, by the frame's size) before tracing; 0: in
+                                     the order they come.  A view whose tuning was never set orders them in Split
+                                     frames that can queue 2^21 or more.  The order takes 68 device bytes per ray
+                                     of max_rays and up to 128 MiB, made for the view's largest frame when the
+                                     tuning asks for it or by the first such frame (not during a stream capture;
+                                     without room that frame and later ones keep the order they come in) */
     uint32_t sort_rays;           /* 1: order interval rays by (direction bin, origin cell) before tracing */
     uint32_t stack_depth;         /* traversal stack entries per thread: 32 or 64 (0 = 64); an overflowing
                                      walk continues with the reference's ordered scan, same answers
