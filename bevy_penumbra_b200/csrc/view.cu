@@ -3469,7 +3469,7 @@ extern "C" lux_status lux_view_destroy(LuxView *v) {
                     D.receiver_ordinal, D.order_keys, D.order_vals, D.cell_rank, D.rank_keys, D.order_temp,
                     D.corner_ids,
                     D.corner_frac, D.accum, D.count, D.merged, D.raw, D.mass, D.hist_cell, D.cell_last,
-                    D.retain_hist, D.retain_limit, D.tables, D.error_flags, D.stats,
+                    D.retain_hist, D.retain_limit, D.pass_list, D.pass_count, D.tables, D.error_flags, D.stats,
                     v->hist.dir_keys, v->hist.dir_ids, v->hist.level_base, v->hist.cell_count, v->hist.raw,
                     v->hist.mass, v->hist.cell_last, v->hist.cell_keys,
                     D.ts.ray_o, D.ts.ray_d, D.ts.ray_h, D.ts.ray_base, D.ts.ray_extra, D.ts.query_slot, D.ts.slot_contrib, D.ts.queue_o, D.ts.queue_d,
