@@ -556,8 +556,9 @@ struct Walker {
     bool have;
 
     // Returns false when the query is already complete (no instances, the ray
-    // misses the TLAS root box: traceRayTracked's early exits; or a ray that
-    // is not finite, which no triangle test accepts).  kLeaveFar: so do far
+    // misses the TLAS root box: traceRayTracked's early exits; or a ray that is
+    // not finite or has no interval, NaN bounds included, which the child tests'
+    // three-operand minima would drop: no hit satisfies them).  kLeaveFar: so do far
     // rays, with `steps` kFarSteps.
     template <bool kLeaveFar = false>
     __device__ __forceinline__ bool start(const SceneView &S, f3 origin, f3 direction, float t_min, float limit) {
@@ -568,7 +569,7 @@ struct Walker {
         hit.b1 = 0.0f;
         hit.b2 = 0.0f;
         if (S.instance_count == 0) return false;
-        if (!(finite3(origin) && finite3(direction))) return false;
+        if (!(finite3(origin) && finite3(direction) && t_min <= limit)) return false;
         // The TLAS root box is read from the live scene words (node 0), so a
         // device-side refit takes effect without a host round trip.
         float re, rx;
@@ -899,7 +900,7 @@ struct FlatWalker {
     template <bool kLeaveFar = false>
     __device__ __forceinline__ bool start(const SceneView &S, Entry *stack, f3 origin, f3 direction, float t_min,
                                           float limit) {
-        if (!(finite3(origin) && finite3(direction))) return false;
+        if (!(finite3(origin) && finite3(direction) && t_min <= limit)) return false;
         float re, rx;
         uint4 ra = __ldg(S.scene_words + 1), rb = __ldg(S.scene_words + 2);
         const f3 rl{as_float(ra.x), as_float(ra.y), as_float(ra.z)}, rh{as_float(rb.x), as_float(rb.y), as_float(rb.z)};
