@@ -133,7 +133,7 @@ struct LuxScene {
     LuxContext *ctx = nullptr;
     SceneView view{};
     void *d_nodes = nullptr, *d_tris = nullptr, *d_inst = nullptr, *d_sw = nullptr, *d_gw = nullptr,
-         *d_lights = nullptr;
+         *d_lights = nullptr, *d_tables = nullptr;
     uint32_t node_count = 0;
     // Refit state (lux_scene_refit): host copies of the instance records and
     // device instances, the TLAS binary nodes by depth, and where every TLAS
@@ -148,7 +148,8 @@ struct LuxScene {
     uint2 *d_slot_source = nullptr;             // (binary node, instance or kEmpty) per slot
     uint32_t light_count = 0;
     // Flattened tree: per instance (first flat node, first leaf record, first
-    // BLAS node, BLAS root node), and its buffers (nullptr: the scene has none).
+    // BLAS node, BLAS root node; in d_tables, as the refit's), and its nodes and
+    // leaves, which lie behind the nodes in d_nodes (flat_count 0: none).
     uint4 *d_flat_inst = nullptr;
     Bvh4Node *d_flat_nodes = nullptr;
     uint2 *d_flat_leaves = nullptr;

@@ -490,17 +490,33 @@ struct HostScene {
 // L2).  A scene of many instances of large meshes keeps the two-level walk.
 constexpr uint64_t kFlatMaxNodes = 1u << 19;
 
-// Levels of inner nodes at and below `root` (a node of a collapsed tree).
-static uint32_t tree_depth(const std::vector<Bvh4Node> &nodes, uint32_t root) {
-    uint32_t deepest = 0;
-    std::vector<std::pair<uint32_t, uint32_t>> todo = {{root, 1u}};
-    while (!todo.empty()) {
-        auto [index, depth] = todo.back();
-        todo.pop_back();
-        deepest = std::max(deepest, depth);
-        for (uint32_t c : nodes[index].child)
-            if (c != lux::kEmpty && !(c & kLeafBit)) todo.push_back({c, depth + 1u});
+// Levels of inner nodes at and below `root`, the root of a collapsed tree whose
+// nodes are [first, end): the collapse makes a node before its children, so one
+// pass in order takes every depth.  With `leaves` the leaf children are numbered
+// on the way.
+static uint32_t tree_depth(std::vector<Bvh4Node> &nodes, size_t first, uint32_t root, std::vector<uint8_t> &depth,
+                           uint32_t *leaves = nullptr) {
+    depth.assign(nodes.size() - first, 0);  // at most 96 binary levels and 2 of a split leaf
+    depth[root - first] = 1;
+    uint8_t deepest = 1;
+    uint32_t count = 0;
+    for (size_t k = first; k < nodes.size(); ++k) {
+        Bvh4Node &n = nodes[k];
+        const uint8_t below = (uint8_t)(depth[k - first] + 1);
+        bool inner = false;
+        for (int c = 0; c < 4; ++c) {
+            const uint32_t child = n.child[c];
+            if (child == lux::kEmpty) continue;
+            if (child & kLeafBit) {
+                if (leaves) n.leaf[c] = count++;
+            } else {
+                depth[child - first] = below;
+                inner = true;
+            }
+        }
+        if (inner) deepest = std::max(deepest, below);
     }
+    if (leaves) *leaves = count;
     return deepest;
 }
 
@@ -542,15 +558,16 @@ static bool flat_conditioned(const float *lfw, const float *wfl) {
 // runs into the step budget (131,072 triangles in 2 units at 1e5: every ray
 // abandoned).  An instance of more than kFlatCoarse nodes needs 2^-10 of the
 // magnitude, else the scene keeps the two-level walk, whose tests are local.
-// wfl: world_from_local rows, `stride` floats apart.
+// wfl: world_from_local rows, `stride` bytes apart.
 constexpr uint32_t kFlatCoarse = 64;
-static bool flat_placed(const std::vector<FlatBox> &boxes, const float *wfl, size_t stride) {
+static bool flat_placed(const std::vector<FlatBox> &boxes, const void *wfl, size_t stride) {
     float magnitude = 0.0f, least = INFINITY;
     for (size_t i = 0; i < boxes.size(); ++i) {
         const FlatBox &b = boxes[i];
-        float extent = 0.0f;
+        float extent = 0.0f, rows[12];
+        std::memcpy(rows, (const char *)wfl + i * stride, sizeof rows);
         for (int r = 0; r < 3; ++r) {
-            const float *m = wfl + i * stride + 4 * r;
+            const float *m = rows + 4 * r;
             const float c = m[0] * b.center[0] + m[1] * b.center[1] + m[2] * b.center[2] + m[3];
             const float h = std::fabs(m[0]) * b.half[0] + std::fabs(m[1]) * b.half[1] + std::fabs(m[2]) * b.half[2];
             if (!std::isfinite(c) || !std::isfinite(h)) return false;
@@ -641,6 +658,7 @@ static lux_status prepare_scene(const uint32_t *sw, size_t sn, const uint32_t *g
         const BinNode &box = bin[inst[i].root];
         for (int r = 0; r < 3; ++r)
             inst[i].extent = std::max({inst[i].extent, std::fabs(box.mn[r]), std::fabs(box.mx[r])});
+        if (i == 0) H.flat_boxes.reserve(inst_count);
         FlatBox fb{};
         for (int r = 0; r < 3; ++r) {
             fb.center[r] = 0.5f * (box.mn[r] + box.mx[r]);
@@ -727,7 +745,8 @@ static lux_status prepare_scene(const uint32_t *sw, size_t sn, const uint32_t *g
     std::vector<uint4> &flat = H.flat_inst;
     uint64_t flat_nodes = H.flat_tlas, flat_leaves = 0;
     bool flat_ok = inst_count > 0;
-    const uint32_t tlas_depth = inst_count ? tree_depth(nodes, tlas_root) : 0u;
+    std::vector<uint8_t> depths;
+    const uint32_t tlas_depth = inst_count ? tree_depth(nodes, 0, tlas_root, depths) : 0u;
     for (uint32_t k = 0; k < H.flat_tlas && flat_ok; ++k)  // leaves of several instances have no single root
         for (uint32_t c : nodes[k].child) flat_ok = flat_ok && (c == lux::kEmpty || !(c & kLeafBit) || ((c >> 27) & 15u) == 0u);
     for (uint32_t i = 0; i < inst_count; ++i) {
@@ -738,10 +757,7 @@ static lux_status prepare_scene(const uint32_t *sw, size_t sn, const uint32_t *g
             uint32_t r = bl.root(inst[i].root);
             if (!bl.error.empty()) return fail(LUX_ERR_MALFORMED_SCENE, "scene upload (BLAS): " + bl.error);
             uint32_t leaves = 0;
-            for (size_t k = node0; k < nodes.size(); ++k)
-                for (int c = 0; c < 4; ++c)
-                    if (nodes[k].child[c] != lux::kEmpty && (nodes[k].child[c] & kLeafBit)) nodes[k].leaf[c] = leaves++;
-            const uint32_t depth = tree_depth(nodes, r);
+            const uint32_t depth = tree_depth(nodes, node0, r, depths, &leaves);
             it = blas_root.emplace(inst[i].root, Blas{r, node0, (uint32_t)nodes.size() - node0, leaves, depth}).first;
         }
         const Blas &b = it->second;
@@ -759,11 +775,7 @@ static lux_status prepare_scene(const uint32_t *sw, size_t sn, const uint32_t *g
         flat_ok = flat_nodes <= kFlatMaxNodes && flat_leaves <= kLeafFirstMask &&
                   3u * (tlas_depth + b.depth) <= (uint32_t)lux::kFlatStack && flat_conditioned(lfw, wfl);
     }
-    if (flat_ok) {  // world_from_local rows as floats, 36 words per instance
-        std::vector<float> words(36 * (size_t)inst_count);
-        std::memcpy(words.data(), sw + 4 * (size_t)inst_base, words.size() * 4);
-        flat_ok = flat_placed(H.flat_boxes, words.data() + 12, 36);
-    }
+    flat_ok = flat_ok && flat_placed(H.flat_boxes, sw + 4 * (size_t)inst_base + 12, 36 * sizeof(uint32_t));
     if (flat_ok) {
         H.flat_count = (uint32_t)flat_nodes;
         H.flat_leaves = (uint32_t)flat_leaves;
@@ -809,16 +821,6 @@ extern "C" lux_status lux_scene_validate(const uint32_t *sw, size_t sn, const ui
         message[n] = '\0';
     }
     return status;
-}
-
-static void flat_free(LuxScene *S) {
-    cudaFree(S->d_flat_inst);
-    cudaFree(S->d_flat_nodes);
-    cudaFree(S->d_flat_leaves);
-    S->d_flat_inst = nullptr;
-    S->d_flat_nodes = nullptr;
-    S->d_flat_leaves = nullptr;
-    S->flat_count = 0;
 }
 
 // Rebuilds the flattened tree from the scene's current words (on the context
@@ -868,14 +870,48 @@ extern "C" lux_status lux_scene_upload(LuxContext *ctx, const uint32_t *sw, size
         if (src && cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice) != cudaSuccess) return false;
         return true;
     };
-    bool ok = alloc_copy(&S->d_nodes, nodes.data(), nodes.size() * sizeof(Bvh4Node)) &&
+    // The flattened tree's nodes lie behind the nodes, in their allocation;
+    // without room for both the scene keeps the two-level walk.
+    const size_t node_bytes = nodes.size() * sizeof(Bvh4Node);
+    if (H.flat_count) {
+        const size_t flat_bytes = H.flat_count * sizeof(Bvh4Node) + H.flat_leaves * sizeof(uint2);
+        if (cudaMalloc(&S->d_nodes, node_bytes + flat_bytes) == cudaSuccess) {
+            S->d_flat_nodes = (Bvh4Node *)S->d_nodes + nodes.size();
+            S->d_flat_leaves = (uint2 *)(S->d_flat_nodes + H.flat_count);
+            S->flat_count = H.flat_count;
+            S->flat_tlas = H.flat_tlas;
+            S->flat_boxes = H.flat_boxes;
+        } else {
+            cudaGetLastError();
+            S->d_nodes = nullptr;
+        }
+    }
+    // The small tables in one allocation and one copy.
+    std::vector<unsigned char> tables;
+    auto table = [&](const void *src, size_t bytes) {
+        const size_t at = (tables.size() + 15) & ~(size_t)15;
+        tables.resize(at + bytes);
+        if (bytes) std::memcpy(tables.data() + at, src, bytes);
+        return at;
+    };
+    const size_t at_source = table(slot_source.data(), slot_source.size() * sizeof(uint2));
+    const size_t at_order = table(refit_order.data(), refit_order.size() * 4);
+    const size_t at_depth = table(depth_start.data(), depth_start.size() * 4);
+    const size_t at_flat = table(H.flat_inst.data(), S->flat_count ? H.flat_inst.size() * sizeof(uint4) : 0);
+    bool ok = (S->d_nodes ? cudaMemcpy(S->d_nodes, nodes.data(), node_bytes, cudaMemcpyHostToDevice) == cudaSuccess
+                          : alloc_copy(&S->d_nodes, nodes.data(), node_bytes)) &&
               alloc_copy(&S->d_tris, tris.data(), tris.size() * sizeof(float4)) &&
               alloc_copy(&S->d_inst, inst.data(), inst.size() * sizeof(DeviceInstance)) &&
               alloc_copy(&S->d_sw, sw, sn * 16) && alloc_copy(&S->d_gw, gw, gn * 16) &&
               alloc_copy(&S->d_lights, lights, (size_t)light_count * sizeof(LuxLight)) &&
-              alloc_copy((void **)&S->d_refit_order, refit_order.data(), refit_order.size() * 4) &&
-              alloc_copy((void **)&S->d_depth_start, depth_start.data(), depth_start.size() * 4) &&
-              alloc_copy((void **)&S->d_slot_source, slot_source.data(), slot_source.size() * sizeof(uint2));
+              alloc_copy(&S->d_tables, tables.data(), tables.size());
+    if (ok) {
+        unsigned char *t = (unsigned char *)S->d_tables;
+        S->d_slot_source = (uint2 *)(t + at_source);
+        S->d_refit_order = (uint32_t *)(t + at_order);
+        S->d_depth_start = (uint32_t *)(t + at_depth);
+        S->d_flat_inst = (uint4 *)(t + at_flat);
+    }
     if (!ok) {
         cudaGetLastError();
         lux_scene_destroy(S);
@@ -899,21 +935,6 @@ extern "C" lux_status lux_scene_upload(LuxContext *ctx, const uint32_t *sw, size
         V.root_lo[k] = root_lo[k];
         V.root_hi[k] = root_hi[k];
     }
-    if (H.flat_count) {
-        // Without room for it the scene keeps the two-level walk.
-        if (cudaMalloc((void **)&S->d_flat_inst, H.flat_inst.size() * sizeof(uint4)) == cudaSuccess &&
-            cudaMalloc((void **)&S->d_flat_nodes, (size_t)H.flat_count * sizeof(Bvh4Node)) == cudaSuccess &&
-            cudaMalloc((void **)&S->d_flat_leaves, std::max<size_t>(H.flat_leaves, 1) * sizeof(uint2)) == cudaSuccess &&
-            cudaMemcpy(S->d_flat_inst, H.flat_inst.data(), H.flat_inst.size() * sizeof(uint4),
-                       cudaMemcpyHostToDevice) == cudaSuccess) {
-            S->flat_count = H.flat_count;
-            S->flat_tlas = H.flat_tlas;
-            S->flat_boxes = H.flat_boxes;
-        } else {
-            cudaGetLastError();
-            flat_free(S);
-        }
-    }
     S->node_count = (uint32_t)nodes.size();
     S->instance_base = inst_base;
     S->instance_words.assign(sw + 4 * (size_t)inst_base, sw + 4 * ((size_t)inst_base + 9 * (size_t)inst_count));
@@ -922,9 +943,15 @@ extern "C" lux_status lux_scene_upload(LuxContext *ctx, const uint32_t *sw, size
     S->slot_count = tlas_slots;
     S->light_count = light_count;
     if (S->flat_count) {
-        lux_status rc = lux_cuda_check(ctx, (int)cudaStreamSynchronize(nullptr), "scene upload");  // the copies above
+        // The tree is built on the context's stream, where it is used, after the
+        // copies above (default stream) and behind whatever frames are queued
+        // there: the host waits for neither.
+        cudaEvent_t copied = nullptr;
+        lux_status rc = lux_cuda_check(ctx, (int)cudaEventCreateWithFlags(&copied, cudaEventDisableTiming), "scene upload");
+        if (rc == LUX_OK) rc = lux_cuda_check(ctx, (int)cudaEventRecord(copied, nullptr), "scene upload");
+        if (rc == LUX_OK) rc = lux_cuda_check(ctx, (int)cudaStreamWaitEvent(ctx->stream, copied, 0), "scene upload");
+        if (copied) cudaEventDestroy(copied);
         if (rc == LUX_OK) rc = flatten(S, true);
-        if (rc == LUX_OK) rc = lux_cuda_check(ctx, (int)cudaStreamSynchronize(ctx->stream), "scene upload");
         if (rc != LUX_OK) {
             lux_scene_destroy(S);
             return rc;
@@ -942,10 +969,7 @@ extern "C" lux_status lux_scene_destroy(LuxScene *S) {
     cudaFree(S->d_sw);
     cudaFree(S->d_gw);
     cudaFree(S->d_lights);
-    cudaFree(S->d_refit_order);
-    cudaFree(S->d_depth_start);
-    cudaFree(S->d_slot_source);
-    flat_free(S);
+    cudaFree(S->d_tables);
     delete S;
     return LUX_OK;
 }
@@ -996,7 +1020,7 @@ extern "C" lux_status lux_scene_refit(LuxScene *S, const float *wfl, uint32_t co
             for (int c = 0; c < 4; ++c) inst[i].row[r][c] = lfw[4 * r + c];
         if (S->flat_count) conditioned = conditioned && flat_conditioned(lfw, m);
     }
-    if (S->flat_count) conditioned = conditioned && flat_placed(S->flat_boxes, wfl, 12);
+    if (S->flat_count) conditioned = conditioned && flat_placed(S->flat_boxes, wfl, 12 * sizeof(float));
     cudaStream_t st = ctx->stream;
     cudaSetDevice(ctx->device);
     uint4 *sw = (uint4 *)S->d_sw;
