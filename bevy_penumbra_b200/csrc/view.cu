@@ -747,10 +747,11 @@ __device__ __forceinline__ uint32_t warp_fetch(uint32_t *counter, uint32_t tile 
 }
 
 // fn(slot, valid) by whole warps for n items over the launch's persistent
-// warps, 32 at a time.  When 1 / kShare of the warps could take all items in
-// one round with kMostFew or fewer each, they do (down to kFewestLanes, the
-// other lanes idle): a short launch waits for the longest walk of a warp, in
-// which the warp's other walks take their turns.  Closest hits gain up to 8 per
+// warps, 32 at a time.  When 1 / kShare of the launch's warps could take all
+// items with kMostFew or fewer each, they do (down to kFewestLanes, the other
+// lanes idle; a launch of 16 blocks per SM holds more warps than are resident
+// at once, the later ones follow as others end): a short launch waits for the
+// longest walk of a warp, in which the warp's other walks take their turns.  Closest hits gain up to 8 per
 // warp (12k rays of a 640x360 frame 72 -> 52 us, 4k rays 58 -> 37; at 16 per
 // warp 61k rays take 153 us, not 118), occlusion walks, which end sooner, up to
 // 16 in half the warps (27k queries 57 -> 48 us).  Warps past the items fetch
