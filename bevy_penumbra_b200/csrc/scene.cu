@@ -201,17 +201,21 @@ __device__ __forceinline__ LuxHit ray_hit(const lux::Hit &h, uint32_t visited) {
     return out;
 }
 
-// A ray that starts far outside the scene: not inlined, and the ray and its hit
-// in memory, or the walk beside it would lose registers (3% of a call).
+// The rays of a warp that start far outside the scene (far: the lane's does),
+// by the whole warp: not inlined, and the rays and their hits in memory, or the
+// walk beside it would lose registers (3% of a call).  300,000 rays of 131,072
+// triangles from 20 sizes away: 139 us (153 on the two-level walk of before).
 template <bool kAnyHit>
-__device__ __noinline__ lux::TraceCounters trace_far_ray(const SceneView &S, const LuxRay *ray, LuxHit *hit) {
-    const LuxRay r = *ray;
+__device__ __noinline__ lux::TraceCounters trace_far_rays(const SceneView &S, const LuxRay *ray, LuxHit *hit, bool far,
+                                                          lux::LeafScratch *L) {
+    LuxRay r{};
+    if (far) r = *ray;
     lux::Hit h;
     lux::TraceCounters cn{0, 0, 0};
-    lux::trace<kAnyHit, lux::kStack, lux::FarSlabRay>(S, lux::f3{r.origin[0], r.origin[1], r.origin[2]},
-                                                     lux::f3{r.direction[0], r.direction[1], r.direction[2]},
-                                                     kAnyHit ? 0.0f : r.tmin, r.limit, h, cn);
-    *hit = ray_hit(h, cn.nodes);
+    lux::trace_warp<kAnyHit, lux::kStack, false, lux::FarSlabRay>(
+        S, far, lux::f3{r.origin[0], r.origin[1], r.origin[2]}, lux::f3{r.direction[0], r.direction[1], r.direction[2]},
+        kAnyHit ? 0.0f : r.tmin, r.limit, h, cn, L);
+    if (far) *hit = ray_hit(h, cn.nodes);
     return cn;
 }
 
@@ -238,10 +242,14 @@ __global__ void __launch_bounds__(128, kFlat ? (kAnyHit ? 8 : 7) : 5)
     } else {
         lux::trace_warp<kAnyHit, lux::kStack, true>(S, active, o, d, tmin, r.limit, h, cn, L);
     }
-    if (h.errors == lux::kFarRay)
-        cn = trace_far_ray<kAnyHit>(S, rays + i, hits + i);
-    else if (active)
-        hits[i] = ray_hit(h, cn.nodes);
+    const bool far = active && h.errors == lux::kFarRay;
+    if (active && !far) hits[i] = ray_hit(h, cn.nodes);
+    if (__any_sync(0xffffffffu, far)) {
+        const lux::TraceCounters more = trace_far_rays<kAnyHit>(S, rays + i, hits + i, far, L);
+        cn.nodes += more.nodes;
+        cn.triangles += more.triangles;
+        cn.instances += more.instances;
+    }
     if (counters) {
         unsigned long long n = cn.nodes, t = cn.triangles, in = cn.instances;
         for (int off = 16; off > 0; off >>= 1) {
@@ -359,7 +367,7 @@ __global__ void __launch_bounds__(1024) refit_kernel(uint4 *__restrict__ sw, uin
 }
 
 // The caller rays of a trace scratch that start far outside the scene (noted in
-// work_counter[2], marked in ray_h), a thread each.  A kernel of its own, nearly
+// work_counter[2], marked in ray_h), by whole warps.  A kernel of its own, nearly
 // always empty (4099 rays 118.5 -> 120.5 us; as a function called from the walk's
 // kernel 400,000 rays took 1.8% more), and in this file: in the one of the
 // frame's kernels the second walk made the compiler spill more there.
@@ -369,14 +377,20 @@ __global__ void __launch_bounds__(128) far_rays_kernel(const __grid_constant__ S
                                                        unsigned long long *instances) {
     lux::after_previous();
     if (T.work_counter[2] == 0u) return;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
-        if (T.ray_h[i].z != lux::kFarRay) continue;
-        const LuxRay r = rays[i];
+    __shared__ lux::LeafScratch scratch[4];
+    const uint32_t lane = threadIdx.x & 31u, warps = gridDim.x * 4u;
+    for (unsigned long long w = blockIdx.x * 4u + (threadIdx.x >> 5); w * 32u < count; w += warps) {
+        const uint32_t i = (uint32_t)w * 32u + lane;
+        const bool far = i < count && T.ray_h[i].z == lux::kFarRay;
+        if (!__any_sync(0xffffffffu, far)) continue;
+        LuxRay r{};
+        if (far) r = rays[i];
         lux::Hit h;
         lux::TraceCounters cn{0, 0, 0};
-        lux::trace<false, lux::kStack, lux::FarSlabRay>(S, lux::f3{r.origin[0], r.origin[1], r.origin[2]},
-                                                        lux::f3{r.direction[0], r.direction[1], r.direction[2]},
-                                                        r.tmin, r.limit, h, cn);
+        lux::trace_warp<false, lux::kStack, false, lux::FarSlabRay>(
+            S, far, lux::f3{r.origin[0], r.origin[1], r.origin[2]},
+            lux::f3{r.direction[0], r.direction[1], r.direction[2]}, r.tmin, r.limit, h, cn, &scratch[threadIdx.x >> 5]);
+        if (!far) continue;
         T.ray_o[i].w = h.t;
         T.ray_d[i].w = h.b1;
         T.ray_h[i] = make_uint4(h.tri, h.inst, h.errors, lux::as_uint(h.b2));
@@ -1094,6 +1108,6 @@ extern "C" lux_status lux_trace_rays(LuxContext *ctx, const LuxScene *scene, con
 void lux_launch_far_rays(LuxContext *ctx, const LuxScene *scene, const TraceScratch &T, const LuxRay *rays,
                          uint32_t count, unsigned long long *nodes, unsigned long long *triangles,
                          unsigned long long *instances) {
-    const uint32_t blocks = std::min<uint32_t>((count + 127u) / 128u, (uint32_t)ctx->sm_count);
+    const uint32_t blocks = std::min<uint32_t>((count + 127u) / 128u, (uint32_t)ctx->sm_count * 4u);
     lux::launch(far_rays_kernel, blocks, 128, 0, ctx->stream, scene->view, T, rays, count, nodes, triangles, instances);
 }

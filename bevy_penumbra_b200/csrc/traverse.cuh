@@ -206,16 +206,27 @@ __device__ __forceinline__ void make_slab(FarSlabRay &r, f3 o, f3 d, float) {
 __device__ __forceinline__ void make_slab(SlabRay &r, f3 o, f3 d, float pad) { r = slab_ray(o, d, pad); }
 __device__ __forceinline__ uint32_t node_test(const Bvh4Node *__restrict__ nodes, uint32_t index, const FarSlabRay &r,
                                               float limit, float tmin, float entry[4], uint32_t child[4]) {
-    const Bvh4Node &n = nodes[index];
-    const bool sx = as_uint(r.ix) >> 31, sy = as_uint(r.iy) >> 31, sz = as_uint(r.iz) >> 31;
+    const float4 *p = reinterpret_cast<const float4 *>(nodes + index);
+    const uint32_t sx = as_uint(r.ix) >> 31, sy = as_uint(r.iy) >> 31, sz = as_uint(r.iz) >> 31;
+    const float4 nx = __ldg(p + sx), fx = __ldg(p + (1u - sx));
+    const float4 ny = __ldg(p + 2u + sy), fy = __ldg(p + (3u - sy));
+    const float4 nz = __ldg(p + 4u + sz), fz = __ldg(p + (5u - sz));
+    const uint4 ch = __ldg(reinterpret_cast<const uint4 *>(p + 6));
+    child[0] = ch.x;
+    child[1] = ch.y;
+    child[2] = ch.z;
+    child[3] = ch.w;
+    const float NX[4] = {nx.x, nx.y, nx.z, nx.w}, FX[4] = {fx.x, fx.y, fx.z, fx.w};
+    const float NY[4] = {ny.x, ny.y, ny.z, ny.w}, FY[4] = {fy.x, fy.y, fy.z, fy.w};
+    const float NZ[4] = {nz.x, nz.y, nz.z, nz.w}, FZ[4] = {fz.x, fz.y, fz.z, fz.w};
     uint32_t mask = 0;
+#pragma unroll
     for (int i = 0; i < 4; ++i) {
-        child[i] = n.child[i];
-        const float lx = (n.lo_x[i] - r.ox) * r.ix, hx = (n.hi_x[i] - r.ox) * r.ix;
-        const float ly = (n.lo_y[i] - r.oy) * r.iy, hy = (n.hi_y[i] - r.oy) * r.iy;
-        const float lz = (n.lo_z[i] - r.oz) * r.iz, hz = (n.hi_z[i] - r.oz) * r.iz;
-        float near_t = fmaxf(fmaxf(sx ? hx : lx, sy ? hy : ly), fmaxf(sz ? hz : lz, 0.0f));
-        float far_t = fminf(fminf(sx ? lx : hx, sy ? ly : hy), sz ? lz : hz);
+        const float ax = (NX[i] - r.ox) * r.ix, bx = (FX[i] - r.ox) * r.ix;
+        const float ay = (NY[i] - r.oy) * r.iy, by = (FY[i] - r.oy) * r.iy;
+        const float az = (NZ[i] - r.oz) * r.iz, bz = (FZ[i] - r.oz) * r.iz;
+        float near_t = fmaxf(fmaxf(ax, ay), fmaxf(az, 0.0f));
+        float far_t = fminf(fminf(bx, by), bz);
         near_t = near_t - fabsf(near_t) * 7.2e-7f;
         far_t = far_t + fabsf(far_t) * 7.2e-7f;
         // An empty slot's inverted infinities come out NaN: every comparison fails.
@@ -228,7 +239,7 @@ __device__ __forceinline__ uint32_t node_test(const Bvh4Node *__restrict__ nodes
 
 // Whether a caller's ray starts so far outside (more than 8 times the scene
 // box's largest coordinate magnitude M) that its padding would be large against
-// the triangles: it is traced by itself then, by FarSlabRay.
+// the triangles: it takes the two-level walk then, by FarSlabRay.
 constexpr float kFarOrigin = 8.0f;
 __device__ __forceinline__ float largest_component(f3 v) { return max3(fabsf(v.x), fabsf(v.y), fabsf(v.z)); }
 constexpr uint32_t kFarSteps = 0xffffffffu;  // `steps` of such a ray's walker
@@ -830,9 +841,9 @@ struct Walker {
 // Closest hit (kAnyHit = false) or any hit of one ray.  kDepth is the stack
 // depth: a shallower stack uses less local memory per thread, and a walk that
 // overflows it continues with the reference's ordered scan (same answers).
-template <bool kAnyHit, int kDepth = kStack, typename Slab = SlabRay>
+template <bool kAnyHit, int kDepth = kStack>
 __device__ void trace(const SceneView &S, f3 o, f3 d, float tmin, float limit, Hit &hit, TraceCounters &cn) {
-    Walker<kAnyHit, kDepth, Slab> w;
+    Walker<kAnyHit, kDepth> w;
     uint2 stack[kDepth];
     if (w.start(S, o, d, tmin, limit))
         while (!w.step(S, stack, cn)) {
@@ -1069,12 +1080,12 @@ struct FlatWalker {
 // has a query), and the BLAS leaves reached in each round are tested by the
 // whole warp (leaf_pass).  A lane without a query returns no hit.
 // kFar: the rays are a caller's and may start far outside the scene; one that
-// does returns no hit and errors = kFarRay, and is traced by itself (trace with
-// FarSlabRay) where that costs the walk beside it least.
-template <bool kAnyHit, int kDepth = kStack, bool kFar = false>
+// does returns no hit and errors = kFarRay, and is traced after the others
+// (trace_warp with FarSlabRay) where that costs the walk beside it least.
+template <bool kAnyHit, int kDepth = kStack, bool kFar = false, typename Slab = SlabRay>
 __device__ __forceinline__ void trace_warp(const SceneView &S, bool active, f3 o, f3 d, float tmin, float limit,
                                            Hit &hit, TraceCounters &cn, LeafScratch *L) {
-    Walker<kAnyHit, kDepth> w;
+    Walker<kAnyHit, kDepth, Slab> w;
     w.hit = Hit{limit, kEmpty, kEmpty, 0u, 0.0f, 0.0f};
     w.steps = 0;
     uint2 stack[kDepth];
