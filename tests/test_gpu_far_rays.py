@@ -17,8 +17,10 @@ pytestmark = pytest.mark.gpu
 SIDE = 256  # quads of the grid's edge
 
 
-def grid_scene(at=(0.0, 0.0, 0.0)):
-    """A bumped grid of 2 units (131,072 triangles), rotated, at a place."""
+def grid_scene(at=(0.0, 0.0, 0.0), alone=False):
+    """A bumped grid of 2 units (131,072 triangles), rotated, at a place;
+    `alone`, or with seven small quads beside it (few turned instances keep the
+    two-level walk, these take the flattened tree)."""
     u = np.linspace(-1.0, 1.0, SIDE + 1)
     x, y = np.meshgrid(u, u, indexing="ij")
     v = np.stack([x, y, 0.1 * np.sin(5 * x) * np.cos(4 * y)], -1).reshape(-1, 3).astype(np.float32)
@@ -31,6 +33,11 @@ def grid_scene(at=(0.0, 0.0, 0.0)):
     m[:, :3] = quat_xyz(0.5, 0.3, 0.0)
     m[:, 3] = at
     desc.add_instance(desc.add_mesh(scenes.Mesh(v, tri.astype(np.uint32))), m, flags=8, material=mat)
+    small = desc.add_mesh(scenes.quad((-0.02, -0.02, 0), (0.02, -0.02, 0), (0.02, 0.02, 0), (-0.02, 0.02, 0)))
+    for k in range(0 if alone else 7):
+        p = m.copy()
+        p[:, 3] += m[:, :3] @ np.float32([0.9, -0.9 + 0.3 * k, -0.05])
+        desc.add_instance(small, p, flags=8, material=mat)
     return bp.PackedScene.from_desc(desc), m
 
 
@@ -85,9 +92,10 @@ def check(packed, rays):
     np.testing.assert_array_equal(from_device(d_out, np.float32, (len(rays), 4))[hit, 3], want["distance"][hit])
 
 
-@pytest.mark.parametrize("distance", [20.0, 60.0, 130.0, 2e3, 2e4, 2e5])
-def test_rays_from_outside(distance):
-    packed, m = grid_scene()
+@pytest.mark.parametrize("alone", [False, True])
+@pytest.mark.parametrize("distance", [3.0, 10.0, 20.0, 60.0, 130.0, 2e3, 2e4, 2e5])
+def test_rays_from_outside(distance, alone):
+    packed, m = grid_scene(alone=alone)
     check(packed, rays_to(m, distance, 700, int(distance)))
 
 
@@ -105,7 +113,10 @@ def test_refit_far_from_the_origin_and_back():
     ctx = bp.LuxContext()
     scene = bp.GpuScene(ctx, near)
     for packed, m in ((far, m1), (near, m0)):
-        scene.refit(m[None])
+        base = int(packed.scene_words[0, 1])
+        rows = packed.scene_words.view(np.float32)
+        caller = {int(c): rows[base + 9 * i + 3:base + 9 * i + 6] for i, c in enumerate(packed.instance_order)}
+        scene.refit(np.stack([caller[int(c)] for c in near.instance_order]))
         rays = rays_to(m, 3.0, 300, 8)
         d_rays, d_hits = to_device(rays), empty_device(len(rays) * bp.HIT_DTYPE.itemsize)
         bp.trace_rays(ctx, scene, d_rays.data_ptr(), len(rays), d_hits.data_ptr())

@@ -18,9 +18,9 @@ pytestmark = pytest.mark.gpu
 def test_rows_that_are_not_inverses(shift):
     packed, m = grid_scene((0.5, 0.25, -0.5))
     words = packed.scene_words.copy()
-    first = int(words[0, 1])
-    rows = words[first:first + 3].view(np.float32)
-    rows[:, 3] += np.float32(shift)
+    for slot in range(len(packed.instance_order)):
+        first = int(words[0, 1]) + 9 * slot
+        words[first:first + 3].view(np.float32)[:, 3] += np.float32(shift)
     rays = rays_to(m, 3.0, 4000, 3)
     want, _ = oracle.OracleScene(words, packed.geometry_words, packed.lights).trace_rays(rays)
     assert np.mean(want["triangle"] != EMPTY) > 0.9
