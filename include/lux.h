@@ -252,7 +252,10 @@ lux_status lux_emissive_lights_at(const uint32_t *geometry_words, size_t geometr
 /* Uploads word streams (host pointers) and builds the device BVH4 layout.
  * scene_words = [header, TLAS node words, BLAS node words, instance words,
  * materials...]; conventional_lights = how many leading light records are
- * conventional (lightCounts.x); the rest are emissive (lightCounts.y). */
+ * conventional (lightCounts.x); the rest are emissive (lightCounts.y).  Device
+ * memory beside the words, nodes and triangles: up to 64 MB of world-space node
+ * copies (128 bytes each, at most 2^19) and 8 bytes per copied leaf, where the
+ * scene allows them and there is room. */
 lux_status lux_scene_upload(LuxContext *ctx,
                             const uint32_t *scene_words, size_t scene_word_count,
                             const uint32_t *geometry_words, size_t geometry_word_count,
@@ -510,7 +513,9 @@ lux_status lux_measure_read_rate(LuxContext *ctx, uint64_t bytes, uint32_t passe
  * backward data gradients; Adam (FP32 master copies) for the table and the
  * weights.  Loss: relative L2, (y - t)^2 / (y^2 + 0.01).  Trained online on
  * interval radiance samples the transport produces and queried for the
- * radiance arriving at a point from a direction. */
+ * radiance arriving at a point from a direction.  Device memory: 44 bytes per
+ * table entry (a 32-byte record of values and moments, 24 of them used, so that
+ * a step moves whole sectors; 8 of gradients, 4 of the BF16 copy). */
 typedef struct LuxCache LuxCache;
 typedef struct LuxCacheDesc {
     uint32_t levels;          /* 16 */
